@@ -171,17 +171,19 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // ------------------------------------------------------------------ launch helpers
 inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK : B200_ERR_CUDA; }
 
-// Whether kernels are launched with the programmatic-stream-serialization attribute: only when the environment
-// variable B200GPT_PDL=1 (read once) asks for it.  Off by default because it measured slower: in a replayed CUDA graph
-// the kernels of the forward already follow each other within 0.3 us, and letting the next kernel's CTAs take their
-// SMs early cost 2 % at 512 x 300 tokens and 3 % at 64 x 300.
+// Whether kernels that do not ask for it are launched with the programmatic-stream-serialization attribute too: only when
+// the environment variable B200GPT_PDL=1 (read once) says so.  Long kernels do not ask: in a replayed CUDA graph they already
+// follow each other within 0.3 us, and letting the next kernel's CTAs take their SMs early cost 2 % of a forward at 512 x 300
+// tokens and 3 % at 64 x 300.  Launches of a few rows (kFewRowsPdl) do: they last 2-10 us, of which the start of the next
+// kernel is a good part.
 bool pdl_enabled();
+constexpr int64_t kFewRowsPdl = 512;
 
 // cudaLaunchConfig_t with room for the two attributes this library uses: cluster size and programmatic serialization.
 struct LaunchSetup {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attrs[2];
-  LaunchSetup(dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream, int cluster_x = 1, bool allow_pdl = true) {
+  LaunchSetup(dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream, int cluster_x = 1, bool pdl = pdl_enabled()) {
     cfg = cudaLaunchConfig_t{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem_bytes, cfg.stream = stream;
     unsigned n = 0;
@@ -190,7 +192,7 @@ struct LaunchSetup {
       attrs[n].val.clusterDim.x = (unsigned)cluster_x, attrs[n].val.clusterDim.y = 1, attrs[n].val.clusterDim.z = 1;
       ++n;
     }
-    if (allow_pdl && pdl_enabled()) {
+    if (pdl) {
       attrs[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attrs[n].val.programmaticStreamSerializationAllowed = 1;
       ++n;

@@ -128,9 +128,61 @@ ln_stats_from_moments_kernel(const float2* __restrict__ moments, int64_t ld, int
   }
 }
 
+// The same for few rows, whose slices are narrow and many (48 for 768 columns): a warp per row, a slice per lane.  Latency is
+// all there is to it: 2 x 48 loads one behind another per thread took 4.6 us at 16 x 768, this takes 2.
+template <typename T>
+__global__ void __launch_bounds__(256)
+ln_stats_few_rows_kernel(const float2* __restrict__ moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int M,
+                         float2* __restrict__ stats, T* __restrict__ ext) {
+  const int row = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (row >= M) return;
+  constexpr int kHeld = 8;  // slices per lane that stay in registers between the two passes
+  float2 part[kHeld];
+  float wsum = 0.f;
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int s = i * 32 + lane;
+    part[i] = s < slices ? moments[(int64_t)s * ld + row] : make_float2(0.f, 0.f);
+  }
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) wsum = fmaf((float)max(min(slice_cols, cols - (i * 32 + lane) * slice_cols), 0), part[i].x, wsum);
+  for (int s = kHeld * 32 + lane; s < slices; s += 32) wsum = fmaf((float)min(slice_cols, cols - s * slice_cols), moments[(int64_t)s * ld + row].x, wsum);
+  const float mean = warp_sum(wsum) / (float)cols;
+  float m2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const float d = part[i].x - mean;
+    m2 += fmaf((float)max(min(slice_cols, cols - (i * 32 + lane) * slice_cols), 0) * d, d, part[i].y);
+  }
+  for (int s = kHeld * 32 + lane; s < slices; s += 32) {
+    const float2 q = moments[(int64_t)s * ld + row];
+    const float d = q.x - mean;
+    m2 += fmaf((float)min(slice_cols, cols - s * slice_cols) * d, d, q.y);
+  }
+  const float sd = sqrtf(warp_sum(m2) / (float)cols + eps);
+  if (lane == 0) stats[row] = make_float2(mean, 1.0f / sd);
+  if (ext && lane < kLnExtCols * 2 / 16)
+    reinterpret_cast<uint4*>(ext + (int64_t)row * kLnExtCols)[lane] = lane == 0 ? ln_ext_head<T>(mean, sd) : make_uint4(0u, 0u, 0u, 0u);
+}
+
+template <typename T>
+static cudaError_t launch_ln_stats(const float2* moments, int64_t ld, int slices, int slice_cols, int64_t N, float eps, int64_t M, float* stats, void* ext,
+                                   cudaStream_t stream) {
+  if (M <= kFewRowsPdl) {
+    LaunchSetup ls(dim3((unsigned)((M + 7) / 8)), dim3(256), 0, stream, 1, true);
+    return cudaLaunchKernelEx(&ls.cfg, ln_stats_few_rows_kernel<T>, moments, ld, slices, slice_cols, (int)N, eps, (int)M, reinterpret_cast<float2*>(stats),
+                              static_cast<T*>(ext));
+  }
+  LaunchSetup ls(dim3((unsigned)((M + 255) / 256)), dim3(256), 0, stream);
+  return cudaLaunchKernelEx(&ls.cfg, ln_stats_from_moments_kernel<T>, moments, ld, slices, slice_cols, (int)N, eps, M, reinterpret_cast<float2*>(stats),
+                            static_cast<T*>(ext));
+}
+
 size_t gemm_ln_workspace_bytes(int64_t M, int64_t N) {
   if (M <= 0 || N <= 0) return 0;
-  const int64_t slices = (N + gemm::NARROW_BN - 1) / gemm::NARROW_BN;  // (the narrow-tile kernel's slices; the wide kernel uses every other one)
+  const int64_t slices = (N + 15) / 16;  // (the narrowest slices, those of at most 64 rows)
   return (size_t)(slices * ((M + 63) / 64 * 64)) * 8;
 }
 
@@ -183,18 +235,14 @@ int launch_gemm_ln(const void* a, const void* b, const void* bias, const void* r
 #undef B200_GEMM_LN_DISPATCH
   if (st != B200_OK || !stats_out) return st;
   // width of the column slices whose moments the GEMM left: the wide kernel's epilogue warps cover EPI_COLS columns, a
-  // narrow tile NARROW_BN
+  // narrow tile NARROW_BN, a tile of at most 64 rows few_rows_cols
   const bool narrow = io_dtype == B200_F16 ? takes_narrow_tiles<__half, 0>(M, out, ld_out, residual, ld_res)
                                            : takes_narrow_tiles<__nv_bfloat16, 0>(M, out, ld_out, residual, ld_res);
-  const int slice_cols = narrow ? NARROW_BN : EPI_COLS;
+  const int slice_cols = !narrow ? EPI_COLS : M <= kFewMaxRows ? few_rows_cols(N, 2) : NARROW_BN;
   const int slices = (int)((N + slice_cols - 1) / slice_cols);
-  LaunchSetup ls(dim3((unsigned)((M + 255) / 256)), dim3(256), 0, stream);
-  const cudaError_t e =
-      io_dtype == B200_F16
-          ? cudaLaunchKernelEx(&ls.cfg, ln_stats_from_moments_kernel<__half>, (const float2*)ln.stats_out, ln.stats_out_ld, slices, slice_cols,
-                               (int)N, eps, M, reinterpret_cast<float2*>(stats_out), static_cast<__half*>(ext_out))
-          : cudaLaunchKernelEx(&ls.cfg, ln_stats_from_moments_kernel<__nv_bfloat16>, (const float2*)ln.stats_out, ln.stats_out_ld, slices,
-                               slice_cols, (int)N, eps, M, reinterpret_cast<float2*>(stats_out), static_cast<__nv_bfloat16*>(ext_out));
+  const cudaError_t e = io_dtype == B200_F16
+                            ? launch_ln_stats<__half>(ln.stats_out, ln.stats_out_ld, slices, slice_cols, N, eps, M, stats_out, ext_out, stream)
+                            : launch_ln_stats<__nv_bfloat16>(ln.stats_out, ln.stats_out_ld, slices, slice_cols, N, eps, M, stats_out, ext_out, stream);
   note_launches(1);
   return status_from_cuda(e);
 }

@@ -188,13 +188,25 @@ struct EpilogueArgs {
   int64_t sq_out_ld;
 };
 
+// Sums of squares of a row's slices, added as eight partial sums (slice i joins partial i % 8) and then pairwise: the loads of
+// a row are independent of each other, and a kernel that gives a row to several threads gets the same bits.
+constexpr int kSumsqParts = 8;
+__device__ __forceinline__ float merge_sumsq_parts(const float (&p)[kSumsqParts]) {
+  return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+}
 template <typename OutT>
 __device__ __forceinline__ float deferred_row_scale(const EpilogueArgs<OutT>& e, int64_t row) {
   if (!e.sq_in) return e.out_scale;
-  float s = 0.f;
-#pragma unroll 8
-  for (int i = 0; i < e.sq_slices; ++i) s += __ldg(e.sq_in + (int64_t)i * e.sq_in_ld + row);
-  return e.out_scale / sqrtf(s / e.sq_cols + e.eps);
+  float p[kSumsqParts] = {};
+  int i = 0;
+  for (; i + kSumsqParts <= e.sq_slices; i += kSumsqParts) {
+#pragma unroll
+    for (int j = 0; j < kSumsqParts; ++j) p[j] += __ldg(e.sq_in + (int64_t)(i + j) * e.sq_in_ld + row);
+  }
+#pragma unroll
+  for (int j = 0; j < kSumsqParts - 1; ++j)
+    if (i + j < e.sq_slices) p[j] += __ldg(e.sq_in + (int64_t)(i + j) * e.sq_in_ld + row);
+  return e.out_scale / sqrtf(merge_sumsq_parts(p) / e.sq_cols + e.eps);
 }
 
 // Shifted sums of one thread's part of an output row (LN == 2): sum and sum of squares of (value - shift), the shift
@@ -293,47 +305,49 @@ __device__ __forceinline__ float activate(float v, int act, float param) {
   }
   return v;
 }
-// The activation of 32 consecutive columns; which one is (almost always) uniform over the chunk.
-__device__ __forceinline__ void activate_chunk(float (&f)[32], int col0, int act_lo, int act_hi, int64_t split, float param) {
-  const bool low = col0 + 32 <= split;
+// The activation of CW consecutive columns; which one is (almost always) uniform over the chunk.
+template <int CW>
+__device__ __forceinline__ void activate_chunk(float (&f)[CW], int col0, int act_lo, int act_hi, int64_t split, float param) {
+  const bool low = col0 + CW <= split;
   if (low || col0 >= split) {
     switch (low ? act_lo : act_hi) {
       case B200_ACT_SILU:
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] *= sigmoid_fast(f[j]);
+        for (int j = 0; j < CW; ++j) f[j] *= sigmoid_fast(f[j]);
         break;
       case B200_ACT_SIGMOID:
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = sigmoid_fast(f[j]);
+        for (int j = 0; j < CW; ++j) f[j] = sigmoid_fast(f[j]);
         break;
       case B200_ACT_GELU_TANH:
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = gelu_fast(f[j]);
+        for (int j = 0; j < CW; ++j) f[j] = gelu_fast(f[j]);
         break;
       case B200_ACT_SOFTCAP: {
         const float k = 2.8853900817779268f / param;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = softcap_fast(f[j], param, k);
+        for (int j = 0; j < CW; ++j) f[j] = softcap_fast(f[j], param, k);
         break;
       }
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = activate(f[j], col0 + j < split ? act_lo : act_hi, param);
+    for (int j = 0; j < CW; ++j) f[j] = activate(f[j], col0 + j < split ? act_lo : act_hi, param);
   }
 }
 
-// f += the fp32 bias of columns col0 .. col0 + 31 (the same addresses for the whole warp).
-__device__ __forceinline__ void add_bias_chunk(float (&f)[32], const float* bias, int col0, int64_t N) {
-  if (col0 + 32 <= N) {
+// f += the fp32 bias of columns col0 .. col0 + CW - 1 (the same addresses for the whole warp).
+template <int CW>
+__device__ __forceinline__ void add_bias_chunk(float (&f)[CW], const float* bias, int col0, int64_t N) {
+  if (col0 + CW <= N) {
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
+    for (int j = 0; j < CW; j += 4) {
       const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col0 + j));
       f[j] += b.x, f[j + 1] += b.y, f[j + 2] += b.z, f[j + 3] += b.w;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
+    for (int j = 0; j < CW; ++j)
       if (col0 + j < N) f[j] += __ldg(bias + col0 + j);
   }
 }
@@ -414,18 +428,18 @@ __device__ __forceinline__ void ld_global_v8(const void* p, uint32_t (&v)[8]) {
                : "memory");
 }
 
-// LN == 4, one thread, one row, 32 consecutive columns: x += row_scale * acc in fp32, optionally gx = 16-bit(gain * x)
+// LN == 4, one thread, one row, CW consecutive columns: x += row_scale * acc in fp32, optionally gx = 16-bit(gain * x)
 // and the running sum of squares of the new x.  `wide`: x and gx rows may be accessed 32 bytes at a time.
-template <typename OutT>
-__device__ __forceinline__ void residual_chunk(const uint32_t (&acc)[32], const EpilogueArgs<OutT>& e, int64_t row, int col0, int64_t N, bool wide,
+template <int CW, typename OutT>
+__device__ __forceinline__ void residual_chunk(const uint32_t (&acc)[CW], const EpilogueArgs<OutT>& e, int64_t row, int col0, int64_t N, bool wide,
                                                float row_scale, float& sq) {
   float* xrow = e.x + row * e.ld_x + col0;
-  if (wide && col0 + 32 <= N) {
-    uint32_t r[4][8];
+  if (wide && col0 + CW <= N) {
+    uint32_t r[CW / 8][8];
 #pragma unroll
-    for (int g = 0; g < 4; ++g) ld_global_v8(xrow + 8 * g, r[g]);
+    for (int g = 0; g < CW / 8; ++g) ld_global_v8(xrow + 8 * g, r[g]);
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {
+    for (int g = 0; g < CW / 8; ++g) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float v = fmaf(row_scale, __uint_as_float(acc[g * 8 + j]), __uint_as_float(r[g][j]));
@@ -435,9 +449,9 @@ __device__ __forceinline__ void residual_chunk(const uint32_t (&acc)[32], const 
       st_global_v8(xrow + 8 * g, r[g]);
     }
     if (e.gain) {
-      uint32_t w[16];
+      uint32_t w[CW / 2];
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
+      for (int g = 0; g < CW / 4; ++g) {
         const float4 gn = __ldg(reinterpret_cast<const float4*>(e.gain + col0) + g);
         const uint32_t* rr = &r[g >> 1][(g & 1) * 4];
         __nv_bfloat162 lo = __floats2bfloat162_rn(__uint_as_float(rr[0]) * gn.x, __uint_as_float(rr[1]) * gn.y);
@@ -446,13 +460,13 @@ __device__ __forceinline__ void residual_chunk(const uint32_t (&acc)[32], const 
         w[2 * g + 1] = *reinterpret_cast<uint32_t*>(&hi);
       }
       __nv_bfloat16* grow = e.gx + row * e.ld_gx + col0;
-      st_global_v8(grow, reinterpret_cast<const uint32_t(&)[8]>(w[0]));
-      st_global_v8(grow + 16, reinterpret_cast<const uint32_t(&)[8]>(w[8]));
+#pragma unroll
+      for (int g = 0; g < CW / 16; ++g) st_global_v8(grow + 16 * g, reinterpret_cast<const uint32_t(&)[8]>(w[8 * g]));
     }
     return;
   }
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < CW; ++j) {
     if (col0 + j < N) {
       const float v = fmaf(row_scale, __uint_as_float(acc[j]), xrow[j]);
       xrow[j] = v;
@@ -514,23 +528,23 @@ __device__ __forceinline__ void gated_pair_chunk(const uint32_t (&za)[32], const
   }
 }
 
-// One thread, one row, 32 consecutive columns starting at col0: acc (+bias) -> GELU -> (+residual) -> out.
-// `bias_s` points at this chunk's 32 fp32 bias values in shared memory (zeros when there is no bias).
+// One thread, one row, CW consecutive columns (staged stores: 32) starting at col0: acc (+bias) -> GELU -> (+residual) -> out.
+// `bias_s` points at this chunk's fp32 bias values in shared memory (zeros when there is no bias).
 // With `stage` != 0 (TMA-store path, 16-bit output) the 64 result bytes go to this thread's row of the warp's
 // staging tile at 16-byte slots [4*half, 4*half+4) (128-byte swizzle); otherwise they are stored to global memory.
-template <typename OutT, bool GELU, int STATS, int LN>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const float* bias_s, const EpilogueArgs<OutT>& e,
+template <typename OutT, bool GELU, int STATS, int LN, int CW = 32>
+__device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[CW], const float* bias_s, const EpilogueArgs<OutT>& e,
                                                const uint4* res_regs, int64_t row, int col0, int64_t N, int mode, uint32_t stage,
                                                int half, int lane, bool row_ok, bool res_staged, RowStats& st, float ln_r, SliceMoments& mom) {
   // Two columns per instruction where the hardware has packed fp32 forms (add, mul, fma: same roundings as the
   // scalar ones); no bias, no add.
-  float f[32];
+  float f[CW];
   if constexpr (LN == 1 || LN == 3) {
     // folded LayerNorm: the extension k-block already put -mean * colsum + ln_bias / rstd into the accumulator
     // (deferred RMS norm: the row scale is all there is)
     const float2 r2 = make_float2(ln_r, ln_r);
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
+    for (int j = 0; j < CW; j += 2) {
       const float2 v2 = __fmul2_rn(make_float2(__uint_as_float(acc[j]), __uint_as_float(acc[j + 1])), r2);
       f[j] = v2.x, f[j + 1] = v2.y;
     }
@@ -540,7 +554,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
     }
   } else if (e.bias) {
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
+    for (int j = 0; j < CW; j += 4) {
       const float4 b = *reinterpret_cast<const float4*>(bias_s + j);
       const float2 lo = __fadd2_rn(make_float2(__uint_as_float(acc[j]), __uint_as_float(acc[j + 1])), make_float2(b.x, b.y));
       const float2 hi = __fadd2_rn(make_float2(__uint_as_float(acc[j + 2]), __uint_as_float(acc[j + 3])), make_float2(b.z, b.w));
@@ -548,21 +562,21 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(acc[j]);
+    for (int j = 0; j < CW; ++j) f[j] = __uint_as_float(acc[j]);
   }
   if (GELU) {
     if constexpr (sizeof(OutT) == 2) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
+      for (int j = 0; j < CW; j += 2) {
         const float2 g = gelu_tanh_approx2(make_float2(f[j], f[j + 1]));
         f[j] = g.x, f[j + 1] = g.y;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = gelu_fast(f[j]);
+      for (int j = 0; j < CW; ++j) f[j] = gelu_fast(f[j]);
     }
   }
-  const bool full = col0 + 32 <= N;
+  const bool full = col0 + CW <= N;
   if constexpr (sizeof(OutT) == 2) {
     if (stage != 0 || (mode != STORE_SCALAR && full)) {
       if (res_staged) {
@@ -570,7 +584,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
         const uint32_t rowaddr = stage + (uint32_t)lane * 128u;
         const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        for (int g = 0; g < CW / 8; ++g) {
           uint32_t rw[4];
           ld_shared_v4(rowaddr + ((((uint32_t)(half * 4 + g)) ^ sw) << 4), rw);
 #pragma unroll
@@ -582,7 +596,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
         }
       } else if (res_regs) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
+        for (int g = 0; g < CW / 8; ++g) {
           const uint32_t* rw = reinterpret_cast<const uint32_t*>(&res_regs[g]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -595,7 +609,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
         // ragged last column chunk on the staged path: element-wise, inside the matrix only
         const OutT* rrow = e.residual + row * e.ld_res + col0;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < CW; ++j)
           if (col0 + j < N) f[j] += to_float(rrow[j]);
       }
       if constexpr (LN == 2) {
@@ -605,15 +619,15 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
         if (full) {
           float2 a1 = make_float2(0.f, 0.f), a2 = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
+          for (int j = 0; j < CW; j += 2) {
             const float2 d = __fadd2_rn(make_float2(f[j], f[j + 1]), sh);
             a1 = __fadd2_rn(a1, d);
             a2 = __ffma2_rn(d, d, a2);
           }
-          mom.s1 += a1.x + a1.y, mom.s2 += a2.x + a2.y, mom.n += 32.f;
+          mom.s1 += a1.x + a1.y, mom.s2 += a2.x + a2.y, mom.n += (float)CW;
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
+          for (int j = 0; j < CW; ++j) {
             if (col0 + j < N) {
               const float d = f[j] - mom.shift;
               mom.s1 += d, mom.s2 = fmaf(d, d, mom.s2), mom.n += 1.f;
@@ -621,9 +635,9 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
           }
         }
       }
-      uint32_t w[16];
+      uint32_t w[CW / 2];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = pack2<OutT>(f[2 * j], f[2 * j + 1]);
+      for (int j = 0; j < CW / 2; ++j) w[j] = pack2<OutT>(f[2 * j], f[2 * j + 1]);
       if constexpr (STATS) {
         // compare what is stored (the rounded values); strict '>' keeps the lowest column among equal maxima
         const float m_old = st.best_val;
@@ -632,13 +646,13 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
           // tile, in the staging tile (find_staged_column), and only for the chunk that won
           uint32_t m = w[0];
 #pragma unroll
-          for (int j = 1; j < 16; ++j) m = max2<OutT>(m, w[j]);
+          for (int j = 1; j < CW / 2; ++j) m = max2<OutT>(m, w[j]);
           const float2 mm = unpack2<OutT>(m);
           const float cm = fmaxf(mm.x, mm.y);
           if (cm > st.best_val) st.best_val = cm, st.pending_col0 = col0;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < CW / 2; ++j) {
             const float2 r = unpack2<OutT>(w[j]);
             if (col0 + 2 * j < N && r.x > st.best_val) st.best_val = r.x, st.best_idx = col0 + 2 * j, st.pending_col0 = -1;
             if (col0 + 2 * j + 1 < N && r.y > st.best_val) st.best_val = r.y, st.best_idx = col0 + 2 * j + 1, st.pending_col0 = -1;
@@ -650,7 +664,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
           const float m2 = st.best_val * kLog2e;
           float acc_sum = st.sumexp * ex2_approx(m_old * kLog2e - m2);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < CW / 2; ++j) {
             const float2 r = unpack2<OutT>(w[j]);
             if (col0 + 2 * j < N) acc_sum += ex2_approx(fmaf(r.x, kLog2e, -m2));
             if (col0 + 2 * j + 1 < N) acc_sum += ex2_approx(fmaf(r.y, kLog2e, -m2));
@@ -662,15 +676,15 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
         const uint32_t rowaddr = stage + (uint32_t)lane * 128u;
         const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll
-        for (int g = 0; g < 4; ++g) st_shared_v4(rowaddr + ((((uint32_t)(half * 4 + g)) ^ sw) << 4), w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+        for (int g = 0; g < CW / 8; ++g) st_shared_v4(rowaddr + ((((uint32_t)(half * 4 + g)) ^ sw) << 4), w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
       } else {
         OutT* orow = e.out + row * e.ld_out + col0;
         if (mode == STORE_32B) {
-          st_global_v8(orow, reinterpret_cast<const uint32_t(&)[8]>(w[0]));
-          st_global_v8(orow + 16, reinterpret_cast<const uint32_t(&)[8]>(w[8]));
+#pragma unroll
+          for (int g = 0; g < CW / 16; ++g) st_global_v8(orow + 16 * g, reinterpret_cast<const uint32_t(&)[8]>(w[8 * g]));
         } else {
 #pragma unroll
-          for (int g = 0; g < 4; ++g) *reinterpret_cast<uint4*>(orow + g * 8) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+          for (int g = 0; g < CW / 8; ++g) *reinterpret_cast<uint4*>(orow + g * 8) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
         }
       }
       return;
@@ -681,24 +695,24 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
       if (e.residual) {
         const float* rrow = reinterpret_cast<const float*>(e.residual) + row * e.ld_res + col0;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
+        for (int j = 0; j < CW; j += 4) {
           const float4 r = *reinterpret_cast<const float4*>(rrow + j);
           f[j] += r.x, f[j + 1] += r.y, f[j + 2] += r.z, f[j + 3] += r.w;
         }
       }
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(orow + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
+      for (int j = 0; j < CW; j += 4) *reinterpret_cast<float4*>(orow + j) = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
       if constexpr (STATS) {
         const float m_old = st.best_val;
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < CW; ++j)
           if (f[j] > st.best_val) st.best_val = f[j], st.best_idx = col0 + j, st.pending_col0 = -1;
         if (STATS == 2 && st.best_val > -INFINITY) {
           const float kLog2e = 1.4426950408889634f;
           const float m2 = st.best_val * kLog2e;
           float acc_sum = st.sumexp * ex2_approx(m_old * kLog2e - m2);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) acc_sum += ex2_approx(fmaf(f[j], kLog2e, -m2));
+          for (int j = 0; j < CW; ++j) acc_sum += ex2_approx(fmaf(f[j], kLog2e, -m2));
           st.sumexp = acc_sum;
         }
       }
@@ -710,7 +724,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
   const OutT* rrow = e.residual ? e.residual + row * e.ld_res + col0 : nullptr;
   const float m_old = st.best_val;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < CW; ++j) {
     if (col0 + j < N) {
       float v = f[j];
       if (rrow) v += to_float(rrow[j]);
@@ -730,7 +744,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[32], const 
     const float m2 = st.best_val * kLog2e;
     float acc_sum = st.sumexp * ex2_approx(m_old * kLog2e - m2);
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
+    for (int j = 0; j < CW; ++j)
       if (col0 + j < N) acc_sum += ex2_approx(fmaf(f[j], kLog2e, -m2));
     st.sumexp = acc_sum;
   }
@@ -1393,6 +1407,270 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
 }
 
+// ------------------------------------------------------------------ at most 64 rows
+// A product of a few rows is the read of its weights: 2 N K bytes against a handful of rows.  gemm_narrow_kernel spent 10-35 us
+// on what HBM delivers in 1-5 because (1) 64 columns a CTA left most SMs without weights to read (N = 768: 12 CTAs, N = 2048:
+// 32), (2) every k-block moved 128 rows of A, nearly all of them zero fill, and (3) nothing started before the kernel in front
+// had ended.  Here a CTA computes NB = 16, 32 or 64 columns (as few as it takes to spread N over the GPU: few_rows_cols), A
+// tiles have 16, 32 or 64 rows, stages hold two k-blocks, two CTAs fit an SM, and what does not depend on the kernel in front
+// runs ahead of griddepcontrol.wait: set-up, descriptors, and the CTA's weights as an L2 prefetch (L2 is where writes of other
+// SMs meet as well, so this is right whoever wrote the weights, and when).  The MMA is M = 64: its unused rows read whatever
+// follows the tile in shared memory (the next tiles, inside this CTA's allocation) and nobody reads their accumulators.
+// k-blocks run in the same order with the same arithmetic as in the other two kernels: the same bits.
+// LN == 4 keeps its sums of squares per 64 columns: the four CTAs of 16 columns form a cluster and meet in the first one.
+// Measured, us per launch in a replayed graph of such launches on weights that are not in L2, 16 rows, before -> now (HBM alone):
+// 2048 x 2048 12.2 -> 8.9 (1.3), 2048 x 8192 (N x K) 35.9 -> 29.9 (5.1), 10880 x 2048 26.4 -> 12.8 (6.8), 32768 x 2048 59 -> 28.4
+// (20.5), 768 x 768 6.0 -> 4.4.
+constexpr int kFewMaxRows = 64;
+constexpr int FEW_THREADS = 192;
+constexpr int FEW_MAX_STAGES = 16;
+constexpr int FEW_CTRL_BYTES = 512;
+constexpr int FEW_TAIL_BYTES = FEW_CTRL_BYTES + NARROW_BN * 4 + (kSumsqParts + 4) * kFewMaxRows * 4;  // control, bias, row sums in and out
+constexpr int FEW_SMEM_BUDGET = 104 * 1024;                                                      // two CTAs per SM
+constexpr int FEW_PREFETCH_BYTES = 192 * 1024;                                                   // of weights, per CTA
+
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* map, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void prefetch_descriptor(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+        "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+template <int CW>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&v)[CW]) {
+  if constexpr (CW == 16) tmem_ld_32x16(taddr, v);
+  else tmem_ld_32x32(taddr, v);
+}
+
+template <typename OutT, bool GELU, int LN, int NB>
+__global__ void __launch_bounds__(FEW_THREADS, 2)
+gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a_ext,
+                const __grid_constant__ CUtensorMap map_b_ext, EpilogueArgs<OutT> epi, int M, int64_t N, int64_t K, int a_rows, int stages, uint32_t idesc,
+                int* status_word) {
+  static_assert(sizeof(OutT) == 2 || LN >= 3, "fp32 outputs exist behind a deferred RMS norm only");
+  static_assert(LN != 5 || NB == 64, "one block of gate and up columns per tile");
+  static_assert(LN != 4 || NB * 4 == NARROW_BN, "a cluster of four shares a slice of the sums of squares");
+  constexpr int CW = NB < 32 ? NB : 32;  // columns per epilogue step
+  constexpr int esz = (int)sizeof(OutT);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t base = smem_u32(smem);
+  const uint32_t a_block = (uint32_t)a_rows * 128u, b_block = (uint32_t)NB * 128u;  // bytes of a k-block's tiles
+  const uint32_t smem_a = base, smem_b = base + (uint32_t)stages * 2u * a_block;
+  uint8_t* ctrl = smem + (uint32_t)stages * 2u * (a_block + b_block);
+  const uint32_t bar_full = smem_u32(ctrl), bar_empty = bar_full + 8 * FEW_MAX_STAGES, bar_acc = bar_empty + 8 * FEW_MAX_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 16 * FEW_MAX_STAGES + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 16 * FEW_MAX_STAGES + 16);
+  static_assert(16 * FEW_MAX_STAGES + 24 <= FEW_CTRL_BYTES, "control block too small");
+  float* bias_s = reinterpret_cast<float*>(ctrl + FEW_CTRL_BYTES);
+  float* parts_s = bias_s + NARROW_BN;  // [kSumsqParts][kFewMaxRows]
+  float* sums_s = parts_s + kSumsqParts * kFewMaxRows;  // LN == 4, first CTA of the cluster: [4][kFewMaxRows]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.x * NB;
+  const int num_kb_ab = n0 < N ? (int)((K + BK - 1) / BK) : 0;  // (the last cluster of LN == 4 may have CTAs without columns)
+  const int num_kb = num_kb_ab + (LN == 1 ? 1 : 0);
+  if (warp == 0 && lane == 0) {
+    prefetch_descriptor(&map_a);
+    prefetch_descriptor(&map_b);
+    const int ahead = min(num_kb_ab, FEW_PREFETCH_BYTES / (NB * 128));
+    for (int kb = 0; kb < ahead; ++kb) tma_prefetch_l2_2d(&map_b, kb * BK, n0);
+  }
+  if (threadIdx.x == 32) {
+    for (int i = 0; i < stages; ++i) {
+      mbar_init(bar_full + 8 * i, 1);
+      mbar_init(bar_empty + 8 * i, 1);
+    }
+    mbar_init(bar_acc, 1);
+    *abort_flag = (base & 1023u) ? 1 : 0;  // (never expected: swizzled tiles need 1024-byte aligned bases)
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async_smem();
+  }
+  constexpr uint32_t TMEM = NB < 32 ? 32 : NB;
+  if (warp == 2) {
+    tmem_alloc(smem_u32(tmem_slot), TMEM);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if constexpr (LN == 4) cluster_sync_all();  // the first CTA's shared memory exists before the others write to it
+  tc_fence_after();
+  const uint32_t tmem_d = *tmem_slot;
+  pdl_launch_dependents();
+  pdl_wait();
+  const bool misplaced = (base & 1023u) != 0;
+  if (misplaced && threadIdx.x == 0 && status_word) atomicCAS(status_word, 0, 99);
+
+  if (misplaced) {
+  } else if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < num_kb; kb += 2) {
+        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status_word, 31)) break;
+        const int blocks = min(2, num_kb - kb);
+        mbar_arrive_expect_tx(bar_full + 8 * stage, (uint32_t)blocks * (a_block + b_block));
+        for (int j = 0; j < blocks; ++j) {
+          const bool ext = LN == 1 && kb + j == num_kb_ab;
+          const int col = ext ? 0 : (kb + j) * BK;
+          tma_load_2d(smem_a + (uint32_t)(2 * stage + j) * a_block, ext ? &map_a_ext : &map_a, bar_full + 8 * stage, col, 0);
+          tma_load_2d(smem_b + (uint32_t)(2 * stage + j) * b_block, ext ? &map_b_ext : &map_b, bar_full + 8 * stage, col, n0);
+        }
+        if (++stage == stages) stage = 0, phase ^= 1u;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool alive = true;
+      for (int kb = 0; kb < num_kb; kb += 2) {
+        if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, status_word, 32)) {
+          alive = false;
+          break;
+        }
+        tc_fence_after();
+        const int blocks = min(2, num_kb - kb);
+        for (int j = 0; j < blocks; ++j) {
+          const uint64_t da = make_smem_desc(smem_a + (uint32_t)(2 * stage + j) * a_block);
+          const uint64_t db = make_smem_desc(smem_b + (uint32_t)(2 * stage + j) * b_block);
+          const int k_steps = (LN == 1 && kb + j == num_kb_ab) ? 1 : BK / UMMA_K;  // (the extension block: 8 non-zero columns)
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            if (k >= k_steps) break;
+            umma_f16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (uint32_t)((kb | j | k) != 0));
+          }
+        }
+        umma_commit(bar_empty + 8 * stage);
+        if (++stage == stages) stage = 0, phase ^= 1u;
+      }
+      if (alive) umma_commit(bar_acc);
+    }
+  } else {
+    // Epilogue.  The accumulator rows of an M = 64 MMA sit in the first 16 lanes of each quarter of tensor memory.
+    const int quarter = warp & 3;
+    const int row_i = quarter * 16 + (lane & 15);
+    const int64_t row = row_i;
+    const bool row_ok = lane < 16 && row_i < M;
+    const int epi_tid = threadIdx.x - 64;
+    if constexpr (LN == 0 || LN == 2) {
+      if (epi_tid < NB) bias_s[epi_tid] = (epi.bias && n0 + epi_tid < N) ? to_float(epi.bias[n0 + epi_tid]) : 0.f;
+    }
+    if constexpr (LN >= 3) {
+      // all 128 threads add up the rows' slices (the order of deferred_row_scale): thread -> (row, every 128 / a_rows-th partial)
+      if (epi.sq_in) {
+        const int r = epi_tid % a_rows;
+        for (int part = epi_tid / a_rows; part < kSumsqParts; part += 128 / a_rows) {
+          float s = 0.f;
+          if (r < M) {
+#pragma unroll 4
+            for (int i = part; i < epi.sq_slices; i += kSumsqParts) s += __ldg(epi.sq_in + (int64_t)i * epi.sq_in_ld + r);
+          }
+          parts_s[part * kFewMaxRows + r] = s;
+        }
+      }
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
+    float ln_r = 1.f;
+    if constexpr (LN == 1) {
+      if (row_ok) ln_r = __ldg(epi.ln_stats + row).y;
+    }
+    if constexpr (LN >= 3) {
+      ln_r = epi.out_scale;
+      if (epi.sq_in && row_ok) {
+        float p[kSumsqParts];
+#pragma unroll
+        for (int j = 0; j < kSumsqParts; ++j) p[j] = parts_s[j * kFewMaxRows + row_i];
+        ln_r = epi.out_scale / sqrtf(merge_sumsq_parts(p) / epi.sq_cols + epi.eps);
+      }
+    }
+    bool x_wide = false;
+    if constexpr (LN == 4) {
+      x_wide = residual_rows_wide(epi);
+      if (row_ok && n0 < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(epi.x + row * epi.ld_x + n0));
+    }
+    const uintptr_t out_al = reinterpret_cast<uintptr_t>(epi.out) | (uintptr_t)(epi.ld_out * esz);
+    const uintptr_t res_al = epi.residual ? (reinterpret_cast<uintptr_t>(epi.residual) | (uintptr_t)(epi.ld_res * esz)) : 0;
+    const int mode = ((out_al | res_al) & 15) == 0 ? STORE_16B : STORE_SCALAR;
+    // residual of this thread's row, fetched while the main loop runs
+    uint4 res[NB / 8];
+    const bool res_in_regs = esz == 2 && epi.residual && mode != STORE_SCALAR && row_ok;
+    if (res_in_regs) {
+      const OutT* rrow = epi.residual + row * epi.ld_res + n0;
+#pragma unroll
+      for (int i = 0; i < NB / 8; ++i)
+        if (n0 + (i / (CW / 8)) * CW + CW <= N) res[i] = *reinterpret_cast<const uint4*>(rrow + i * 8);
+    }
+    SliceMoments mom{0.f, 0.f, 0.f, 0.f};
+    if (num_kb > 0 && mbar_wait(bar_acc, 0, abort_flag, status_word, 33)) {
+      tc_fence_after();
+      RowStats unused{-INFINITY, 0, 0.f, -1};
+      const uint32_t at = tmem_d + ((uint32_t)(quarter * 32) << 16);
+      if constexpr (LN == 5) {
+        uint32_t za[32], zb[32];
+        tmem_ld_32x32(at, za);
+        tmem_ld_32x32(at + 32u, zb);
+        tmem_ld_wait();
+        if (row_ok) gated_pair_chunk(za, zb, epi, row, n0, ln_r, 0u, 0, lane, mode != STORE_SCALAR);
+      } else {
+#pragma unroll
+        for (int c = 0; c < NB / CW; ++c) {
+          const int col0 = n0 + c * CW;
+          if (col0 >= N) break;  // (warp-uniform)
+          uint32_t v[CW];
+          tmem_ld_cols<CW>(at + (uint32_t)(c * CW), v);
+          tmem_ld_wait();
+          if constexpr (LN == 4) {
+            if (row_ok) residual_chunk(v, epi, row, col0, N, x_wide, ln_r, mom.s2);
+          } else if (row_ok) {
+            epilogue_chunk<OutT, GELU, 0, LN, CW>(v, bias_s + c * CW, epi, (res_in_regs && col0 + CW <= N) ? &res[c * (CW / 8)] : nullptr, row, col0, N, mode, 0u,
+                                                  0, lane, row_ok, false, unused, ln_r, mom);
+          }
+        }
+      }
+      if constexpr (LN == 2) {
+        if (row_ok && mom.n > 0.f) {
+          const float inv = 1.0f / mom.n;
+          epi.stats_out[(int64_t)blockIdx.x * epi.stats_out_ld + row] = make_float2(fmaf(mom.s1, inv, mom.shift), fmaxf(mom.s2 - mom.s1 * mom.s1 * inv, 0.f));
+        }
+      }
+    }
+    if constexpr (LN == 4) {
+      if (row_ok && epi.gain) {
+        const uint32_t rank = cluster_ctarank();
+        const uint32_t to = mapa_shared(smem_u32(sums_s + rank * kFewMaxRows + row_i), 0);
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(mom.s2) : "memory");
+      }
+    }
+  }
+
+  if constexpr (LN == 4) {
+    __syncwarp();
+    cluster_sync_all();  // the four sums of every row are in the first CTA
+    const int r = (int)threadIdx.x;
+    if (epi.gain && (blockIdx.x & 3) == 0 && r < M && r < kFewMaxRows)
+      epi.sq_out[(int64_t)(blockIdx.x >> 2) * epi.sq_out_ld + r] =
+          (sums_s[r] + sums_s[kFewMaxRows + r]) + (sums_s[2 * kFewMaxRows + r] + sums_s[3 * kFewMaxRows + r]);
+  }
+  // ------------------------------------------------------------ teardown
+  __syncwarp();
+  if (*abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc(tmem_d, TMEM);
+  }
+}
+
 // ------------------------------------------------------------------ host side
 // 2-D map over a row-major [rows, cols] 16-bit matrix with leading dimension ld; box = 64 columns x box_rows.
 static int make_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int64_t ld, int box_rows, int op_dtype) {
@@ -1469,12 +1747,76 @@ static constexpr uint32_t make_idesc_narrow(int ab_format) {
   return (1u << 4) | ((uint32_t)ab_format << 7) | ((uint32_t)ab_format << 10) | ((uint32_t)(NARROW_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
+// Columns per CTA: as many as leave one CTA per SM (148), and at least 16, the narrowest tile of an MMA that also holds a
+// 32-byte store.  LN == 4: 16 (four CTAs share a 64-column slice); LN == 5: 64 (one block of gate and up columns).
+inline int few_rows_cols(int64_t N, int ln) {
+  if (ln == 4) return 16;
+  if (ln == 5 || N > 64 * 120) return 64;
+  return N > 32 * 120 ? 32 : 16;
+}
+
+template <typename OutT, bool GELU, int LN, int NB>
+static int launch_few_cols(const void* a, const void* b, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                           int op_dtype, const LnArgs& ln, int* status_word, cudaStream_t stream) {
+  static std::atomic<bool> attr_set[kMaxDevices];
+  const int slot = device_slot();
+  if (slot < 0) return B200_ERR_CUDA;
+  if (!attr_set[slot].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(gemm_few_kernel<OutT, GELU, LN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM_BUDGET) != cudaSuccess)
+      return B200_ERR_CUDA;
+    attr_set[slot].store(true, std::memory_order_release);
+  }
+  const int a_rows = M <= 16 ? 16 : M <= 32 ? 32 : 64;
+  const int num_kb = (int)((K + BK - 1) / BK) + (LN == 1 ? 1 : 0);
+  const int stage_bytes = 2 * (a_rows + NB) * BK * 2;
+  int stages = (FEW_SMEM_BUDGET - FEW_TAIL_BYTES) / stage_bytes;
+  if (stages > FEW_MAX_STAGES) stages = FEW_MAX_STAGES;
+  if (stages > (num_kb + 1) / 2) stages = (num_kb + 1) / 2;
+  if (stages < 2) stages = 2;  // an MMA reads 64 rows from a tile's base: what lies behind the last A tile has to be inside the ring of B
+  static_assert(2 * 2 * NB * BK * 2 >= (kFewMaxRows - 16) * BK * 2, "the B ring is shorter than what an MMA reads behind the A ring");
+  CUtensorMap ma, mb, mae, mbe;
+  memset(&mae, 0, sizeof(mae));
+  memset(&mbe, 0, sizeof(mbe));
+  int st = make_map(&ma, a, M, K, lda, a_rows, op_dtype);
+  if (st == B200_OK) st = make_map(&mb, b, N, K, ldb, NB, op_dtype);
+  if (st == B200_OK && LN == 1) st = make_map(&mae, ln.a_ext, M, kLnExtCols, kLnExtCols, a_rows, op_dtype);
+  if (st == B200_OK && LN == 1) st = make_map(&mbe, ln.b_ext, N, kLnExtCols, kLnExtCols, NB, op_dtype);
+  if (st != B200_OK) return st;
+  constexpr int cluster = LN == 4 ? 4 : 1;
+  const unsigned ctas = (unsigned)((N + NB * cluster - 1) / (NB * cluster) * cluster);
+  const uint32_t idesc = (1u << 4) | ((op_dtype == B200_BF16 ? 1u : 0u) << 7) | ((op_dtype == B200_BF16 ? 1u : 0u) << 10) | ((uint32_t)(NB >> 3) << 17) |
+                         ((uint32_t)(kFewMaxRows >> 4) << 24);
+  LaunchSetup ls(dim3(ctas), dim3(FEW_THREADS), (size_t)(stages * stage_bytes + FEW_TAIL_BYTES), stream, cluster, true);
+  const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, gemm_few_kernel<OutT, GELU, LN, NB>, ma, mb, mae, mbe, epi, (int)M, N, K, a_rows, stages, idesc, status_word);
+  note_launches(1);
+  return status_from_cuda(e);
+}
+
+template <typename OutT, bool GELU, int LN>
+static int launch_few(const void* a, const void* b, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int op_dtype,
+                      const LnArgs& ln, int* status_word, cudaStream_t stream) {
+  if constexpr (sizeof(OutT) != 2 && LN < 3) {
+    return B200_ERR_UNSUPPORTED;
+  } else if constexpr (LN == 4) {
+    return launch_few_cols<OutT, GELU, LN, 16>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+  } else if constexpr (LN == 5) {
+    return launch_few_cols<OutT, GELU, LN, 64>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+  } else {
+    switch (few_rows_cols(N, LN)) {
+      case 16: return launch_few_cols<OutT, GELU, LN, 16>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+      case 32: return launch_few_cols<OutT, GELU, LN, 32>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+      default: return launch_few_cols<OutT, GELU, LN, 64>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+    }
+  }
+}
+
 template <typename OutT, bool GELU, int LN>
 static int launch_narrow(const void* a, const void* b, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                          int op_dtype, const LnArgs& ln, int* status_word, cudaStream_t stream) {
   if constexpr (sizeof(OutT) != 2 && LN < 3) {
     return B200_ERR_UNSUPPORTED;
   } else {
+    if (M <= kFewMaxRows) return launch_few<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
     static std::atomic<bool> attr_set[kMaxDevices];
     const int slot = device_slot();
     if (slot < 0) return B200_ERR_CUDA;
@@ -1491,7 +1833,7 @@ static int launch_narrow(const void* a, const void* b, const EpilogueArgs<OutT>&
     if (st == B200_OK && LN == 1) st = make_map(&mae, ln.a_ext, M, kLnExtCols, kLnExtCols, BM, op_dtype);
     if (st == B200_OK && LN == 1) st = make_map(&mbe, ln.b_ext, N, kLnExtCols, kLnExtCols, NARROW_BN, op_dtype);
     if (st != B200_OK) return st;
-    LaunchSetup ls(dim3((unsigned)((N + NARROW_BN - 1) / NARROW_BN), (unsigned)((M + BM - 1) / BM)), dim3(NARROW_THREADS), NARROW_SMEM_BYTES, stream);
+    LaunchSetup ls(dim3((unsigned)((N + NARROW_BN - 1) / NARROW_BN), (unsigned)((M + BM - 1) / BM)), dim3(NARROW_THREADS), NARROW_SMEM_BYTES, stream, 1, true);
     const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, gemm_narrow_kernel<OutT, GELU, LN>, ma, mb, mae, mbe, epi, M, N, K,
                                              make_idesc_narrow(op_dtype == B200_BF16 ? 1 : 0), status_word);
     note_launches(1);
