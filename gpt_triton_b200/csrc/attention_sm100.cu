@@ -126,7 +126,7 @@ attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + BAR_BYTES + 8);
   float* xchg = reinterpret_cast<float*>(ctrl + CTRL_BYTES);  // [2][128]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qt = (p.L + BLOCK_M - 1) / BLOCK_M;
   const int bh_total = p.B * p.NH;
   const int64_t n_items = (int64_t)n_qt * bh_total;
@@ -165,7 +165,7 @@ attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t qi = 0, ki = 0;
       bool alive = true;
       for (int64_t idx = blockIdx.x; idx < n_items && alive; idx += gridDim.x) {
@@ -197,7 +197,7 @@ attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t qi = 0, ks = 0, kp = 0, si = 0, pi = 0;
       bool alive = true;
       // S_next = Q . K^T into S[si & 1]: needs the block's K/V stage and that buffer's previous scores to be in registers

@@ -238,7 +238,7 @@ int launch_gemm_ln(const void* a, const void* b, const void* bias, const void* r
   // narrow tile NARROW_BN, a tile of at most 64 rows few_rows_cols
   const bool narrow = io_dtype == B200_F16 ? takes_narrow_tiles<__half, 0>(M, out, ld_out, residual, ld_res)
                                            : takes_narrow_tiles<__nv_bfloat16, 0>(M, out, ld_out, residual, ld_res);
-  const int slice_cols = !narrow ? EPI_COLS : M <= kFewMaxRows ? few_rows_cols(N, 2) : NARROW_BN;
+  const int slice_cols = !narrow ? EPI_COLS : takes_few_rows(M, N, 2) ? few_rows_cols(M, N, 2) : NARROW_BN;
   const int slices = (int)((N + slice_cols - 1) / slice_cols);
   const cudaError_t e = io_dtype == B200_F16
                             ? launch_ln_stats<__half>(ln.stats_out, ln.stats_out_ld, slices, slice_cols, N, eps, M, stats_out, ext_out, stream)

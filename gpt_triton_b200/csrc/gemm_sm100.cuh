@@ -855,7 +855,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 8 * NUM_BARS + 8);
   float* bias_smem = reinterpret_cast<float*>(ctrl + CTRL_BYTES);  // [2][BN]
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = CTAS == 2 ? cluster_ctarank() : 0u;  // 0 = leader (issues the MMAs)
   const int64_t group_id = CTAS == 2 ? (int64_t)(blockIdx.x >> 1) : (int64_t)blockIdx.x;
@@ -903,7 +903,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
@@ -941,7 +941,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader CTA's only, for a pair)
-    if (lane == 0 && cta_rank == 0) {
+    if (cta_rank == 0 && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -1253,7 +1253,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   static_assert(16 * NARROW_STAGES + 24 <= NARROW_CTRL_BYTES, "control block too small");
   float* bias_s = reinterpret_cast<float*>(ctrl + NARROW_CTRL_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * NARROW_BN, m0 = blockIdx.y * BM;
   const int num_kb_ab = (int)((K + BK - 1) / BK);
   const int num_kb = num_kb_ab + (LN == 1 ? 1 : 0);
@@ -1279,7 +1279,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   pdl_wait();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < num_kb; ++kb) {
@@ -1292,7 +1292,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
@@ -1407,23 +1407,28 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
 }
 
-// ------------------------------------------------------------------ at most 64 rows
+// ------------------------------------------------------------------ tiles of 64 rows
 // A product of a few rows is the read of its weights: 2 N K bytes against a handful of rows.  gemm_narrow_kernel spent 10-35 us
 // on what HBM delivers in 1-5 because (1) 64 columns a CTA left most SMs without weights to read (N = 768: 12 CTAs, N = 2048:
 // 32), (2) every k-block moved 128 rows of A, nearly all of them zero fill, and (3) nothing started before the kernel in front
-// had ended.  Here a CTA computes NB = 16, 32 or 64 columns (as few as it takes to spread N over the GPU: few_rows_cols), A
-// tiles have 16, 32 or 64 rows, stages hold two k-blocks, two CTAs fit an SM, and what does not depend on the kernel in front
-// runs ahead of griddepcontrol.wait: set-up, descriptors, and the CTA's weights as an L2 prefetch (L2 is where writes of other
-// SMs meet as well, so this is right whoever wrote the weights, and when).  The MMA is M = 64: its unused rows read whatever
-// follows the tile in shared memory (the next tiles, inside this CTA's allocation) and nobody reads their accumulators.
-// k-blocks run in the same order with the same arithmetic as in the other two kernels: the same bits.
+// had ended.  Here a CTA computes NB = 16, 32 or 64 columns (as few as it takes to spread the product over the GPU: few_rows_cols)
+// of 64 rows, A tiles have 16, 32 or 64 rows, stages hold two k-blocks, two CTAs fit an SM, and what does not depend on the kernel
+// in front runs ahead of griddepcontrol.wait: set-up, descriptors, and the CTA's weights as an L2 prefetch (L2 is where writes of
+// other SMs meet as well, so this is right whoever wrote the weights, and when).  The MMA is M = 64: with fewer rows its unused rows
+// read whatever follows the tile in shared memory (the next tiles, inside this CTA's allocation) and nobody reads their
+// accumulators.  k-blocks run in the same order with the same arithmetic as in the other two kernels: the same bits.
 // LN == 4 keeps its sums of squares per 64 columns: the four CTAs of 16 columns form a cluster and meet in the first one.
-// Measured, us per launch in a replayed graph of such launches on weights that are not in L2, 16 rows, before -> now (HBM alone):
-// 2048 x 2048 12.2 -> 8.9 (1.3), 2048 x 8192 (N x K) 35.9 -> 29.9 (5.1), 10880 x 2048 26.4 -> 12.8 (6.8), 32768 x 2048 59 -> 28.4
-// (20.5), 768 x 768 6.0 -> 4.4.
+// What bounds it: the MMAs of a CTA are one chain, K / 16 of them at 23 clocks (an M = 64, N = 16 MMA is the read of its 64 rows of
+// A from shared memory); K = 768 is 0.6 us of that, K = 8192 6.3.  The issuing thread had needed 65 clocks for each before it
+// ran under elect_one with straight-line code.
+// Measured, us per launch in a replayed graph of such launches on weights that are not in L2, gemm_narrow_kernel -> this kernel
+// (HBM alone), N x K: 16 rows: 2048 x 2048 11.6 -> 5.7 (1.3), 2048 x 8192 35.0 -> 17.1 (5.2), 10880 x 2048 25.2 -> 10.2 (6.9),
+// 768 x 768 5.9 -> 3.1 (0.2), 768 x 3072 15.2 -> 7.5 (0.7).  256 rows (both issuing under elect_one): 768 x 768 4.4 -> 3.6,
+// 768 x 3072 11.7 -> 7.6, 2304 x 768 5.4 -> 4.5, 2048 x 2048 8.7 -> 7.1.
 constexpr int kFewMaxRows = 64;
 constexpr int FEW_THREADS = 192;
 constexpr int FEW_MAX_STAGES = 16;
+constexpr int FEW_GROUP = 2;  // k-blocks per stage
 constexpr int FEW_CTRL_BYTES = 512;
 constexpr int FEW_TAIL_BYTES = FEW_CTRL_BYTES + NARROW_BN * 4 + (kSumsqParts + 4) * kFewMaxRows * 4;  // control, bias, row sums in and out
 constexpr int FEW_SMEM_BUDGET = 104 * 1024;                                                      // two CTAs per SM
@@ -1460,8 +1465,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
   const uint32_t a_block = (uint32_t)a_rows * 128u, b_block = (uint32_t)NB * 128u;  // bytes of a k-block's tiles
-  const uint32_t smem_a = base, smem_b = base + (uint32_t)stages * 2u * a_block;
-  uint8_t* ctrl = smem + (uint32_t)stages * 2u * (a_block + b_block);
+  const uint32_t smem_a = base, smem_b = base + (uint32_t)(stages * FEW_GROUP) * a_block;
+  uint8_t* ctrl = smem + (uint32_t)(stages * FEW_GROUP) * (a_block + b_block);
   const uint32_t bar_full = smem_u32(ctrl), bar_empty = bar_full + 8 * FEW_MAX_STAGES, bar_acc = bar_empty + 8 * FEW_MAX_STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 16 * FEW_MAX_STAGES + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 16 * FEW_MAX_STAGES + 16);
@@ -1470,14 +1475,13 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   float* parts_s = bias_s + NARROW_BN;  // [kSumsqParts][kFewMaxRows]
   float* sums_s = parts_s + kSumsqParts * kFewMaxRows;  // LN == 4, first CTA of the cluster: [4][kFewMaxRows]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = (int)blockIdx.x * NB;
-  const int num_kb_ab = n0 < N ? (int)((K + BK - 1) / BK) : 0;  // (the last cluster of LN == 4 may have CTAs without columns)
-  const int num_kb = num_kb_ab + (LN == 1 ? 1 : 0);
-  if (warp == 0 && lane == 0) {
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int n0 = (int)blockIdx.x * NB, m0 = (int)blockIdx.y * kFewMaxRows;
+  const int num_kb = n0 < N ? (int)((K + BK - 1) / BK) : 0;  // (the last cluster of LN == 4 may have CTAs without columns)
+  if (warp == 0 && elect_one()) {
     prefetch_descriptor(&map_a);
     prefetch_descriptor(&map_b);
-    const int ahead = min(num_kb_ab, FEW_PREFETCH_BYTES / (NB * 128));
+    const int ahead = min(num_kb, FEW_PREFETCH_BYTES / (NB * 128));
     for (int kb = 0; kb < ahead; ++kb) tma_prefetch_l2_2d(&map_b, kb * BK, n0);
   }
   if (threadIdx.x == 32) {
@@ -1507,46 +1511,64 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
   if (misplaced) {
   } else if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < num_kb; kb += 2) {
-        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status_word, 31)) break;
-        const int blocks = min(2, num_kb - kb);
-        mbar_arrive_expect_tx(bar_full + 8 * stage, (uint32_t)blocks * (a_block + b_block));
-        for (int j = 0; j < blocks; ++j) {
-          const bool ext = LN == 1 && kb + j == num_kb_ab;
-          const int col = ext ? 0 : (kb + j) * BK;
-          tma_load_2d(smem_a + (uint32_t)(2 * stage + j) * a_block, ext ? &map_a_ext : &map_a, bar_full + 8 * stage, col, 0);
-          tma_load_2d(smem_b + (uint32_t)(2 * stage + j) * b_block, ext ? &map_b_ext : &map_b, bar_full + 8 * stage, col, n0);
-        }
-        if (++stage == stages) stage = 0, phase ^= 1u;
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool alive = true;
-      for (int kb = 0; kb < num_kb; kb += 2) {
+      for (int kb = 0; kb < num_kb; kb += FEW_GROUP) {
+        if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status_word, 31)) {
+          alive = false;
+          break;
+        }
+        const uint32_t full = bar_full + 8 * stage, at_a = smem_a + (uint32_t)(stage * FEW_GROUP) * a_block, at_b = smem_b + (uint32_t)(stage * FEW_GROUP) * b_block;
+        const int blocks = min(FEW_GROUP, num_kb - kb);
+        mbar_arrive_expect_tx(full, (uint32_t)blocks * (a_block + b_block));
+        for (int j = 0; j < blocks; ++j) {
+          tma_load_2d(at_a + (uint32_t)j * a_block, &map_a, full, (kb + j) * BK, m0);
+          tma_load_2d(at_b + (uint32_t)j * b_block, &map_b, full, (kb + j) * BK, n0);
+        }
+        if (++stage == stages) stage = 0, phase ^= 1u;
+      }
+      if (LN == 1 && alive && mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, status_word, 31)) {
+        // the extension k-block, in a stage of its own
+        mbar_arrive_expect_tx(bar_full + 8 * stage, a_block + b_block);
+        tma_load_2d(smem_a + (uint32_t)(stage * FEW_GROUP) * a_block, &map_a_ext, bar_full + 8 * stage, 0, m0);
+        tma_load_2d(smem_b + (uint32_t)(stage * FEW_GROUP) * b_block, &map_b_ext, bar_full + 8 * stage, 0, n0);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool alive = true;
+      for (int kb = 0; kb < num_kb; kb += FEW_GROUP) {
         if (!mbar_wait(bar_full + 8 * stage, phase, abort_flag, status_word, 32)) {
           alive = false;
           break;
         }
         tc_fence_after();
-        const int blocks = min(2, num_kb - kb);
-        for (int j = 0; j < blocks; ++j) {
-          const uint64_t da = make_smem_desc(smem_a + (uint32_t)(2 * stage + j) * a_block);
-          const uint64_t db = make_smem_desc(smem_b + (uint32_t)(2 * stage + j) * b_block);
-          const int k_steps = (LN == 1 && kb + j == num_kb_ab) ? 1 : BK / UMMA_K;  // (the extension block: 8 non-zero columns)
+        // (straight-line code for a whole stage: an M = 64, N = 16 MMA takes 23 clocks, which leaves the issuing thread few instructions)
+        const uint64_t da = make_smem_desc(smem_a + (uint32_t)(stage * FEW_GROUP) * a_block);
+        const uint64_t db = make_smem_desc(smem_b + (uint32_t)(stage * FEW_GROUP) * b_block);
+        umma_f16(tmem_d, da, db, idesc, (uint32_t)(kb != 0));
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            if (k >= k_steps) break;
-            umma_f16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (uint32_t)((kb | j | k) != 0));
-          }
+        for (int k = 1; k < BK / UMMA_K; ++k) umma_f16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, 1u);
+        if (kb + 1 < num_kb) {
+          const uint64_t da1 = da + (uint64_t)(a_block >> 4), db1 = db + (uint64_t)(b_block >> 4);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) umma_f16(tmem_d, da1 + (uint64_t)(2 * k), db1 + (uint64_t)(2 * k), idesc, 1u);
         }
         umma_commit(bar_empty + 8 * stage);
         if (++stage == stages) stage = 0, phase ^= 1u;
+      }
+      if (LN == 1 && alive) {
+        if (mbar_wait(bar_full + 8 * stage, phase, abort_flag, status_word, 32)) {
+          tc_fence_after();  // (8 non-zero columns: one MMA)
+          umma_f16(tmem_d, make_smem_desc(smem_a + (uint32_t)(stage * FEW_GROUP) * a_block), make_smem_desc(smem_b + (uint32_t)(stage * FEW_GROUP) * b_block), idesc,
+                   (uint32_t)(num_kb != 0));
+        } else {
+          alive = false;
+        }
       }
       if (alive) umma_commit(bar_acc);
     }
@@ -1554,8 +1576,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     // Epilogue.  The accumulator rows of an M = 64 MMA sit in the first 16 lanes of each quarter of tensor memory.
     const int quarter = warp & 3;
     const int row_i = quarter * 16 + (lane & 15);
-    const int64_t row = row_i;
-    const bool row_ok = lane < 16 && row_i < M;
+    const int64_t row = m0 + row_i;
+    const bool row_ok = lane < 16 && row < M;
     const int epi_tid = threadIdx.x - 64;
     if constexpr (LN == 0 || LN == 2) {
       if (epi_tid < NB) bias_s[epi_tid] = (epi.bias && n0 + epi_tid < N) ? to_float(epi.bias[n0 + epi_tid]) : 0.f;
@@ -1566,9 +1588,9 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const int r = epi_tid % a_rows;
         for (int part = epi_tid / a_rows; part < kSumsqParts; part += 128 / a_rows) {
           float s = 0.f;
-          if (r < M) {
+          if (m0 + r < M) {
 #pragma unroll 4
-            for (int i = part; i < epi.sq_slices; i += kSumsqParts) s += __ldg(epi.sq_in + (int64_t)i * epi.sq_in_ld + r);
+            for (int i = part; i < epi.sq_slices; i += kSumsqParts) s += __ldg(epi.sq_in + (int64_t)i * epi.sq_in_ld + m0 + r);
           }
           parts_s[part * kFewMaxRows + r] = s;
         }
@@ -1652,8 +1674,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __syncwarp();
     cluster_sync_all();  // the four sums of every row are in the first CTA
     const int r = (int)threadIdx.x;
-    if (epi.gain && (blockIdx.x & 3) == 0 && r < M && r < kFewMaxRows)
-      epi.sq_out[(int64_t)(blockIdx.x >> 2) * epi.sq_out_ld + r] =
+    if (epi.gain && (blockIdx.x & 3) == 0 && r < kFewMaxRows && m0 + r < M)
+      epi.sq_out[(int64_t)(blockIdx.x >> 2) * epi.sq_out_ld + m0 + r] =
           (sums_s[r] + sums_s[kFewMaxRows + r]) + (sums_s[2 * kFewMaxRows + r] + sums_s[3 * kFewMaxRows + r]);
   }
   // ------------------------------------------------------------ teardown
@@ -1749,10 +1771,23 @@ static constexpr uint32_t make_idesc_narrow(int ab_format) {
 
 // Columns per CTA: as many as leave one CTA per SM (148), and at least 16, the narrowest tile of an MMA that also holds a
 // 32-byte store.  LN == 4: 16 (four CTAs share a 64-column slice); LN == 5: 64 (one block of gate and up columns).
-inline int few_rows_cols(int64_t N, int ln) {
+inline int few_rows_cols(int64_t M, int64_t N, int ln) {
   if (ln == 4) return 16;
-  if (ln == 5 || N > 64 * 120) return 64;
-  return N > 32 * 120 ? 32 : 16;
+  if (ln == 5) return 64;
+  const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows;
+  if (row_tiles == 1 && (N + 63) / 64 > 120) return 64;
+  return (N + 31) / 32 * row_tiles > 120 ? 32 : 16;
+}
+// Whether a product of at most kNarrowMaxRows rows goes to gemm_few_kernel: up to 64 rows always, above that as long as its tiles
+// of 64 rows and 16 or 32 columns fit the GPU at once (two CTAs per SM; the clusters of LN == 4 do not get the last few places).
+// Beyond that its smaller tiles read A and B more often than they help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of
+// gemm_narrow_kernel; LN == 4, 384 rows, 768 x 3072 (288 CTAs): 18.2 against 13.5, 256 rows (192 CTAs): 10.0 against 13.7.
+inline bool takes_few_rows(int64_t M, int64_t N, int ln) {
+  if (M <= kFewMaxRows) return true;
+  if (ln == 5) return false;
+  const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows;
+  const int cols = few_rows_cols(M, N, ln);
+  return (N + cols - 1) / cols * row_tiles <= (ln == 4 ? 256 : 296);
 }
 
 template <typename OutT, bool GELU, int LN, int NB>
@@ -1767,13 +1802,14 @@ static int launch_few_cols(const void* a, const void* b, const EpilogueArgs<OutT
     attr_set[slot].store(true, std::memory_order_release);
   }
   const int a_rows = M <= 16 ? 16 : M <= 32 ? 32 : 64;
-  const int num_kb = (int)((K + BK - 1) / BK) + (LN == 1 ? 1 : 0);
-  const int stage_bytes = 2 * (a_rows + NB) * BK * 2;
+  const int num_kb = (int)((K + BK - 1) / BK);
+  const int stage_bytes = FEW_GROUP * (a_rows + NB) * BK * 2;
   int stages = (FEW_SMEM_BUDGET - FEW_TAIL_BYTES) / stage_bytes;
   if (stages > FEW_MAX_STAGES) stages = FEW_MAX_STAGES;
-  if (stages > (num_kb + 1) / 2) stages = (num_kb + 1) / 2;
+  const int needed = (num_kb + FEW_GROUP - 1) / FEW_GROUP + (LN == 1 ? 1 : 0);
+  if (stages > needed) stages = needed;
   if (stages < 2) stages = 2;  // an MMA reads 64 rows from a tile's base: what lies behind the last A tile has to be inside the ring of B
-  static_assert(2 * 2 * NB * BK * 2 >= (kFewMaxRows - 16) * BK * 2, "the B ring is shorter than what an MMA reads behind the A ring");
+  static_assert(2 * FEW_GROUP * NB * BK * 2 >= (kFewMaxRows - 16) * BK * 2, "the B ring is shorter than what an MMA reads behind the A ring");
   CUtensorMap ma, mb, mae, mbe;
   memset(&mae, 0, sizeof(mae));
   memset(&mbe, 0, sizeof(mbe));
@@ -1786,7 +1822,7 @@ static int launch_few_cols(const void* a, const void* b, const EpilogueArgs<OutT
   const unsigned ctas = (unsigned)((N + NB * cluster - 1) / (NB * cluster) * cluster);
   const uint32_t idesc = (1u << 4) | ((op_dtype == B200_BF16 ? 1u : 0u) << 7) | ((op_dtype == B200_BF16 ? 1u : 0u) << 10) | ((uint32_t)(NB >> 3) << 17) |
                          ((uint32_t)(kFewMaxRows >> 4) << 24);
-  LaunchSetup ls(dim3(ctas), dim3(FEW_THREADS), (size_t)(stages * stage_bytes + FEW_TAIL_BYTES), stream, cluster, true);
+  LaunchSetup ls(dim3(ctas, (unsigned)((M + kFewMaxRows - 1) / kFewMaxRows)), dim3(FEW_THREADS), (size_t)(stages * stage_bytes + FEW_TAIL_BYTES), stream, cluster, true);
   const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, gemm_few_kernel<OutT, GELU, LN, NB>, ma, mb, mae, mbe, epi, (int)M, N, K, a_rows, stages, idesc, status_word);
   note_launches(1);
   return status_from_cuda(e);
@@ -1802,7 +1838,7 @@ static int launch_few(const void* a, const void* b, const EpilogueArgs<OutT>& ep
   } else if constexpr (LN == 5) {
     return launch_few_cols<OutT, GELU, LN, 64>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
   } else {
-    switch (few_rows_cols(N, LN)) {
+    switch (few_rows_cols(M, N, LN)) {
       case 16: return launch_few_cols<OutT, GELU, LN, 16>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
       case 32: return launch_few_cols<OutT, GELU, LN, 32>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
       default: return launch_few_cols<OutT, GELU, LN, 64>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
@@ -1816,7 +1852,7 @@ static int launch_narrow(const void* a, const void* b, const EpilogueArgs<OutT>&
   if constexpr (sizeof(OutT) != 2 && LN < 3) {
     return B200_ERR_UNSUPPORTED;
   } else {
-    if (M <= kFewMaxRows) return launch_few<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+    if (takes_few_rows(M, N, LN)) return launch_few<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
     static std::atomic<bool> attr_set[kMaxDevices];
     const int slot = device_slot();
     if (slot < 0) return B200_ERR_CUDA;

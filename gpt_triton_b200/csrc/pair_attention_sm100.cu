@@ -130,7 +130,7 @@ pair_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   float* row_l = xchg + 8 * BLOCK_M;   // [map][half][128]
   float* row_sq = row_l + 4 * BLOCK_M;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qt = (p.L + BLOCK_M - 1) / BLOCK_M;
   const int bh = p.B * p.H;
   const int64_t n_items = (int64_t)n_qt * bh;
@@ -172,7 +172,7 @@ pair_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t qi = 0, ki = 0;
       bool alive = true;
       for (int64_t idx = blockIdx.x; idx < n_items && alive; idx += gridDim.x) {
@@ -212,7 +212,7 @@ pair_attention_sm100_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t qi = 0, ks = 0, kp = 0;  // items; key blocks whose scores / products have been issued
       bool alive = true;
       auto issue_s = [&](uint32_t qb) -> bool {

@@ -17,6 +17,17 @@ constexpr long long WAIT_LIMIT_CYCLES = 2000000000LL;  // about one second
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// One lane of a converged warp.  Single-thread loops of tensor-core and TMA instructions sit under this and under a
+// warp-uniform warp number (warp_index), not under `lane == 0`: those instructions take uniform registers, and only here does
+// the compiler know that one thread runs the loop.  Measured on a loop of M = 64, N = 16 MMAs: 23 clocks each instead of 46 (65 in
+// gemm_few_kernel's loop), which is more than such an MMA takes the tensor core.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }

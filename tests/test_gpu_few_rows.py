@@ -1,12 +1,13 @@
-"""Products of at most 64 rows (gemm_few_kernel): rows at the edges of its tiles of A (16, 32, 64 rows; 65 goes to the next
-kernel), columns at the edges of its 16, 32 and 64-column tiles, depths below and above one k-block and one pass through the ring."""
+"""Products on tiles of 64 rows (gemm_few_kernel): rows at the edges of its tiles of A (16, 32, 64 rows) and of one and several row
+tiles (above 64 rows the larger of the shapes below go to the next kernel, and those of 300 rows and 264 columns stay),
+columns at the edges of its 16, 32 and 64-column tiles, depths below and above one k-block and one pass through the ring."""
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
-ROWS = [1, 15, 16, 17, 33, 64, 65]
+ROWS = [1, 15, 16, 17, 33, 64, 65, 128, 300]
 
 
 def _randn(*shape, seed, scale=1.0):
