@@ -51,6 +51,18 @@ __device__ __forceinline__ float ex2_ftz(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// eight 16-bit elements that were loaded as 16 bytes
+template <typename T>
+__device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 t;
+    if constexpr (DType<T>::code == B200_F16) t = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    else t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+    f[2 * i] = t.x, f[2 * i + 1] = t.y;
+  }
+}
 // N consecutive elements moved as one access (N * sizeof(T) is 2, 4, 8 or 16 bytes; the address is aligned to it)
 template <typename T, int N>
 struct alignas(sizeof(T) * N) Vec {
@@ -73,31 +85,33 @@ __device__ __forceinline__ float warp_max(float v) {
 // piece of the output row in registers (the rescale factor of a block is the same for all lanes); at the end the
 // 16 pieces of each half are added by a halving exchange (D/2 -> D/32 values per lane in four shuffle rounds) that
 // leaves lane l with output columns (l & 1) * D/2 + (l >> 1) * D/32 + [0, D/32).
-// SPLIT = 1: one warp per (batch, head), four per block, no block-level synchronisation.  SPLIT = 4 (few sequences:
-// not enough warps to fill the GPU): the four warps of a block share one (batch, head) and take the 64-key blocks
-// 4g .. 4g + 3 of a group g side by side; the block maxima of a group go through shared memory (one block-level
-// barrier per group), so that warp w still uses the running maximum over blocks 0 .. 4g + w; the warps' partial
-// rows are merged through shared memory at the end.
-template <typename T, int D, int SPLIT>
-__global__ void __launch_bounds__(128)  // (76 registers at D = 64, six blocks per SM; capping at 64 registers for eight measured 16 % slower)
+// SPLIT = 1: one warp per (batch, head), four per block, no block-level synchronisation.  SPLIT > 1: the SPLIT warps of a block
+// share one (batch, head) and take the 64-key blocks of a group of SPLIT side by side; the block maxima of a group go through
+// shared memory (one block-level barrier per group), so that a warp still uses the running maximum over the blocks up to its own;
+// the warps' partial rows are merged through shared memory at the end.
+// What bounds it: the bytes of the cache with many sequences, the chain position -> keys -> scores -> values with few.  AHEAD (half
+// rows of 16-bit data of at most 64 bytes): all keys and values of a block are loaded into registers before the first is used, one
+// trip to memory per block instead of two; worth it while the warps that these registers cost are not missed.
+// Before (four warps, or one from 16 per SM on, values loaded behind the softmax) -> now, us (HBM alone), 12 heads of 64, bf16: 8
+// sequences, 330 keys 17.5 -> 6.7; 16 17.6 -> 10.2; 32 18.2 -> 13.4; 128 38.8 -> 31.3 (20); 197 56.7 -> 39.3 (31); 256 56.0 (40), as
+// before; 512, 1000 keys 305 -> 272 (242).
+template <typename T, int D, int SPLIT, bool AHEAD>
+__global__ void __launch_bounds__(SPLIT == 1 ? 128 : 32 * SPLIT)
 attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T* __restrict__ out, int64_t BH, int NH, int64_t cache_len,
                         float scale_log2e, const int* __restrict__ pos_dev, int* status_word) {
-  __shared__ __align__(16) float q_s[4][D + 4];  // the second half of q sits 4 floats further on: the two lanes of a pair read different banks
-  __shared__ float part_o[4][D];
-  __shared__ float part_ml[4][2];
-  __shared__ float group_max[2][4];
+  constexpr int WARPS = SPLIT == 1 ? 4 : SPLIT;
+  __shared__ __align__(16) float q_s[WARPS][D + 4];  // the second half of q sits 4 floats further on: the two lanes of a pair read different banks
+  __shared__ float part_o[SPLIT == 1 ? 1 : WARPS][D];
+  __shared__ float part_ml[WARPS][2];
+  __shared__ float group_max[2][WARPS];
   constexpr int DPL = D / 32;  // output columns per lane
   constexpr int DH = D / 2;    // elements of a row per lane of a pair
+  constexpr int VECS = DH * (int)sizeof(T) / 16;  // 16-byte pieces of that
+  static_assert(!AHEAD || (sizeof(T) == 2 && VECS <= 4), "a block's keys and values fit the registers");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int side = lane & 1, kl = lane >> 1;  // which half of the rows; which of the 16 key slots
   const int64_t w = SPLIT == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
   const int part = SPLIT == 1 ? 0 : warp;
-  const int pos = pos_dev[0];
-  if (pos < 0 || pos >= cache_len) {
-    if (threadIdx.x == 0 && status_word) atomicCAS(status_word, 0, kSiteCachePosition);
-    return;
-  }
-  if (w >= BH) return;  // (SPLIT = 4: the whole block leaves together)
   const int64_t b = w / NH;
   const int h = (int)(w % NH);
   const int64_t H = (int64_t)NH * D, pitch = 2 * H;
@@ -106,6 +120,30 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
   const T* vn = kn + H;
   T* kc = cache + b * cache_len * pitch + (int64_t)h * D;
   T* vc = kc + H;
+  pdl_launch_dependents();
+  // Ahead of the kernel in front: this warp's first block of keys and values towards L2.  (The position may still be the previous
+  // step's, or anything at all: it only decides which lines of the cache are prefetched.)
+  if (AHEAD && SPLIT > 2 && w < BH) {
+    const int64_t end = min((int64_t)*reinterpret_cast<const volatile int*>(pos_dev), cache_len);
+#pragma unroll
+    for (int r = 0; r < 64; r += 32) {
+      const int64_t key = part * 64 + r + lane;
+      if (key < end) {
+#pragma unroll
+        for (int c = 0; c < D * (int)sizeof(T); c += 128) {
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(kc + key * pitch) + c));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(vc + key * pitch) + c));
+        }
+      }
+    }
+  }
+  pdl_wait();
+  const int pos = pos_dev[0];
+  if (pos < 0 || pos >= cache_len) {
+    if (threadIdx.x == 0 && status_word) atomicCAS(status_word, 0, kSiteCachePosition);
+    return;
+  }
+  if (w >= BH) return;  // (SPLIT > 1: the whole block leaves together)
   for (int i = lane; i < D; i += 32) {
     q_s[warp][i + (i >= D / 2 ? 4 : 0)] = dot_operand<T>(to_float(qn[i]));
     if (part == 0) {
@@ -126,17 +164,35 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
   const float* q_mine = q_s[warp] + side * (DH + 4);
   for (int g = 0; g < n_groups; ++g) {
     const int k0 = (g * SPLIT + part) * 64;
+    uint4 kraw[AHEAD ? 4 : 1][AHEAD ? VECS : 1], vraw[AHEAD ? 4 : 1][AHEAD ? VECS : 1];
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + j * 16 + kl;
+        const uint4* kr = reinterpret_cast<const uint4*>((key == pos ? kn : kc + (int64_t)key * pitch) + side * DH);
+#pragma unroll
+        for (int c = 0; c < VECS; ++c) kraw[j][c] = key < n_keys ? kr[c] : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + j * 16 + kl;
+        const uint4* vr = reinterpret_cast<const uint4*>((key == pos ? vn : vc + (int64_t)key * pitch) + side * DH);
+#pragma unroll
+        for (int c = 0; c < VECS; ++c) vraw[j][c] = key < n_keys ? vr[c] : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
     float s[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int key = k0 + j * 16 + kl;
       float a = 0.f;
-      if (key < n_keys) {
+      if (AHEAD || key < n_keys) {
         const T* kr = (key == pos ? kn : kc + (int64_t)key * pitch) + side * DH;
 #pragma unroll
         for (int c = 0; c < DH; c += 8) {
           float f[8];
-          load8(kr + c, f);
+          if constexpr (AHEAD) unpack8<T>(kraw[j][c / 8], f);
+          else load8(kr + c, f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) a = fmaf(q_mine[c + i], dot_operand<T>(f[i]), a);
         }
@@ -158,7 +214,7 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
     } else {
       m_all = m_new;
     }
-    if (bm == -INFINITY) continue;  // no key of this block exists (warp-uniform; SPLIT = 4 only)
+    if (bm == -INFINITY) continue;  // no key of this block exists (warp-uniform; SPLIT > 1 only)
     const float mult = ex2_ftz(m_run - m_new);  // 0 for the warp's first block
     m_run = m_new;
     float ph[4], psum = 0.f;
@@ -179,7 +235,8 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
 #pragma unroll
         for (int c = 0; c < DH; c += 8) {
           float f[8];
-          load8(vr + c, f);
+          if constexpr (AHEAD) unpack8<T>(vraw[j][c / 8], f);
+          else load8(vr + c, f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[c + i] = fmaf(ph[j], dot_operand<T>(f[i]), o[c + i]);
         }
@@ -225,18 +282,44 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
   *reinterpret_cast<Vec<T, DPL>*>(out + b * H + (int64_t)h * D + col0) = res;
 }
 
+template <typename T, int D, int SPLIT, bool AHEAD>
+int attention_decode_split(const void* qkv_new, void* cache, void* out, int64_t BH, int64_t NH, int64_t cache_len, float sl, const int* pos_dev,
+                           int* status_word, cudaStream_t stream) {
+  const int64_t blocks = SPLIT == 1 ? (BH + 3) / 4 : BH;
+  // (an early start helps blocks that all find room; 3072 of them in the way of the product in front cost a step with 256 sequences 10 %)
+  LaunchSetup ls(dim3((unsigned)blocks), dim3(SPLIT == 1 ? 128 : 32 * SPLIT), 0, stream, 1, pdl_enabled() || blocks <= 2 * sm_count());
+  const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, attention_decode_kernel<T, D, SPLIT, AHEAD>, (const T*)qkv_new, (T*)cache, (T*)out, BH, (int)NH, cache_len, sl,
+                                           pos_dev, status_word);
+  note_launches(1);
+  return status_from_cuda(e);
+}
+
 template <typename T, int D>
 int attention_decode_sized(const void* qkv_new, void* cache, void* out, int64_t BH, int64_t NH, int64_t cache_len, float sl, const int* pos_dev,
                            int* status_word, cudaStream_t stream) {
-  // one warp per (batch, head) fills the GPU from about 16 warps per SM on; below that, four warps share one
-  if (BH >= (int64_t)sm_count() * 16)
-    attention_decode_kernel<T, D, 1><<<(unsigned)((BH + 3) / 4), 128, 0, stream>>>((const T*)qkv_new, (T*)cache, (T*)out, BH, (int)NH, cache_len, sl,
-                                                                                    pos_dev, status_word);
-  else
-    attention_decode_kernel<T, D, 4><<<(unsigned)BH, 128, 0, stream>>>((const T*)qkv_new, (T*)cache, (T*)out, BH, (int)NH, cache_len, sl, pos_dev,
-                                                                       status_word);
-  note_launches(1);
-  return status_from_cuda(cudaGetLastError());
+  const int64_t sms = sm_count();
+#define B200_DECODE(SPLIT, AHEAD) return attention_decode_split<T, D, SPLIT, AHEAD>(qkv_new, cache, out, BH, NH, cache_len, sl, pos_dev, status_word, stream)
+  if constexpr (sizeof(T) == 2 && D <= 64) {
+    // Warps per (batch, head), us at 12 heads of 64 and 100 / 330 / 1000 keys, the neighbours in brackets:
+    //   8 sequences, eight ahead 4.9 / 6.7 / 12.0 [four ahead 4.3 / 8.2 / 14.8]; 16, four ahead 6.0 / 10.2 / 18.9 [two ahead 5.8 / 11.4 / 24.8];
+    //   32, two ahead 6.6 / 13.4 / 30.1 [four 8.9 / 18.9 / 35.4]; 64, one ahead 9.8 / 20.9 / 49.6, four 11.8 / 20.5 / 42.3;
+    //   128, two 12.7 / 31.3 / 78.1 [one 17.4 / 45.3 / 124]; 256, one 20.9 / 56.0 / 155 [two 23.4 / 60.7 / 160]: these warps are about as many
+    //   as find room at once (24 per SM); 512, two 37.7 / 100 / 272 [one 39.1 / 107 / 304].
+    if (BH <= sms) B200_DECODE(8, true);
+    if (BH <= 2 * sms) B200_DECODE(4, true);
+    if (BH <= 4 * sms) B200_DECODE(2, true);
+    if (BH <= 8 * sms) {
+      if (cache_len <= 256) B200_DECODE(1, true);
+      B200_DECODE(4, false);
+    }
+    if (BH > 18 * sms && BH <= 24 * sms) B200_DECODE(1, false);
+    B200_DECODE(2, false);
+  } else {
+    // rows too wide to be held: one warp per (batch, head) fills the GPU from about 16 warps per SM on; below that, four share one
+    if (BH >= sms * 16) B200_DECODE(1, false);
+    B200_DECODE(4, false);
+  }
+#undef B200_DECODE
 }
 
 template <typename T>
