@@ -128,8 +128,8 @@ ln_stats_from_moments_kernel(const float2* __restrict__ moments, int64_t ld, int
   }
 }
 
-// The same for few rows, whose slices are narrow and many (48 for 768 columns): a warp per row, a slice per lane.  Latency is
-// all there is to it: 2 x 48 loads one behind another per thread took 4.6 us at 16 x 768, this takes 2.
+// The same for few rows: a warp per row, a slice per lane.  Latency is all there is to it: the slices' loads one behind another per
+// thread took 4.6 us at 16 rows and 48 slices, this takes 2.
 template <typename T>
 __global__ void __launch_bounds__(256)
 ln_stats_few_rows_kernel(const float2* __restrict__ moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int M,
@@ -182,7 +182,7 @@ static cudaError_t launch_ln_stats(const float2* moments, int64_t ld, int slices
 
 size_t gemm_ln_workspace_bytes(int64_t M, int64_t N) {
   if (M <= 0 || N <= 0) return 0;
-  const int64_t slices = (N + 15) / 16;  // (the narrowest slices, those of at most 64 rows)
+  const int64_t slices = (N + gemm::NARROW_BN - 1) / gemm::NARROW_BN;  // (the narrower of the two slice widths)
   return (size_t)(slices * ((M + 63) / 64 * 64)) * 8;
 }
 
@@ -234,11 +234,11 @@ int launch_gemm_ln(const void* a, const void* b, const void* bias, const void* r
   else B200_GEMM_LN_DISPATCH(__nv_bfloat16);
 #undef B200_GEMM_LN_DISPATCH
   if (st != B200_OK || !stats_out) return st;
-  // width of the column slices whose moments the GEMM left: the wide kernel's epilogue warps cover EPI_COLS columns, a
-  // narrow tile NARROW_BN, a tile of at most 64 rows few_rows_cols
+  // width of the column slices whose moments the GEMM left: the wide kernel's epilogue warps cover EPI_COLS columns, the others
+  // leave NARROW_BN
   const bool narrow = io_dtype == B200_F16 ? takes_narrow_tiles<__half, 0>(M, out, ld_out, residual, ld_res)
                                            : takes_narrow_tiles<__nv_bfloat16, 0>(M, out, ld_out, residual, ld_res);
-  const int slice_cols = !narrow ? EPI_COLS : takes_few_rows(M, N, 2) ? few_rows_cols(M, N, 2) : NARROW_BN;
+  const int slice_cols = narrow ? NARROW_BN : EPI_COLS;
   const int slices = (int)((N + slice_cols - 1) / slice_cols);
   const cudaError_t e = io_dtype == B200_F16
                             ? launch_ln_stats<__half>(ln.stats_out, ln.stats_out_ld, slices, slice_cols, N, eps, M, stats_out, ext_out, stream)

@@ -1417,7 +1417,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 // other SMs meet as well, so this is right whoever wrote the weights, and when).  The MMA is M = 64: with fewer rows its unused rows
 // read whatever follows the tile in shared memory (the next tiles, inside this CTA's allocation) and nobody reads their
 // accumulators.  k-blocks run in the same order with the same arithmetic as in the other two kernels: the same bits.
-// LN == 4 keeps its sums of squares per 64 columns: the four CTAs of 16 columns form a cluster and meet in the first one.
+// LN == 2 and 4 leave their row sums per 64 columns: the CTAs of 64 columns form a cluster and meet in the first one.
 // What bounds it: the MMAs of a CTA are one chain, K / 16 of them at 23 clocks (an M = 64, N = 16 MMA is the read of its 64 rows of
 // A from shared memory); K = 768 is 0.6 us of that, K = 8192 6.3.  The issuing thread had needed 65 clocks for each before it
 // ran under elect_one with straight-line code.
@@ -1430,7 +1430,7 @@ constexpr int FEW_THREADS = 192;
 constexpr int FEW_MAX_STAGES = 16;
 constexpr int FEW_GROUP = 2;  // k-blocks per stage
 constexpr int FEW_CTRL_BYTES = 512;
-constexpr int FEW_TAIL_BYTES = FEW_CTRL_BYTES + NARROW_BN * 4 + (kSumsqParts + 4) * kFewMaxRows * 4;  // control, bias, row sums in and out
+constexpr int FEW_TAIL_BYTES = FEW_CTRL_BYTES + NARROW_BN * 4 + (kSumsqParts + 8) * kFewMaxRows * 4;  // control, bias, row sums in and out
 constexpr int FEW_SMEM_BUDGET = 104 * 1024;                                                      // two CTAs per SM
 constexpr int FEW_PREFETCH_BYTES = 192 * 1024;                                                   // of weights, per CTA
 
@@ -1473,7 +1473,8 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   static_assert(16 * FEW_MAX_STAGES + 24 <= FEW_CTRL_BYTES, "control block too small");
   float* bias_s = reinterpret_cast<float*>(ctrl + FEW_CTRL_BYTES);
   float* parts_s = bias_s + NARROW_BN;  // [kSumsqParts][kFewMaxRows]
-  float* sums_s = parts_s + kSumsqParts * kFewMaxRows;  // LN == 4, first CTA of the cluster: [4][kFewMaxRows]
+  float* sums_s = parts_s + kSumsqParts * kFewMaxRows;  // LN == 2 and 4, first CTA of the cluster: [2 or 1][4][kFewMaxRows]
+  constexpr int CLUSTER = LN == 2 || LN == 4 ? NARROW_BN / NB : 1;
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = (int)blockIdx.x * NB, m0 = (int)blockIdx.y * kFewMaxRows;
@@ -1501,7 +1502,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
-  if constexpr (LN == 4) cluster_sync_all();  // the first CTA's shared memory exists before the others write to it
+  if constexpr (CLUSTER > 1) cluster_sync_all();  // the first CTA's shared memory exists before the others write to it
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
   pdl_launch_dependents();
@@ -1657,7 +1658,14 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       if constexpr (LN == 2) {
         if (row_ok && mom.n > 0.f) {
           const float inv = 1.0f / mom.n;
-          epi.stats_out[(int64_t)blockIdx.x * epi.stats_out_ld + row] = make_float2(fmaf(mom.s1, inv, mom.shift), fmaxf(mom.s2 - mom.s1 * mom.s1 * inv, 0.f));
+          const float mean = fmaf(mom.s1, inv, mom.shift), m2 = fmaxf(mom.s2 - mom.s1 * mom.s1 * inv, 0.f);
+          if constexpr (CLUSTER > 1) {
+            const uint32_t to = mapa_shared(smem_u32(sums_s + cluster_ctarank() * kFewMaxRows + row_i), 0);
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(mean) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + 4 * kFewMaxRows * 4), "f"(m2) : "memory");
+          } else {
+            epi.stats_out[(int64_t)blockIdx.x * epi.stats_out_ld + row] = make_float2(mean, m2);
+          }
         }
       }
     }
@@ -1670,6 +1678,30 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   }
 
+  if constexpr (LN == 2 && CLUSTER > 1) {
+    __syncwarp();
+    cluster_sync_all();  // the moments of every row are in the first CTA: merged into those of a 64-column slice, as a row's slices are later
+    const int r = (int)threadIdx.x;
+    if (blockIdx.x % CLUSTER == 0 && r < kFewMaxRows && m0 + r < M) {
+      float n[CLUSTER], total = 0.f, wsum = 0.f;
+#pragma unroll
+      for (int i = 0; i < CLUSTER; ++i) {
+        n[i] = (float)max((int)min((int64_t)NB, N - (n0 + i * NB)), 0);
+        total += n[i];
+        if (n[i] > 0.f) wsum = fmaf(n[i], sums_s[i * kFewMaxRows + r], wsum);
+      }
+      const float mean = wsum / total;
+      float m2 = 0.f;
+#pragma unroll
+      for (int i = 0; i < CLUSTER; ++i) {
+        if (n[i] > 0.f) {
+          const float d = sums_s[i * kFewMaxRows + r] - mean;
+          m2 += fmaf(n[i] * d, d, sums_s[(4 + i) * kFewMaxRows + r]);
+        }
+      }
+      epi.stats_out[(int64_t)(blockIdx.x / CLUSTER) * epi.stats_out_ld + m0 + r] = make_float2(mean, m2);
+    }
+  }
   if constexpr (LN == 4) {
     __syncwarp();
     cluster_sync_all();  // the four sums of every row are in the first CTA
@@ -1779,7 +1811,7 @@ inline int few_rows_cols(int64_t M, int64_t N, int ln) {
   return (N + 31) / 32 * row_tiles > 120 ? 32 : 16;
 }
 // Whether a product of at most kNarrowMaxRows rows goes to gemm_few_kernel: up to 64 rows always, above that as long as its tiles
-// of 64 rows and 16 or 32 columns fit the GPU at once (two CTAs per SM; the clusters of LN == 4 do not get the last few places).
+// of 64 rows and 16 or 32 columns fit the GPU at once (two CTAs per SM; the clusters of LN == 2 and 4 do not get the last few places).
 // Beyond that its smaller tiles read A and B more often than they help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of
 // gemm_narrow_kernel; LN == 4, 384 rows, 768 x 3072 (288 CTAs): 18.2 against 13.5, 256 rows (192 CTAs): 10.0 against 13.7.
 inline bool takes_few_rows(int64_t M, int64_t N, int ln) {
@@ -1787,7 +1819,7 @@ inline bool takes_few_rows(int64_t M, int64_t N, int ln) {
   if (ln == 5) return false;
   const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows;
   const int cols = few_rows_cols(M, N, ln);
-  return (N + cols - 1) / cols * row_tiles <= (ln == 4 ? 256 : 296);
+  return (N + cols - 1) / cols * row_tiles <= (ln == 4 || ln == 2 ? 256 : 296);
 }
 
 template <typename OutT, bool GELU, int LN, int NB>
@@ -1818,7 +1850,7 @@ static int launch_few_cols(const void* a, const void* b, const EpilogueArgs<OutT
   if (st == B200_OK && LN == 1) st = make_map(&mae, ln.a_ext, M, kLnExtCols, kLnExtCols, a_rows, op_dtype);
   if (st == B200_OK && LN == 1) st = make_map(&mbe, ln.b_ext, N, kLnExtCols, kLnExtCols, NB, op_dtype);
   if (st != B200_OK) return st;
-  constexpr int cluster = LN == 4 ? 4 : 1;
+  constexpr int cluster = LN == 2 || LN == 4 ? NARROW_BN / NB : 1;
   const unsigned ctas = (unsigned)((N + NB * cluster - 1) / (NB * cluster) * cluster);
   const uint32_t idesc = (1u << 4) | ((op_dtype == B200_BF16 ? 1u : 0u) << 7) | ((op_dtype == B200_BF16 ? 1u : 0u) << 10) | ((uint32_t)(NB >> 3) << 17) |
                          ((uint32_t)(kFewMaxRows >> 4) << 24);
