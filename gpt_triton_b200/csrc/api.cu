@@ -154,6 +154,14 @@ int b200_gemm(const void* a, const void* b, const void* bias, const void* residu
                                 status_word, (cudaStream_t)stream));
 }
 
+int b200_gemm_operand(const void* a, const void* b, const float* bias, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                      int64_t ld_out, int add_gelu, int* status_word, void* stream) {
+  if (M < 0 || N < 0 || K < 1 || M > kMaxExtent || N > kMaxExtent || K > kMaxExtent) return B200_ERR_BAD_ARGUMENT;
+  if (M == 0 || N == 0) return B200_OK;
+  if (!a || !b || !out || lda < K || ldb < K || ld_out < N) return B200_ERR_BAD_ARGUMENT;
+  return note(b200::launch_gemm_operand(a, b, bias, out, M, N, K, lda, ldb, ld_out, add_gelu, status_word, (cudaStream_t)stream));
+}
+
 size_t b200_gemm_argmax_workspace_bytes(int64_t M, int64_t N) { return b200::gemm_argmax_workspace_bytes(M, N); }
 
 int b200_gemm_argmax(const void* a, const void* b, const void* bias, const void* residual, void* out, int64_t M, int64_t N,

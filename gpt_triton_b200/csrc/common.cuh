@@ -257,6 +257,8 @@ int launch_attention(const void* q, const void* k, const void* v, void* out, int
 int64_t linear_sm100_slice_cols(int64_t M);
 int64_t linear_f32_slice_cols();
 int launch_linear_sm100(const b200_linear_args& p, cudaStream_t stream);
+int launch_gemm_operand(const void* a, const void* b, const float* bias, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                        int64_t ld_out, int add_gelu, int* status_word, cudaStream_t stream);
 int launch_linear_f32(const b200_linear_args& p, cudaStream_t stream);
 int launch_embedding_rms(const int64_t* ids, const void* table, const float* gain, float* x, void* gx, float* sumsq, int64_t T, int64_t V, int64_t W,
                          int64_t ld_gx, int dtype, cudaStream_t stream);

@@ -30,6 +30,20 @@ int fill_and_launch(const b200_linear_args& p, cudaStream_t stream) {
 
 }  // namespace
 
+// fp16([gelu](A B^T + bias)) from fp16 operands with a float32 bias: a product of a float32 model whose result is only ever an
+// operand.  GELU and rounding are those of the float32 epilogue and of pack_kernel behind it: the same bits in one pass.  16 x 300
+// tokens, 768 -> 3072 with GELU: 52 us + 13 us of pack_kernel on the next product's side before.
+int launch_gemm_operand(const void* a, const void* b, const float* bias, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                        int64_t ld_out, int add_gelu, int* status_word, cudaStream_t stream) {
+  if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(bias)) & 15) || lda % 8 || ldb % 8) return B200_ERR_ALIGNMENT;
+  b200_linear_args p;
+  memset(&p, 0, sizeof(p));
+  p.a = a, p.b = b, p.M = M, p.N = N, p.K = K, p.lda = lda, p.ldb = ldb, p.out = out, p.ld_out = ld_out, p.op_dtype = B200_F16, p.out_dtype = B200_F16;
+  p.bias = bias, p.out_scale = 1.f, p.status_word = status_word;
+  p.act_lo = add_gelu ? B200_ACT_GELU_TANH : 0, p.act_hi = p.act_lo, p.act_split = N;
+  return fill_and_launch<__half, 3>(p, stream);
+}
+
 int64_t linear_sm100_slice_cols(int64_t M) { return M <= gemm::kNarrowMaxRows ? gemm::NARROW_BN : gemm::EPI_COLS; }
 
 int launch_linear_sm100(const b200_linear_args& p, cudaStream_t stream) {

@@ -463,6 +463,51 @@ def ffn_row_statistics(x, weight, bias=None, targets=None, want_lse=True):
     return ids.view(lead), (lse.view(lead) if want_lse else None), (picked.view(lead) if picked is not None else None)
 
 
+# ----------------------------------------------------------------------------- float32 storage, operands kept as operands
+# The reference rounds every dot operand of a float32 model to fp16 (kernels.py:229-234).  What is only ever such an operand can
+# leave its producer as fp16: the same values, half the bytes, and no pass that converts them.
+def takes_operand_rows(x, weight, bias):
+    """Whether the two products below take a float32 model's rows of x's width, its PackedWeight and its bias.  More than 128 rows:
+    with fewer a conversion pass is a launch of 2 us, and the operator sequence stays what it is documented to be; at 4800 x 768
+    the passes take 13 us each, a fifth of the forward."""
+    return (x.dtype == torch.float32 and x.is_cuda and x.shape[-1] % 8 == 0 and x.numel() > 128 * x.shape[-1] and weight.storage_dtype == torch.float32
+            and weight.data.dtype == torch.float16 and weight.N % 8 == 0 and (bias is None or bias.data_ptr() % 16 == 0))
+
+
+def _operand_rows_checked(x, weight, bias):
+    """(M, K, N, device) of operand rows x (*, K) and the PackedWeight of a float32 model."""
+    require_cuda(x, bias)
+    assert x.dtype == torch.float16 and x.is_contiguous() and weight.storage_dtype == torch.float32 and x.shape[-1] == weight.K
+    assert bias is None or (bias.dtype == torch.float32 and bias.is_contiguous() and bias.shape == (weight.N,))
+    return x.numel() // weight.K, weight.K, weight.N, _same_device(x, weight.data, bias)
+
+
+@torch.no_grad()
+def operand_ffn(x, weight, bias=None, add_gelu=False):
+    """fp16([gelu_new](x @ weight + bias)): x (*, K) fp16 operand rows of a float32 model, weight its PackedWeight, bias float32
+    (N,).  What fused_ffn would compute in float32 from the same operands, rounded as an operand."""
+    M, K, N, dev = _operand_rows_checked(x, weight, bias)
+    z = torch.empty((*x.shape[:-1], N), device=dev, dtype=torch.float16)
+    with torch.cuda.device(dev):
+        st = _lib.load().b200_gemm_operand(x.data_ptr(), weight.data.data_ptr(), _ptr(bias), z.data_ptr(), M, N, K, K, weight.data.stride(0), N,
+                                           int(bool(add_gelu)), _status_ptr(dev), stream_ptr(dev))
+    check(st, "operand_ffn")
+    return z
+
+
+@torch.no_grad()
+def operand_ffn_residual(x, weight, bias=None, residual=None):
+    """x @ weight + bias + residual in float32: x (*, K) fp16 operand rows of a float32 model (see operand_ffn)."""
+    M, K, N, dev = _operand_rows_checked(x, weight, bias)
+    assert residual is None or (residual.dtype == torch.float32 and residual.is_contiguous() and residual.numel() == M * N and residual.device == dev)
+    z = torch.empty((*x.shape[:-1], N), device=dev, dtype=torch.float32)
+    with torch.cuda.device(dev):
+        st = _lib.load().b200_gemm(x.data_ptr(), weight.data.data_ptr(), _ptr(bias), _ptr(residual), z.data_ptr(), M, N, K, K, weight.data.stride(0), N, N,
+                                   _lib.F16, _lib.F32, 0, _status_ptr(dev), stream_ptr(dev))
+    check(st, "operand_ffn_residual")
+    return z
+
+
 # ----------------------------------------------------------------------------- qkv split
 @torch.no_grad()
 def matmul_and_split_qkv(x, weight, bias, num_heads):

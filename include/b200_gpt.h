@@ -153,6 +153,13 @@ int b200_gemm(const void* a, const void* b, const void* bias, const void* residu
               int add_gelu, int* status_word, void* stream);
 
 /*
+ * A product of a float32 model whose result is only ever an operand (fp16 there): out [M,N] = fp16([gelu](A B^T + bias)), A [M,K]
+ * and B [N,K] fp16, 16-byte aligned, lda and ldb multiples of 8; bias fp32 [N], 16-byte aligned, or NULL.
+ */
+int b200_gemm_operand(const void* a, const void* b, const float* bias, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                      int64_t ld_out, int add_gelu, int* status_word, void* stream);
+
+/*
  * b200_gemm that additionally returns, per output row, the column of the row's maximum:
  * argmax_out[row] (int64, device) = argmax over the stored (rounded) out[row, 0..N), the lowest
  * column on ties.  Meant for the tied lm_head (gpt.py:159-161, 172-179 of the reference): greedy
