@@ -4,7 +4,9 @@ There is no fallback: if the library is missing or a symbol cannot be bound, imp
 the operators fails with an error that says how to build it.
 """
 
+import contextlib
 import ctypes
+import functools
 import os
 
 import torch
@@ -161,7 +163,30 @@ def check(status, what):
 
 
 def stream_ptr(device):
-    return torch.cuda.current_stream(device).cuda_stream
+    """The raw current stream of `device`, without the Stream object around it (2 us per launch)."""
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+_STAY = contextlib.nullcontext()
+
+
+def on_device(device):
+    """Context in which `device` is the current one.  It nearly always is already, and entering torch.cuda.device costs 4 us."""
+    return _STAY if device.index is None or torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
+def without_grad(fn):
+    """torch.no_grad() around fn, entered only where gradients are being recorded (3 us per call)."""
+
+    @functools.wraps(fn)
+    def call(*args, **kwargs):
+        if not torch.is_grad_enabled():
+            return fn(*args, **kwargs)
+        with torch.no_grad():
+            return fn(*args, **kwargs)
+
+    return call
 
 
 def require_cuda(*tensors):

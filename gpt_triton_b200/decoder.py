@@ -53,8 +53,10 @@ class StreamDecoder(GeneratesTokens, _EvalOnly):
         B, n = ids.shape
         rows = self._run(ids.reshape(-1).contiguous(), PromptContext(B, n, start, cache), "prompt", tap)
         if want is None:
-            want = torch.tensor([n - 1], device=ids.device)
-        index = (torch.arange(B, device=ids.device)[:, None] * n + want[None, :]).reshape(-1)
+            # made on the device: a tensor of host values would be a copy that waits for every kernel above
+            index = torch.arange(n - 1, B * n, n, device=ids.device)
+        else:
+            index = (torch.arange(B, device=ids.device)[:, None] * n + want[None, :]).reshape(-1)
         return rows if index.numel() == B * n and n == 1 else K.select_rows(rows, index)
 
     def decode_pass(self, ids, cache, pos):

@@ -97,7 +97,7 @@ class GenerationSession:
         step = portion if portion > 0 else L0
         for t in range(0, L0, step):
             last = self.extend(ids[:, t:t + step].contiguous())
-        self.pos.copy_(torch.tensor([L0, L0], dtype=torch.int32), non_blocking=False)
+        self.pos.fill_(L0)
         first = m.pick(last, self.temperature, self.top_k, self.seed, self.pos)
         K.decode_append(first, self.tokens, self.pos, advance=False, feedback=self.feedback)
         steps = max_new_tokens - 1

@@ -27,7 +27,7 @@ import math
 import torch
 
 from . import _lib
-from ._lib import check, dtype_code, require_cuda, stream_ptr
+from ._lib import check, dtype_code, on_device, require_cuda, stream_ptr, without_grad
 
 _lib.load()  # fail at import time, loudly, if the extension is not built
 
@@ -78,7 +78,7 @@ def bounded_wait_selftest(limit_cycles=200_000_000, device=None):
     code it reports once the wait has run out: B200_ERR_DEVICE_WAIT (6) on a healthy GPU.  Synchronises."""
     dev = torch.device("cuda", torch.cuda.current_device() if device is None else torch.device(device).index)
     word = torch.zeros(1, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(_lib.load().b200_selftest_bounded_wait(word.data_ptr(), int(limit_cycles), stream_ptr(dev)), "bounded_wait_selftest")
     return int(word.item())
 
@@ -115,7 +115,7 @@ class RowStats:
         return self.data[:, 1]
 
 
-@torch.no_grad()
+@without_grad
 def row_stats(x):
     """RowStats of the rows of x (*, H) (the statistics half of the reference's fused_layer_norm,
     kernels.py:116-130): what ``fused_ffn(..., ln_stats=...)`` needs for rows that no operator of this
@@ -126,13 +126,13 @@ def row_stats(x):
     M = x.numel() // H if H else 0
     data = torch.empty((max(M, 1), 2), device=x.device, dtype=torch.float32)
     ext = torch.empty((max(M, 1), LN_EXT_COLS), device=x.device, dtype=x.dtype) if x.dtype != torch.float32 else None
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         st = _lib.load().b200_row_ln_stats(x.data_ptr(), data.data_ptr(), _ptr(ext), M, H, LN_EPS, dtype_code(x.dtype), stream_ptr(x.device))
     check(st, "row_stats")
     return RowStats(data[:M], H, None if ext is None else ext[:M])
 
 
-@torch.no_grad()
+@without_grad
 def fused_embeddings(x, wte, wpe, dropout_prob=0.0, *, return_row_stats=False, position=None):
     """z[b, l, :] = wte[x[b, l], :] + wpe[l, :]  (reference kernels.py:76-101).  With ``return_row_stats`` the
     result is ``(z, RowStats of z's rows)``, taken while the rows are written.  ``position`` (a CUDA int32 tensor;
@@ -157,7 +157,7 @@ def fused_embeddings(x, wte, wpe, dropout_prob=0.0, *, return_row_stats=False, p
         assert position.dtype == torch.int32 and position.device == dev and position.numel() >= 1
         stats = torch.empty((max(B * L, 1), 2), device=dev, dtype=torch.float32) if return_row_stats else None
         ext = torch.empty((max(B * L, 1), LN_EXT_COLS), device=dev, dtype=wte.dtype) if return_row_stats and wte.dtype != torch.float32 else None
-        with torch.cuda.device(dev):
+        with on_device(dev):
             st = _lib.load().b200_embedding_at(x.data_ptr(), wte.data_ptr(), wpe.data_ptr(), z.data_ptr(), B, L, V, P, H, dtype_code(wte.dtype),
                                                None, LN_EPS, _ptr(stats), _ptr(ext), position.data_ptr(), stream_ptr(dev))
         check(st, "fused_embeddings(position)")
@@ -166,12 +166,12 @@ def fused_embeddings(x, wte, wpe, dropout_prob=0.0, *, return_row_stats=False, p
     if return_row_stats:
         stats = torch.empty((max(B * L, 1), 2), device=dev, dtype=torch.float32)
         ext = torch.empty((max(B * L, 1), LN_EXT_COLS), device=dev, dtype=wte.dtype) if wte.dtype != torch.float32 else None
-        with torch.cuda.device(dev):
+        with on_device(dev):
             st = _lib.load().b200_embedding_ln_stats(x.data_ptr(), wte.data_ptr(), wpe.data_ptr(), z.data_ptr(), B, L, V, P, H,
                                                      dtype_code(wte.dtype), None, LN_EPS, stats.data_ptr(), _ptr(ext), stream_ptr(dev))
         check(st, "fused_embeddings")
         return z.view((B, L, H)), RowStats(stats[:B * L], H, None if ext is None else ext[:B * L])
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_embedding(x.data_ptr(), wte.data_ptr(), wpe.data_ptr(), z.data_ptr(), B, L, V, P, H,
                                         dtype_code(wte.dtype), None, stream_ptr(dev))
     check(st, "fused_embeddings")
@@ -179,7 +179,7 @@ def fused_embeddings(x, wte, wpe, dropout_prob=0.0, *, return_row_stats=False, p
 
 
 # ----------------------------------------------------------------------------- layer norm
-@torch.no_grad()
+@without_grad
 def fused_layer_norm(x, weight, bias, *, out_dtype=None):
     """Row LayerNorm, fp32 statistics, eps 1e-5 (reference kernels.py:149-164)."""
     require_cuda(x, weight, bias)
@@ -194,7 +194,7 @@ def fused_layer_norm(x, weight, bias, *, out_dtype=None):
     M = x.numel() // H if H else 0
     dev = _same_device(x, weight, bias)
     z = torch.empty(x.shape, device=dev, dtype=out_dtype or x.dtype)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_layernorm(x.data_ptr(), weight.data_ptr(), bias.data_ptr(), z.data_ptr(), M, H, LN_EPS,
                                         dtype_code(x.dtype), dtype_code(z.dtype), stream_ptr(dev))
     check(st, "fused_layer_norm")
@@ -215,7 +215,7 @@ class PackedWeight:
         self.data, self.K, self.N, self.storage_dtype = data, K, N, storage_dtype
 
 
-@torch.no_grad()
+@without_grad
 def pack_weight(weight, *, weight_is_nk=False):
     """Round a [K, N] (or, with weight_is_nk, [N, K]) weight to its 16-bit operand type and
     store it [N, K_padded] K-major.  fp32 and fp16 weights become fp16 (the rounding the
@@ -230,7 +230,7 @@ def pack_weight(weight, *, weight_is_nk=False):
     dev = weight.device
     packed = torch.empty((N, kp), device=dev, dtype=op_dtype)
     rows, cols = weight.shape
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_pack_operand(weight.data_ptr(), packed.data_ptr(), rows, cols, cols, kp,
                                            0 if weight_is_nk else 1, dtype_code(weight.dtype), dtype_code(op_dtype),
                                            stream_ptr(dev))
@@ -250,7 +250,7 @@ class FoldedWeight:
         self.data, self.colsum, self.bias, self.ext, self.K, self.N, self.storage_dtype = data, colsum, bias, ext, K, N, storage_dtype
 
 
-@torch.no_grad()
+@without_grad
 def fold_layer_norm(weight, ln_weight, ln_bias, bias=None):
     """Fold ``fused_layer_norm(x, ln_weight, ln_bias)`` into the GEMM ``fused_ffn(., weight, bias)`` that follows it
     (reference gpt.py:40-43, 94-101; its author's TODO at kernels.py:132-133):
@@ -272,7 +272,7 @@ def fold_layer_norm(weight, ln_weight, ln_bias, bias=None):
     colsum = torch.empty((N,), device=dev, dtype=torch.float32)
     fbias = torch.empty((N,), device=dev, dtype=torch.float32)
     ext = torch.empty((N, LN_EXT_COLS), device=dev, dtype=weight.dtype)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_fold_layernorm(weight.data_ptr(), ln_weight.data_ptr(), ln_bias.data_ptr(), _ptr(bias), data.data_ptr(),
                                              colsum.data_ptr(), fbias.data_ptr(), ext.data_ptr(), K, N, K, dtype_code(weight.dtype),
                                              stream_ptr(dev))
@@ -300,7 +300,7 @@ def _ffn_layer_norm_aware(x, weight, bias, residual, add_gelu, out, ln_stats, re
     lib = _lib.load()
     dt = dtype_code(x.dtype)
     stats_out = None
-    with torch.cuda.device(dev):
+    with on_device(dev):
         if ln_stats is not None:
             assert isinstance(weight, FoldedWeight), "ln_stats needs the FoldedWeight made by fold_layer_norm"
             assert bias is None, "the bias is part of the FoldedWeight"
@@ -325,7 +325,7 @@ def _ffn_layer_norm_aware(x, weight, bias, residual, add_gelu, out, ln_stats, re
     return (zz, RowStats(stats_out[:M], N, ext_out[:M])) if return_row_stats else zz
 
 
-@torch.no_grad()
+@without_grad
 def fused_ffn(x, weight, bias=None, residual=None, add_gelu=False, dropout_prob=0.0, *, weight_is_nk=False, out=None,
               return_argmax=False, return_lse=False, ln_stats=None, return_row_stats=False):
     """z = [gelu_new](x @ weight + bias) + residual  (reference kernels.py:261-315).
@@ -380,7 +380,7 @@ def fused_ffn(x, weight, bias=None, residual=None, add_gelu=False, dropout_prob=
     ld_out = z.stride(0) if M > 1 else max(N, z.stride(0))
     lib = _lib.load()
     dt = dtype_code(x.dtype)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         stream = stream_ptr(dev)
         if return_argmax or return_lse:
             assert packed is not None and dt != _lib.F32 and K % 8 == 0 and x.data_ptr() % 16 == 0, \
@@ -423,7 +423,7 @@ def fused_ffn(x, weight, bias=None, residual=None, add_gelu=False, dropout_prob=
     return z.view((*out_shape_0, N))
 
 
-@torch.no_grad()
+@without_grad
 def ffn_row_statistics(x, weight, bias=None, targets=None, want_lse=True):
     """Row statistics of z = x @ weight (+ bias) without materialising z (no counterpart in the reference, whose
     lm_head is commented out, gpt.py:172-179): ``(ids, lse, target_value)`` with ids (*,) int64 the argmax of each
@@ -455,7 +455,7 @@ def ffn_row_statistics(x, weight, bias=None, targets=None, want_lse=True):
     lib = _lib.load()
     need = lib.b200_gemm_argmax_workspace_bytes(M, N)
     ws = torch.empty((max(need, 16),), device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib.b200_gemm_rowstats(x.data_ptr(), weight.data.data_ptr(), _ptr(bias), M, N, K, K, weight.data.stride(0),
                                     dtype_code(weight.data.dtype), dt, _ptr(targets), ids.data_ptr(), _ptr(lse), _ptr(picked),
                                     ws.data_ptr(), need, _status_ptr(dev), stream_ptr(dev))
@@ -482,26 +482,26 @@ def _operand_rows_checked(x, weight, bias):
     return x.numel() // weight.K, weight.K, weight.N, _same_device(x, weight.data, bias)
 
 
-@torch.no_grad()
+@without_grad
 def operand_ffn(x, weight, bias=None, add_gelu=False):
     """fp16([gelu_new](x @ weight + bias)): x (*, K) fp16 operand rows of a float32 model, weight its PackedWeight, bias float32
     (N,).  What fused_ffn would compute in float32 from the same operands, rounded as an operand."""
     M, K, N, dev = _operand_rows_checked(x, weight, bias)
     z = torch.empty((*x.shape[:-1], N), device=dev, dtype=torch.float16)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_gemm_operand(x.data_ptr(), weight.data.data_ptr(), _ptr(bias), z.data_ptr(), M, N, K, K, weight.data.stride(0), N,
                                            int(bool(add_gelu)), _status_ptr(dev), stream_ptr(dev))
     check(st, "operand_ffn")
     return z
 
 
-@torch.no_grad()
+@without_grad
 def operand_ffn_residual(x, weight, bias=None, residual=None):
     """x @ weight + bias + residual in float32: x (*, K) fp16 operand rows of a float32 model (see operand_ffn)."""
     M, K, N, dev = _operand_rows_checked(x, weight, bias)
     assert residual is None or (residual.dtype == torch.float32 and residual.is_contiguous() and residual.numel() == M * N and residual.device == dev)
     z = torch.empty((*x.shape[:-1], N), device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_gemm(x.data_ptr(), weight.data.data_ptr(), _ptr(bias), _ptr(residual), z.data_ptr(), M, N, K, K, weight.data.stride(0), N, N,
                                    _lib.F16, _lib.F32, 0, _status_ptr(dev), stream_ptr(dev))
     check(st, "operand_ffn_residual")
@@ -509,7 +509,7 @@ def operand_ffn_residual(x, weight, bias=None, residual=None):
 
 
 # ----------------------------------------------------------------------------- qkv split
-@torch.no_grad()
+@without_grad
 def matmul_and_split_qkv(x, weight, bias, num_heads):
     """c_attn projection and head split (reference kernels.py:348-367).
 
@@ -539,7 +539,7 @@ def _bhl_strides(t):
     return (ctypes.c_int64 * 3)(t.stride(0), t.stride(1), t.stride(2))
 
 
-@torch.no_grad()
+@without_grad
 def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False):
     """Causal softmax(q k^T / sqrt(H)) v with the reference's 64-key online softmax
     (reference kernels.py:478-525).  q, k, v: (batch, heads, seqlen, head_size), contiguous or
@@ -564,7 +564,7 @@ def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False):
         z = torch.empty((B, N, Lq, H), device=dev, dtype=q.dtype)
         zv = z
     scale = 1 / math.sqrt(H)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), z.data_ptr(), B, N, Lq, H, _bhl_strides(q),
                                         _bhl_strides(k), _bhl_strides(v), _bhl_strides(zv), scale, dtype_code(q.dtype),
                                         dtype_code(z.dtype), _status_ptr(dev), stream_ptr(dev))
@@ -576,7 +576,7 @@ def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False):
 # No counterpart in the reference (its README.md:55 lists "KV cache + sampling" as not built).  ``pos`` below is a
 # CUDA int32 tensor of two elements, {tokens in the cache, prompt length}: the kernels read it on the device, so the
 # launches of a decode step can be captured once in a CUDA graph and replayed for every step.
-@torch.no_grad()
+@without_grad
 def kv_cache_fill(qkv, cache):
     """cache[b, l, :] = qkv[b, l, H:3H] for the L positions of a prompt: qkv (B, L, 3H) is the fused c_attn output
     (q | k | v), cache (B, cache_len, 2H) holds k | v.  Both contiguous, same dtype."""
@@ -586,13 +586,13 @@ def kv_cache_fill(qkv, cache):
     assert H3 == 3 * H and cache.dim() == 3 and cache.shape[0] == B and cache.shape[2] == 2 * H and cache.shape[1] >= L
     assert qkv.is_contiguous() and cache.is_contiguous() and qkv.dtype == cache.dtype
     dev = _same_device(qkv, cache)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_kv_cache_fill(qkv.data_ptr(), cache.data_ptr(), B, L, H, cache.shape[1], dtype_code(qkv.dtype), stream_ptr(dev))
     check(st, "kv_cache_fill")
     return cache
 
 
-@torch.no_grad()
+@without_grad
 def attention_decode(qkv_new, cache, pos, num_heads):
     """One decode step of causal attention: qkv_new (B, 3H) is q | k | v of the token at position pos[0]; its k, v are
     stored into cache[:, pos[0]] and the result (B, H) is softmax(q K^T / sqrt(D)) V over positions 0..pos[0], with the
@@ -608,14 +608,14 @@ def attention_decode(qkv_new, cache, pos, num_heads):
     assert pos.dtype == torch.int32 and pos.numel() >= 2
     dev = _same_device(qkv_new, cache, pos)
     out = torch.empty((B, H), device=dev, dtype=qkv_new.dtype)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_attention_decode(qkv_new.data_ptr(), cache.data_ptr(), out.data_ptr(), B, num_heads, D, cache.shape[1],
                                                1 / math.sqrt(D), dtype_code(qkv_new.dtype), pos.data_ptr(), _status_ptr(dev), stream_ptr(dev))
     check(st, "attention_decode")
     return out
 
 
-@torch.no_grad()
+@without_grad
 def decode_append(next_ids, tokens, pos, advance, feedback=None):
     """tokens[:, pos[0] - pos[1] + advance] = next_ids (and feedback[:] = next_ids, the buffer the next decode step
     embeds), then pos[0] += 1 if advance -- all on the device."""
@@ -625,13 +625,13 @@ def decode_append(next_ids, tokens, pos, advance, feedback=None):
     assert next_ids.dtype == tokens.dtype == torch.int64 and next_ids.is_contiguous() and tokens.dim() == 2 and tokens.stride(1) == 1
     assert tokens.shape[0] == next_ids.numel() and pos.dtype == torch.int32 and pos.numel() >= 2
     dev = _same_device(next_ids, tokens, pos, feedback)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_decode_append(next_ids.data_ptr(), tokens.data_ptr(), tokens.stride(0) if tokens.shape[0] > 1 else tokens.shape[1],
                                             tokens.shape[1], tokens.shape[0], pos.data_ptr(), int(bool(advance)), _ptr(feedback), _status_ptr(dev), stream_ptr(dev))
     check(st, "decode_append")
 
 
-@torch.no_grad()
+@without_grad
 def sample_logits(logits, temperature=1.0, top_k=0, seed=0, step=None, out=None):
     """One id per row of logits (B, V), drawn from softmax(logits / temperature) over the row's top_k largest logits
     (0 = all; ties with the k-th largest stay in).  Gumbel-max with counter-based uniforms: the same
@@ -644,7 +644,7 @@ def sample_logits(logits, temperature=1.0, top_k=0, seed=0, step=None, out=None)
     assert ids.dtype == torch.int64 and ids.is_contiguous() and ids.numel() == B and ids.device == dev
     if step is not None:
         assert step.dtype == torch.int32 and step.numel() >= 1
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_sample_logits(logits.data_ptr(), logits.stride(0) if B > 1 else V, B, V, dtype_code(logits.dtype), float(temperature),
                                             int(top_k), int(seed) & 0xFFFFFFFFFFFFFFFF, _ptr(step), ids.data_ptr(), stream_ptr(dev))
     check(st, "sample_logits")
@@ -730,7 +730,7 @@ def _linear_args(rows, weight):
     return p, a, dev
 
 
-@torch.no_grad()
+@without_grad
 def embedding_rms(ids, table, gain, eps):
     """Start of an fp32 residual stream: ids (n,) int64 -> (x (n, width) float32 = table[ids], NormedRows of x under an RMS
     norm with weights `gain` (width,) float32)."""
@@ -743,14 +743,14 @@ def embedding_rms(ids, table, gain, eps):
     x = torch.empty((n, W), device=dev, dtype=torch.float32)
     gx = _rows_empty(n, W, table.dtype, dev)
     sumsq = torch.empty((1, n), device=dev, dtype=torch.float32)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_embedding_rms(ids.data_ptr(), table.data_ptr(), gain.data_ptr(), x.data_ptr(), gx.data_ptr(), sumsq.data_ptr(), n, V, W,
                                             max(gx.stride(0), W), dtype_code(table.dtype), stream_ptr(dev))
     check(st, "embedding_rms")
     return x, NormedRows(gx, sumsq, W, eps)
 
 
-@torch.no_grad()
+@without_grad
 def linear(rows, weight, *, bias=None, act=None, act_split=None, act_after=None, act_param=0.0, out_scale=1.0, out_dtype=None):
     """act(norm(rows) @ weight^T * out_scale + bias): rows a NormedRows or a plain (M, K) matrix, weight (N, K), bias float32
     (N,).  `act` applies to the output columns below `act_split` (default: all), `act_after` to the rest; `act_param`: the
@@ -765,12 +765,12 @@ def linear(rows, weight, *, bias=None, act=None, act_split=None, act_after=None,
     p.act_lo, p.act_hi = ACTIVATIONS[act], ACTIVATIONS[act_after]
     p.act_split = p.N if act_split is None else act_split
     p.out_scale = out_scale
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(_lib.load().b200_linear(ctypes.byref(p), stream_ptr(dev)), "linear")
     return out
 
 
-@torch.no_grad()
+@without_grad
 def linear_residual(rows, weight, x, gain=None, eps=0.0):
     """x += norm(rows) @ weight^T, in place on the fp32 residual stream x (M, N).  With `gain` (N,) float32 returns the
     NormedRows of the new x under an RMS norm with those weights."""
@@ -787,13 +787,13 @@ def linear_residual(rows, weight, x, gain=None, eps=0.0):
         sumsq = torch.empty(((p.N + cols - 1) // cols, p.M), device=dev, dtype=torch.float32)
         p.gain, p.gx, p.ld_gx, p.sumsq_out, p.sumsq_out_ld = gain.data_ptr(), gx.data_ptr(), max(gx.stride(0), p.N), sumsq.data_ptr(), p.M
         normed = NormedRows(gx, sumsq, p.N, eps)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.b200_linear(ctypes.byref(p), stream_ptr(dev)), "linear_residual")
     return normed
 
 
 # ----------------------------------------------------------------------------- latent attention
-@torch.no_grad()
+@without_grad
 def latent_append(raw, weight, eps, batch, *, cache=None, hist=0, start=0, pos=None, keep_rows=True):
     """RMS norm (plain `weight` (R,) float32) of the new tokens' latents raw (batch * n, R).  They join `cache` (batch, ring,
     R) at the slots position % ring, the first position being `start`, or pos[0] on the device; with `keep_rows` the
@@ -809,7 +809,7 @@ def latent_append(raw, weight, eps, batch, *, cache=None, hist=0, start=0, pos=N
         ring = cache.shape[1]
     work = torch.empty((batch, hist + n, R), device=dev, dtype=raw.dtype) if keep_rows else None
     lib, dt = _lib.load(), dtype_code(raw.dtype)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         if hist:
             check(lib.b200_latent_gather(cache.data_ptr(), work.data_ptr(), batch, n, R, hist, ring, start, dt, stream_ptr(dev)), "latent_gather")
         st = lib.b200_latent_append(raw.data_ptr(), max(raw.stride(0), R), weight.data_ptr(), float(eps), _ptr(work), _ptr(cache), batch, n, R, hist, ring,
@@ -818,7 +818,7 @@ def latent_append(raw, weight, eps, batch, *, cache=None, hist=0, start=0, pos=N
     return work
 
 
-@torch.no_grad()
+@without_grad
 def window_attention(q, k, v, batch, heads, dim, vdim, window, scale, sink=None):
     """Causal sliding-window softmax attention with an optional sink (float32 (heads,), one extra exp(sink) in the
     denominator).  q (batch * n, heads * dim); k, v (batch * m, heads * dim / vdim), m >= n: the n queries are the last n of
@@ -832,7 +832,7 @@ def window_attention(q, k, v, batch, heads, dim, vdim, window, scale, sink=None)
         assert sink.dtype == torch.float32 and sink.numel() == heads and sink.is_contiguous()
     dev = _same_device(q, k, v, sink)
     out = _rows_empty(M, heads * vdim, q.dtype, dev)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = _lib.load().b200_window_attention(q.data_ptr(), max(q.stride(0), heads * dim), k.data_ptr(), max(k.stride(0), heads * dim), v.data_ptr(),
                                                max(v.stride(0), heads * vdim), out.data_ptr(), max(out.stride(0), heads * vdim), batch, n, m - n, heads, dim,
                                                vdim, window, float(scale), _ptr(sink), dtype_code(q.dtype), _status_ptr(dev), stream_ptr(dev))
@@ -840,7 +840,7 @@ def window_attention(q, k, v, batch, heads, dim, vdim, window, scale, sink=None)
     return out
 
 
-@torch.no_grad()
+@without_grad
 def latent_decode(q, w_uk, w_uv, cache, pos, heads, dim, vdim, window, scale, sink=None):
     """One token per sequence at position pos[0] (its latent is in the cache already): window attention straight on the
     cached latents, W_uk applied to the query and W_uv to the weighted latent.  q (batch, heads * dim), w_uk (heads * dim,
@@ -857,7 +857,7 @@ def latent_decode(q, w_uk, w_uv, cache, pos, heads, dim, vdim, window, scale, si
     window = min(window, ring)
     need = lib.b200_latent_decode_workspace_bytes(B, heads, R, window, dt)
     ws = torch.empty((need,), device=dev, dtype=torch.uint8)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib.b200_latent_decode(q.data_ptr(), max(q.stride(0), heads * dim), w_uk.data_ptr(), w_uv.data_ptr(), cache.data_ptr(), out.data_ptr(),
                                     max(out.stride(0), heads * vdim), B, heads, dim, vdim, R, ring, window, float(scale), _ptr(sink), dt, pos.data_ptr(),
                                     ws.data_ptr(), need, stream_ptr(dev))
@@ -866,7 +866,7 @@ def latent_decode(q, w_uk, w_uv, cache, pos, heads, dim, vdim, window, scale, si
 
 
 # ----------------------------------------------------------------------------- decayed linear attention
-@torch.no_grad()
+@without_grad
 def decayed_attention(qkvg, offsets, decay, weight, state, batch, heads, dim, vdim, eps, *, fresh=False):
     """S <- decay * S + k v^T, o = S^T q per head over the n tokens of each sequence, then o * weight * gate as NormedRows of
     an RMS norm over all heads * vdim columns.  qkvg (batch * n, .) holds q | k | v | gate from the columns 0 and
@@ -884,7 +884,7 @@ def decayed_attention(qkvg, offsets, decay, weight, state, batch, heads, dim, vd
     sumsq = torch.empty((lib.b200_decayed_attention_slices(n, heads, dim, vdim, dt), M), device=dev, dtype=torch.float32)
     need = lib.b200_decayed_attention_workspace_bytes(batch, n, heads, dim, vdim, dt)
     ws = torch.empty((need,), device=dev, dtype=torch.uint8) if need else None
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib.b200_decayed_attention(qkvg.data_ptr(), max(qkvg.stride(0), qkvg.shape[1]), *offsets, decay.data_ptr(), weight.data_ptr(), state.data_ptr(),
                                         int(bool(fresh)), y.data_ptr(), max(y.stride(0), heads * vdim), sumsq.data_ptr(), M, batch, n, heads, dim, vdim, dt,
                                         _ptr(ws), need, _status_ptr(dev), stream_ptr(dev))
@@ -897,7 +897,7 @@ def _pitch(t):
     return max(t.stride(0), t.shape[1])
 
 
-@torch.no_grad()
+@without_grad
 def stream_update(x, eps, *, y=None, y_gain=None, ids=None, table=None, table_scale=1.0, shift=None, gain=None, out_dtype=None):
     """One pass over an fp32 stream between two sublayers: x += norm(y) * y_gain + table[ids] * table_scale + shift, each
     optional, in place; with `gain` returns norm(x) * gain in `out_dtype`, the rows of the next product.  `x` an int: a new
@@ -926,7 +926,7 @@ def stream_update(x, eps, *, y=None, y_gain=None, ids=None, table=None, table_sc
     if gain is not None:
         rows = _rows_empty(p.T, p.W, dtype, dev)
         p.h, p.ld_h = rows.data_ptr(), _pitch(rows)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(_lib.load().b200_stream_update(ctypes.byref(p), stream_ptr(dev)), "stream_update")
     return x, rows
 
@@ -943,7 +943,7 @@ def interleave_gated(gate, up):
     return torch.cat([pad(gate), pad(up)], dim=1).reshape(2 * blocks * GATED_BLOCK, *gate.shape[1:]).contiguous()
 
 
-@torch.no_grad()
+@without_grad
 def gated_linear(rows, weight, bias, ff, *, limit, alpha):
     """gate * sigmoid(alpha * gate) * (up + 1), gate = min(., limit) and up = clamp(., -limit, limit) being the two halves of
     rows @ weight^T + bias, weight and bias from `interleave_gated`; (M, ff)."""
@@ -954,11 +954,11 @@ def gated_linear(rows, weight, bias, ff, *, limit, alpha):
         assert bias.dtype == torch.float32 and bias.shape == (p.N,) and bias.is_contiguous() and bias.device == dev
         p.out, p.ld_out, p.out_dtype, p.act_split = out.data_ptr(), _pitch(out), dtype_code(out.dtype), p.N
         p.bias, p.pair_cols, p.pair_limit, p.pair_alpha = bias.data_ptr(), ff, limit, alpha
-        with torch.cuda.device(dev):
+        with on_device(dev):
             check(lib.b200_linear(ctypes.byref(p), stream_ptr(dev)), "gated_linear")
         return out
     z = linear(rows, weight, bias=bias)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         st = lib.b200_gated_pairs(z.data_ptr(), _pitch(z), out.data_ptr(), _pitch(out), p.M, ff, limit, alpha, dtype_code(z.dtype), stream_ptr(dev))
     check(st, "gated_linear")
     return out
@@ -971,7 +971,7 @@ def rotary_frequencies(base, dims, device):
     return torch.stack([hi, (f - hi.double()).float()], dim=1).contiguous().to(device)
 
 
-@torch.no_grad()
+@without_grad
 def rotary_append(qkv, offsets, q_weight, k_weight, freq, eps, batch, *, q_heads, kv_heads, maps, dim, vdim, cache=None, hist=0, start=0, pos=None,
                   keep_rows=True, v_dtype=None):
     """RMS norm per head and rotation by position of the queries (in place) and keys of qkv (batch * n, .), whose keys and
@@ -999,7 +999,7 @@ def rotary_append(qkv, offsets, q_weight, k_weight, freq, eps, batch, *, q_heads
         k = _rows_empty(batch * (hist + p.n), kv_heads * maps * dim, qkv.dtype, dev)
         v = _rows_empty(batch * (hist + p.n), kv_heads * vdim, v_dtype or qkv.dtype, dev)
         p.k_rows, p.ld_k, p.v_rows, p.ld_v = k.data_ptr(), _pitch(k), v.data_ptr(), _pitch(v)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(_lib.load().b200_rotary_append(ctypes.byref(p), stream_ptr(dev)), "rotary_append")
     return k, v
 
@@ -1009,7 +1009,7 @@ def pair_attention_v_dtype(dim, vdim, dtype):
     return _lib.CODE_TO_TORCH[_lib.load().b200_pair_attention_v_dtype(dim, vdim, dtype_code(dtype))]
 
 
-@torch.no_grad()
+@without_grad
 def pair_attention(q, k, v, gate, lam, batch, *, heads, kv_heads, dim, vdim, window, scale, softcap, eps, out_scale, pos=None):
     """Differential attention with a sliding window: per head two softmax maps over the same values, a1 - lam * a2, RMS-normed
     over vdim, times out_scale and the head's gate (batch * n, heads).  A prompt: q (batch * n, .) are the last n positions
@@ -1043,7 +1043,7 @@ def pair_attention(q, k, v, gate, lam, batch, *, heads, kv_heads, dim, vdim, win
     p.workspace_bytes = lib.b200_pair_attention_workspace_bytes(ctypes.byref(p))
     ws = torch.empty((p.workspace_bytes,), device=dev, dtype=torch.uint8) if p.workspace_bytes else None
     p.workspace = _ptr(ws)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.b200_pair_attention(ctypes.byref(p), stream_ptr(dev)), "pair_attention")
     return out
 
@@ -1052,7 +1052,7 @@ def pair_attention(q, k, v, gate, lam, batch, *, heads, kv_heads, dim, vdim, win
 UNIT_EPS = 1e-6
 
 
-@torch.no_grad()
+@without_grad
 def gated_delta(rows, offsets, conv_w, a_log, dt_bias, norm_w, state, conv_state, batch, *, heads, kv_heads, dim, vdim, eps, q_scale, start=0, pos=None):
     """Short convolutions, unit norms and the gated delta rule over the n tokens of each sequence, the output normed per head
     and gated; (batch * n, heads * vdim).  rows (batch * n, .) holds q | k | v | a | b | gate from the columns 0 and `offsets`
@@ -1083,6 +1083,6 @@ def gated_delta(rows, offsets, conv_w, a_log, dt_bias, norm_w, state, conv_state
     p.workspace_bytes = lib.b200_delta_workspace_bytes(ctypes.byref(p))
     ws = torch.empty((p.workspace_bytes,), device=dev, dtype=torch.uint8) if p.workspace_bytes else None
     p.workspace = _ptr(ws)
-    with torch.cuda.device(dev):
+    with on_device(dev):
         check(lib.b200_delta(ctypes.byref(p), stream_ptr(dev)), "gated_delta")
     return y

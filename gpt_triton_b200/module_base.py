@@ -20,7 +20,7 @@ class _OperandCache:
 
     @staticmethod
     def _tag(param):
-        return (param.data_ptr(), param._version, param.dtype, param.device, tuple(param.shape))
+        return (param.data_ptr(), param._version, param.dtype, param.device, param.shape)
 
     def derived(self, key, params, make):
         """`make()` cached under `key` until one of `params` changes."""
