@@ -52,7 +52,7 @@ constexpr int EPI_COLS = BN / (NUM_EPI_WARPS / 4);  // columns per epilogue warp
 constexpr int EPI_CHUNKS = EPI_COLS / 32;
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_ROWS = 2048;  // rows per raster group (keeps a group's A rows and B columns L2-resident)
-constexpr int CTRL_BYTES = 256;   // mbarriers, tensor-memory base, abort flag
+constexpr int CTRL_BYTES = 512;   // mbarriers, tensor-memory base, abort flag
 constexpr int BIAS_BYTES = 2 * BN * 4;  // bias of the current and the next tile, as fp32
 constexpr int EPI_BOX_COLS = 64;        // TMA store box: 64 columns (128 bytes of 16-bit data) x 32 rows
 constexpr int EPI_BOX_BYTES = 32 * EPI_BOX_COLS * 2;        // 4 KB
@@ -475,6 +475,74 @@ __device__ __forceinline__ void residual_chunk(const uint32_t (&acc)[CW], const 
     }
   }
 }
+// fp32 results of one thread's row, 32 columns, through a staging box (32 rows of 128 bytes, 128-byte swizzle) that holds the
+// residual if there is one and takes the result: LN == 0, 3 (bias, activation) and 4 (the residual stream, see residual_chunk).
+// From registers a warp's accesses touch 32 rows each, and the load/store unit took longer over a tile than its main loop.
+template <typename OutT, bool GELU, int LN>
+__device__ __forceinline__ void f32_staged_chunk(const uint32_t (&acc)[32], const float* bias_s, const EpilogueArgs<OutT>& e, int64_t row, bool row_ok, int col0,
+                                                 int64_t N, bool gx_wide, float row_scale, uint32_t box, bool has_res, int lane, float& sq) {
+  const uint32_t rowaddr = box + (uint32_t)lane * 128u, sw = (uint32_t)(lane & 7);
+  const bool full = col0 + 32 <= N;
+  float f[32];
+  if constexpr (LN == 4) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(acc[j]);
+  } else if constexpr (LN == 3) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(acc[j]) * row_scale;
+    if (e.fbias) add_bias_chunk(f, e.fbias, col0, N);
+    activate_chunk(f, col0, e.act_lo, e.act_hi, e.act_split, e.act_param);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(acc[j]);
+    if (e.bias) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] += bias_s[j];
+    }
+    if constexpr (GELU) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] = gelu_fast(f[j]);
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    const uint32_t at = rowaddr + ((((uint32_t)g) ^ sw) << 4);
+    if (LN == 4 || has_res) {
+      uint32_t r[4];
+      ld_shared_v4(at, r);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (LN == 4) {
+          f[4 * g + j] = fmaf(row_scale, f[4 * g + j], __uint_as_float(r[j]));
+          if (full || col0 + 4 * g + j < N) sq = fmaf(f[4 * g + j], f[4 * g + j], sq);
+        } else {
+          f[4 * g + j] += __uint_as_float(r[j]);
+        }
+      }
+    }
+    st_shared_v4(at, __float_as_uint(f[4 * g]), __float_as_uint(f[4 * g + 1]), __float_as_uint(f[4 * g + 2]), __float_as_uint(f[4 * g + 3]));
+  }
+  if constexpr (LN == 4) {
+    if (e.gain && row_ok) {
+      __nv_bfloat16* grow = e.gx + row * e.ld_gx + col0;
+      if (gx_wide && full) {
+        uint32_t w[16];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          const float4 gn = __ldg(reinterpret_cast<const float4*>(e.gain + col0) + g);
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(f[4 * g] * gn.x, f[4 * g + 1] * gn.y), hi = __floats2bfloat162_rn(f[4 * g + 2] * gn.z, f[4 * g + 3] * gn.w);
+          w[2 * g] = *reinterpret_cast<const uint32_t*>(&lo), w[2 * g + 1] = *reinterpret_cast<const uint32_t*>(&hi);
+        }
+        st_global_v8(grow, reinterpret_cast<const uint32_t(&)[8]>(w[0]));
+        st_global_v8(grow + 16, reinterpret_cast<const uint32_t(&)[8]>(w[8]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (col0 + j < N) grow[j] = __float2bfloat16_rn(f[j] * e.gain[col0 + j]);
+      }
+    }
+  }
+}
 // Whether residual_chunk's 32-byte accesses are allowed.
 template <typename OutT>
 __device__ __forceinline__ bool residual_rows_wide(const EpilogueArgs<OutT>& e) {
@@ -848,8 +916,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t bar_acc_full = bar_empty + 8 * STAGES;
   const uint32_t bar_acc_empty = bar_acc_full + 16;
   const uint32_t bar_bias = bar_acc_empty + 16;
-  const uint32_t bar_res = bar_bias + 16;  // [NUM_EPI_WARPS]: residual boxes of a warp have landed
-  constexpr int NUM_BARS = 2 * STAGES + 6 + NUM_EPI_WARPS;
+  const uint32_t bar_res = bar_bias + 16;  // [NUM_EPI_WARPS][2]: residual boxes of a warp have landed (16-bit: both on the first)
+  constexpr int NUM_BARS = 2 * STAGES + 6 + 2 * NUM_EPI_WARPS;
   static_assert(8 * NUM_BARS + 16 <= CTRL_BYTES, "control block too small");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 8 * NUM_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 8 * NUM_BARS + 8);
@@ -877,7 +945,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(bar_acc_empty + 8 * a, NUM_EPI_WARPS * CTAS);  // the leader's barrier collects both CTAs' epilogue warps
       mbar_init(bar_bias + 8 * a, NUM_EPI_WARPS);
     }
-    for (int w = 0; w < NUM_EPI_WARPS; ++w) mbar_init(bar_res + 8 * w, 1);
+    for (int w = 0; w < 2 * NUM_EPI_WARPS; ++w) mbar_init(bar_res + 8 * w, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1001,8 +1069,12 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const bool res_tma = use_tma && epi.residual != nullptr;  // (the host only sets tma_store when the residual can be mapped too)
     const uint32_t stage_addr = use_tma ? smem_epi + (uint32_t)(warp - 2) * EPI_WARP_STAGE_BYTES : 0u;
     const uint32_t stats_stage = smem_epi + (uint32_t)(warp - 2) * EPI_WARP_STAGE_BYTES;  // statistics-only launches park chunks here
-    const uint32_t my_res_bar = bar_res + 8 * (uint32_t)(warp - 2);
-    uint32_t res_phase = 0;
+    const uint32_t my_res_bar = bar_res + 16 * (uint32_t)(warp - 2);
+    uint32_t res_phase = 0;  // (fp32: one bit per box)
+    // fp32 results leave through the same two boxes, 32 rows x 32 columns each, chunk by chunk
+    const bool f32_tma = sizeof(OutT) == 4 && STATS == 0 && epi.tma_store != 0;
+    const bool f32_res = f32_tma && (LN == 4 || epi.residual != nullptr);
+    const uint32_t f32_stage = smem_epi + (uint32_t)(warp - 2) * EPI_WARP_STAGE_BYTES;
     const uint64_t out_policy = l2_policy_evict_first();
     bool x_wide = false;
     if constexpr (LN == 4) x_wide = residual_rows_wide(epi);
@@ -1027,6 +1099,21 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         __syncwarp();
       }
+      if (f32_tma) {
+        if (lane == 0) {
+          tma_store_wait_read();  // the previous tile's stores have read both boxes
+          if (f32_res) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+              if (col_base + b * 32 < N) {
+                mbar_arrive_expect_tx(my_res_bar + 8 * b, EPI_BOX_BYTES);
+                tma_load_2d(f32_stage + b * EPI_BOX_BYTES, &map_res, my_res_bar + 8 * b, col_base + b * 32, row_warp);
+              }
+            }
+          }
+        }
+        __syncwarp();
+      }
       float* bias_s = bias_smem + acc * BN;
       for (int i = epi_tid; i < BN; i += 32 * NUM_EPI_WARPS) {
         const int c = tc.n * BN + i;
@@ -1041,8 +1128,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (row_ok) ln_r = deferred_row_scale(epi, row);
       }
       if constexpr (LN == 4) {
-        // the residual rows are read straight from global memory: start them towards L2 while the main loop runs
-        if (row_ok) {
+        // without staging the residual rows are read straight from global memory: start them towards L2 while the main loop runs
+        if (row_ok && !f32_tma) {
 #pragma unroll
           for (int i = 0; i < EPI_COLS; i += 32)
             if (col_base + i < N) asm volatile("prefetch.global.L2 [%0];" ::"l"(epi.x + row * epi.ld_x + col_base + i));
@@ -1127,6 +1214,31 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               stats_only_chunk<OutT>(v, bias_s + col_half * EPI_COLS + c * 32, epi.bias != nullptr, epi.amax_sum != nullptr, col0, N, tgt,
                                      stats_stage + (uint32_t)(c >> 1) * EPI_BOX_BYTES, c & 1, lane, stats, picked);
           }
+        } else if (f32_tma) {
+          if (col0 < N) {  // (warp-uniform)
+            const uint32_t box = f32_stage + (uint32_t)(c & 1) * EPI_BOX_BYTES;
+            if (f32_res) {
+              if (c >= 1 && c + 1 < EPI_CHUNKS && col0 + 32 < N && lane == 0) {
+                // the other box: its store, one chunk ago, has been read; the chunk behind this one lands in it
+                tma_store_wait_read();
+                const uint32_t other = (uint32_t)((c + 1) & 1);
+                mbar_arrive_expect_tx(my_res_bar + 8 * other, EPI_BOX_BYTES);
+                tma_load_2d(f32_stage + other * EPI_BOX_BYTES, &map_res, my_res_bar + 8 * other, col0 + 32, row_warp);
+              }
+              if (!mbar_wait(my_res_bar + 8 * (uint32_t)(c & 1), (res_phase >> (c & 1)) & 1u, abort_flag, status_word, 6)) break;
+              res_phase ^= 1u << (c & 1);
+            } else if (c >= 2) {
+              if (lane == 0) tma_store_wait_read_but_one();
+              __syncwarp();
+            }
+            f32_staged_chunk<OutT, GELU, LN>(v, bias_s + col_half * EPI_COLS + c * 32, epi, row, row_ok, col0, N, x_wide, ln_r, box, f32_res, lane, mom.s2);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (row_warp < M) tma_store_2d(&map_out, box, col0, row_warp);
+              tma_store_commit();
+            }
+          }
         } else if constexpr (LN == 4) {
           if (row_ok && col0 < N) residual_chunk(v, epi, row, col0, N, x_wide, ln_r, mom.s2);
         } else if (use_tma) {
@@ -1193,7 +1305,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         acc_phase ^= 1u;
       }
     }
-    if (use_tma && lane == 0) tma_store_wait_read();  // staging memory must outlive the last bulk store's read
+    if ((use_tma || f32_tma) && lane == 0) tma_store_wait_read();  // staging memory must outlive the last bulk store's read
   }
 
   // ------------------------------------------------------------ teardown
@@ -1763,6 +1875,13 @@ static int make_out_map(CUtensorMap* map, void* ptr, int64_t M, int64_t N, int64
   return encode_tensor_map(map, ptr, 2, dims, strides, box, io_dtype, CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
+// The same over an fp32 matrix: boxes of 32 columns x 32 rows.
+static int make_f32_map(CUtensorMap* map, const void* ptr, int64_t M, int64_t N, int64_t ld) {
+  const uint64_t dims[2] = {(uint64_t)N, (uint64_t)M}, strides[1] = {(uint64_t)ld * 4};
+  const uint32_t box[2] = {32, 32};
+  return encode_tensor_map(map, ptr, 2, dims, strides, box, B200_F32, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+}
+
 template <typename OutT, bool GELU, int CTAS, int STATS, int LN>
 static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mr, const CUtensorMap& mae,
                           const CUtensorMap& mbe, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int op_dtype, int64_t groups,
@@ -1929,8 +2048,17 @@ static int launch_wide(const void* a, const void* b, EpilogueArgs<OutT> epi, int
       make_out_map(&mo, epi.out, M, LN == 5 ? epi.pair_cols : N, epi.ld_out, DType<OutT>::code) == B200_OK &&
       (!epi.residual || make_out_map(&mr, const_cast<OutT*>(epi.residual), M, N, epi.ld_res, DType<OutT>::code) == B200_OK))
     epi.tma_store = 1;
+  if constexpr (sizeof(OutT) == 4 && STATS == 0) {
+    // fp32 results (LN == 4: the residual stream, in place): the same, in boxes of 32 columns
+    const void* out = LN == 4 ? static_cast<const void*>(epi.x) : epi.out;
+    const void* res = LN == 4 ? out : epi.residual;
+    const int64_t ld = LN == 4 ? epi.ld_x : epi.ld_out, ld_res = LN == 4 ? epi.ld_x : epi.ld_res;
+    if (((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(res)) & 15) == 0 && ld % 4 == 0 && (!res || ld_res % 4 == 0) &&
+        make_f32_map(&mo, out, M, N, ld) == B200_OK && (!res || make_f32_map(&mr, res, M, N, ld_res) == B200_OK))
+      epi.tma_store = 1;
+  }
   if ((LN == 1 || LN == 2 || LN == 5) && !epi.tma_store) return B200_ERR_UNSUPPORTED;  // these epilogues exist on the staged 16-bit path only
-  epi.stream_out = epi.tma_store && (double)N * (double)K * 2.0 >= 32e6 && (double)M * (double)N * sizeof(OutT) >= 512e6;
+  epi.stream_out = epi.tma_store && sizeof(OutT) == 2 && (double)N * (double)K * 2.0 >= 32e6 && (double)M * (double)N * sizeof(OutT) >= 512e6;
   const int64_t n_tiles = (N + BN - 1) / BN;
   const int pairs = M > BM ? max_pairs<OutT, GELU, STATS, LN>() : 0;
   CUtensorMap ma, mb, mae, mbe;

@@ -190,7 +190,7 @@ inline EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// Tiled tensor map over 16-bit data, 128-byte swizzle, no interleave, zero fill: the only kind this library uses.
+// Tiled tensor map over 16-bit or fp32 data, 128-byte swizzle, no interleave, zero fill: the only kind this library uses.
 // Encoding one costs the host about a microsecond and a forward pass asks for the same few hundred maps again and
 // again, so encoded maps are kept in a process-wide table keyed by everything that goes into the encoding (base
 // pointer, extents, byte strides, box, element type, L2 promotion).  A map owns nothing: an entry stays correct for
@@ -236,7 +236,7 @@ inline int encode_tensor_map(CUtensorMap* out, const void* ptr, int rank, const 
   cuuint32_t bx[4], estr[4] = {1, 1, 1, 1};
   for (int i = 0; i < rank; ++i) d[i] = dims[i], bx[i] = box[i];
   for (int i = 0; i + 1 < rank; ++i) st[i] = strides[i];
-  const CUresult r = fn(out, dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank,
+  const CUresult r = fn(out, dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : dtype == B200_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank,
                         const_cast<void*>(ptr), d, st, bx, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promotion,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return B200_ERR_CUDA;
