@@ -540,12 +540,13 @@ def _bhl_strides(t):
 
 
 @without_grad
-def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False):
+def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False, out_dtype=None):
     """Causal softmax(q k^T / sqrt(H)) v with the reference's 64-key online softmax
     (reference kernels.py:478-525).  q, k, v: (batch, heads, seqlen, head_size), contiguous or
     strided views with a contiguous last dim.  Returns a contiguous (B, N, L, H) tensor, or with
     ``merged_heads=True`` the (B, L, N*H) tensor the reference gets by transposing afterwards
-    (gpt.py:51)."""
+    (gpt.py:51).  ``out_dtype=torch.float16`` rounds the result of float32 tensors on its way out, for a
+    product that takes it as an operand."""
     _no_dropout(dropout_prob)
     require_cuda(q, k, v)
     assert q.shape[:2] == k.shape[:2]
@@ -558,10 +559,10 @@ def flash_attention_v1(q, k, v, dropout_prob=0.0, *, merged_heads=False):
     assert q.dtype == k.dtype == v.dtype
     dev = _same_device(q, k, v)
     if merged_heads:
-        z = torch.empty((B, Lq, N, H), device=dev, dtype=q.dtype)
+        z = torch.empty((B, Lq, N, H), device=dev, dtype=out_dtype or q.dtype)
         zv = z.transpose(1, 2)
     else:
-        z = torch.empty((B, N, Lq, H), device=dev, dtype=q.dtype)
+        z = torch.empty((B, N, Lq, H), device=dev, dtype=out_dtype or q.dtype)
         zv = z
     scale = 1 / math.sqrt(H)
     with on_device(dev):
