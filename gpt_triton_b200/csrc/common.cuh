@@ -161,10 +161,18 @@ __device__ __forceinline__ float gelu_new(float x) {
 // A kernel launched with the programmatic-stream-serialization attribute may start while its predecessor in the
 // stream is still running.  pdl_wait() blocks until the predecessor grid has completed and its memory is visible, so
 // what a kernel does before it (barrier set-up, tensor-memory allocation) overlaps the predecessor's tail;
-// pdl_launch_dependents() lets the successor's CTAs be scheduled as soon as SM resources free up.  Both are no-ops in a
-// kernel launched without the attribute.  Every CTA of every kernel that is launched with the attribute calls
-// pdl_wait() before its first access to global memory, on every path, so that "my predecessor has completed" stays
-// transitive along the stream (kernels launched without it are serialised by the stream as usual).
+// pdl_launch_dependents() lets the successor's CTAs be scheduled as soon as SM resources free up, if the successor is
+// launched with the attribute.  pdl_wait() is a no-op in a kernel launched without it.  Rules:
+//   - every CTA of every kernel that is launched with the attribute calls pdl_wait() on every path, so that "my
+//     predecessor has completed" stays transitive along the stream (kernels launched without it are serialised by the
+//     stream as usual), and before it writes global memory;
+//   - before pdl_wait() global memory is only prefetched, or read for a value that decides nothing but what is
+//     prefetched (gemm_few_kernel, attention_decode_kernel);
+//   - such a kernel's life begins before the kernels in front have written its inputs.  __ldg and const __restrict__
+//     pointers promise that nobody writes the data during that life, and a load through a __restrict__ pointer that
+//     depends on nothing behind pdl_wait() may be moved ahead of it: weights, biases and gains only.  What another
+//     kernel of a pass writes (rows, row sums and statistics, ids, positions) is read by ordinary loads through ordinary
+//     pointers.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

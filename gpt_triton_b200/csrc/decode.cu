@@ -97,8 +97,8 @@ __device__ __forceinline__ float warp_max(float v) {
 // before; 512, 1000 keys 305 -> 272 (242).
 template <typename T, int D, int SPLIT, bool AHEAD>
 __global__ void __launch_bounds__(SPLIT == 1 ? 128 : 32 * SPLIT)
-attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T* __restrict__ out, int64_t BH, int NH, int64_t cache_len,
-                        float scale_log2e, const int* __restrict__ pos_dev, int* status_word) {
+attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__ out, int64_t BH, int NH, int64_t cache_len, float scale_log2e,
+                        const int* pos_dev, int* status_word) {
   constexpr int WARPS = SPLIT == 1 ? 4 : SPLIT;
   __shared__ __align__(16) float q_s[WARPS][D + 4];  // the second half of q sits 4 floats further on: the two lanes of a pair read different banks
   __shared__ float part_o[SPLIT == 1 ? 1 : WARPS][D];
@@ -138,6 +138,7 @@ attention_decode_kernel(const T* __restrict__ qkv_new, T* __restrict__ cache, T*
     }
   }
   pdl_wait();
+  // (an ordinary load behind the wait, on which every load of the cache depends: the cache may stay __restrict__, see common.cuh)
   const int pos = pos_dev[0];
   if (pos < 0 || pos >= cache_len) {
     if (threadIdx.x == 0 && status_word) atomicCAS(status_word, 0, kSiteCachePosition);

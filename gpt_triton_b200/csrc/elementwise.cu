@@ -49,9 +49,9 @@ constexpr int kWarpsPerBlock = 8;
 // rows of its input.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-embedding_kernel(const int64_t* __restrict__ ids, const T* __restrict__ wte, const T* __restrict__ wpe,
+embedding_kernel(const int64_t* ids, const T* __restrict__ wte, const T* __restrict__ wpe,
                  T* __restrict__ out, int64_t T_rows, int64_t L, int64_t V, int64_t H, int* bad_id_flag, float2* __restrict__ stats, T* __restrict__ ext,
-                 float eps, const int* __restrict__ pos0_dev, int64_t P) {
+                 float eps, const int* pos0_dev, int64_t P) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
@@ -112,7 +112,7 @@ embedding_kernel(const int64_t* __restrict__ ids, const T* __restrict__ wte, con
 // no kernel of this library produced.
 template <typename T>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-row_ln_stats_kernel(const T* __restrict__ x, int64_t M, int64_t H, float eps, float2* __restrict__ stats, T* __restrict__ ext) {
+row_ln_stats_kernel(const T* x, int64_t M, int64_t H, float eps, float2* __restrict__ stats, T* __restrict__ ext) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
@@ -260,7 +260,7 @@ int launch_embedding_rms(const int64_t* ids, const void* table, const float* gai
 // registers, not over memory).
 template <typename TI, typename TO, int NV>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-layernorm_vec_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* __restrict__ b, TO* __restrict__ out,
+layernorm_vec_kernel(const TI* x, const TI* __restrict__ w, const TI* __restrict__ b, TO* __restrict__ out,
                      int64_t M, int H, float eps) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -314,7 +314,7 @@ layernorm_vec_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const T
 // Any H, any alignment: three passes over the row (it stays in L1 after the first).
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-layernorm_generic_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* __restrict__ b,
+layernorm_generic_kernel(const TI* x, const TI* __restrict__ w, const TI* __restrict__ b,
                          TO* __restrict__ out, int64_t M, int64_t H, float eps) {
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);

@@ -13,8 +13,8 @@ namespace b200 {
 constexpr int kReduceRows = 32, kReduceSplit = 8;
 __device__ __forceinline__ int partial_column(int enc) { return enc < 0 ? -enc - 1 : enc; }
 __global__ void __launch_bounds__(kReduceRows * kReduceSplit)
-argmax_reduce_kernel(const float* __restrict__ val, const int* __restrict__ idx, const float* __restrict__ sum, int64_t ld, int slices,
-                     int64_t M, int64_t* __restrict__ out, float* __restrict__ lse_out, const void* __restrict__ product, int64_t ld_product,
+argmax_reduce_kernel(const float* val, const int* idx, const float* sum, int64_t ld, int slices,
+                     int64_t M, int64_t* __restrict__ out, float* __restrict__ lse_out, const void* product, int64_t ld_product,
                      int product_is_bf16, int64_t N) {
   __shared__ float s_val[kReduceSplit][kReduceRows];
   __shared__ int s_idx[kReduceSplit][kReduceRows];
@@ -87,7 +87,7 @@ static int launch_argmax_reduce(const float* val, const int* idx, const float* s
 // row; the slices of 32 consecutive rows are consecutive in memory.
 template <typename T>
 __global__ void __launch_bounds__(256)
-ln_stats_from_moments_kernel(const float2* __restrict__ moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int64_t M,
+ln_stats_from_moments_kernel(const float2* moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int64_t M,
                              float2* __restrict__ stats, T* __restrict__ ext) {
   const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
@@ -132,7 +132,7 @@ ln_stats_from_moments_kernel(const float2* __restrict__ moments, int64_t ld, int
 // thread took 4.6 us at 16 rows and 48 slices, this takes 2.
 template <typename T>
 __global__ void __launch_bounds__(256)
-ln_stats_few_rows_kernel(const float2* __restrict__ moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int M,
+ln_stats_few_rows_kernel(const float2* moments, int64_t ld, int slices, int slice_cols, int cols, float eps, int M,
                          float2* __restrict__ stats, T* __restrict__ ext) {
   const int row = (int)blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   pdl_launch_dependents();

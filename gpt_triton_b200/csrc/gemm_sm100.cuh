@@ -201,11 +201,11 @@ __device__ __forceinline__ float deferred_row_scale(const EpilogueArgs<OutT>& e,
   int i = 0;
   for (; i + kSumsqParts <= e.sq_slices; i += kSumsqParts) {
 #pragma unroll
-    for (int j = 0; j < kSumsqParts; ++j) p[j] += __ldg(e.sq_in + (int64_t)(i + j) * e.sq_in_ld + row);
+    for (int j = 0; j < kSumsqParts; ++j) p[j] += e.sq_in[(int64_t)(i + j) * e.sq_in_ld + row];
   }
 #pragma unroll
   for (int j = 0; j < kSumsqParts - 1; ++j)
-    if (i + j < e.sq_slices) p[j] += __ldg(e.sq_in + (int64_t)(i + j) * e.sq_in_ld + row);
+    if (i + j < e.sq_slices) p[j] += e.sq_in[(int64_t)(i + j) * e.sq_in_ld + row];
   return e.out_scale / sqrtf(merge_sumsq_parts(p) / e.sq_cols + e.eps);
 }
 
@@ -1122,7 +1122,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // folded LayerNorm: this row's rstd
       float ln_r = 1.f;
       if constexpr (LN == 1) {
-        if (row_ok) ln_r = __ldg(epi.ln_stats + row).y;
+        if (row_ok) ln_r = epi.ln_stats[row].y;
       }
       if constexpr (LN >= 3) {
         if (row_ok) ln_r = deferred_row_scale(epi, row);
@@ -1440,7 +1440,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
     float ln_r = 1.f;
     if constexpr (LN == 1) {
-      if (row_ok) ln_r = __ldg(epi.ln_stats + row).y;
+      if (row_ok) ln_r = epi.ln_stats[row].y;
     }
     if constexpr (LN >= 3) {
       if (row_ok) ln_r = deferred_row_scale(epi, row);
@@ -1703,7 +1703,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           float s = 0.f;
           if (m0 + r < M) {
 #pragma unroll 4
-            for (int i = part; i < epi.sq_slices; i += kSumsqParts) s += __ldg(epi.sq_in + (int64_t)i * epi.sq_in_ld + m0 + r);
+            for (int i = part; i < epi.sq_slices; i += kSumsqParts) s += epi.sq_in[(int64_t)i * epi.sq_in_ld + m0 + r];
           }
           parts_s[part * kFewMaxRows + r] = s;
         }
@@ -1712,7 +1712,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps only
     float ln_r = 1.f;
     if constexpr (LN == 1) {
-      if (row_ok) ln_r = __ldg(epi.ln_stats + row).y;
+      if (row_ok) ln_r = epi.ln_stats[row].y;
     }
     if constexpr (LN >= 3) {
       ln_r = epi.out_scale;
