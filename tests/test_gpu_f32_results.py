@@ -55,3 +55,45 @@ def test_residual_stream_and_row_sums(rows, K_, N):
     logits = K.linear(normed, K.operand_rows(w.to(DEV))[0], out_dtype=torch.float32)
     assert ((logits.double().cpu() - z).abs() <= bound).all()
     assert K.device_status() == 0
+
+
+# Several tiles of 256 x 256 per CTA pair (20000 rows: 79 row tiles), so that the boxes' barriers are used again from tile to tile;
+# 1056 columns leave one box in the last tile's slice, 1124 a whole tile and an odd number of boxes, 1252 a slice without columns.
+@pytest.mark.parametrize("N", [1056, 1124, 1252])
+def test_many_tiles_with_a_residual(N):
+    from gpt_triton_b200 import kernels as K
+
+    g = torch.Generator(device=DEV).manual_seed(N)
+    rows, K_ = 20000, 64
+    x, w = torch.randn((rows, K_), device=DEV, generator=g), K.pack_weight(torch.randn((K_, N), device=DEV, generator=g) * 0.1)
+    b, r = torch.randn(N, device=DEV, generator=g), torch.randn((rows, N), device=DEV, generator=g)
+    for kw in ({"bias": b, "residual": r}, {"bias": b, "residual": r, "add_gelu": True}, {"bias": b}):
+        odd = torch.full((rows, N + 1), 7.0, device=DEV)
+        K.fused_ffn(x, w, out=odd[:, :N], **kw)
+        assert torch.equal(K.fused_ffn(x, w, **kw), odd[:, :N])
+    assert K.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [1056, 1124, 1252])
+@pytest.mark.parametrize("with_gain", [False, True])
+def test_residual_stream_over_many_tiles(N, with_gain):
+    """Bounds as in test_residual_stream_and_row_sums."""
+    from gpt_triton_b200 import kernels as K
+
+    g = torch.Generator(device=DEV).manual_seed(N)
+    rows, K_ = 20000, 64
+    a, w = torch.randn((rows, K_), device=DEV, generator=g).bfloat16(), (torch.randn((N, K_), device=DEV, generator=g) / 8).bfloat16()
+    sumsq = torch.rand((1, rows), device=DEV, generator=g) * K_ + 1
+    scale = (sumsq[0].double() / K_ + 1e-3).rsqrt()[:, None]
+    z, bound = a.double() @ w.double().T * scale, 2e-6 * (a.double().abs() @ w.double().abs().T * scale) + 1e-6
+    x0, gain = torch.randn((rows, N), device=DEV, generator=g), 1 + 0.1 * torch.randn(N, device=DEV, generator=g)
+    x = x0.clone()
+    nxt = K.linear_residual(K.NormedRows(a, sumsq, K_, 1e-3), K.operand_rows(w)[0], x, gain if with_gain else None, 1e-3)
+    want = x0.double() + z
+    assert ((x.double() - want).abs() <= bound + want.abs() * 2.0 ** -22).all()
+    if with_gain:
+        assert torch.equal(nxt.data, (x * gain).bfloat16())
+        for i in range(nxt.sumsq.shape[0]):
+            part = x.double()[:, i * 128:(i + 1) * 128].pow(2).sum(1)
+            assert ((nxt.sumsq[i].double() - part).abs() <= 1e-5 * part + 1e-9).all()
+    assert K.device_status() == 0
