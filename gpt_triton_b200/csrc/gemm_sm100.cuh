@@ -796,7 +796,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&acc)[CW], const 
     if (col0 + j < N) {
       float v = f[j];
       if (rrow) v += to_float(rrow[j]);
-      if constexpr (LN == 2) {  // (reached by the narrow-tile kernel's ragged last chunk only)
+      if constexpr (LN == 2) {  // (reached by the ragged last chunk of gemm_narrow_kernel and gemm_few_kernel only)
         if (mom.n == 0.f) mom.shift = v;
         const float d = v - mom.shift;
         mom.s1 += d, mom.s2 = fmaf(d, d, mom.s2), mom.n += 1.f;
@@ -1920,25 +1920,29 @@ static constexpr uint32_t make_idesc_narrow(int ab_format) {
   return (1u << 4) | ((uint32_t)ab_format << 7) | ((uint32_t)ab_format << 10) | ((uint32_t)(NARROW_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
-// Columns per CTA: as many as leave one CTA per SM (148), and at least 16, the narrowest tile of an MMA that also holds a
-// 32-byte store.  LN == 4: 16 (four CTAs share a 64-column slice); LN == 5: 64 (one block of gate and up columns).
+// Columns per CTA: the widest of 64 (one row tile only), 32 and 16 whose tiles number more than 13/16 of the SMs (fewer leave too
+// many SMs without weights to read), and at least 16, the narrowest tile of an MMA that also holds a 32-byte store.  LN == 4: 16
+// (four CTAs share a 64-column slice); LN == 5: 64 (one block of gate and up columns).
 inline int few_rows_cols(int64_t M, int64_t N, int ln) {
   if (ln == 4) return 16;
   if (ln == 5) return 64;
   const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows;
-  if (row_tiles == 1 && (N + 63) / 64 > 120) return 64;
-  return (N + 31) / 32 * row_tiles > 120 ? 32 : 16;
+  const int64_t enough = (int64_t)sm_count() * 13 / 16;
+  if (row_tiles == 1 && (N + 63) / 64 > enough) return 64;
+  return (N + 31) / 32 * row_tiles > enough ? 32 : 16;
 }
-// Whether a product of at most kNarrowMaxRows rows goes to gemm_few_kernel: up to 64 rows always, above that as long as its tiles
-// of 64 rows and 16 or 32 columns fit the GPU at once (two CTAs per SM; the clusters of LN == 2 and 4 do not get the last few places).
-// Beyond that its smaller tiles read A and B more often than they help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of
-// gemm_narrow_kernel; LN == 4, 384 rows, 768 x 3072 (288 CTAs): 18.2 against 13.5, 256 rows (192 CTAs): 10.0 against 13.7.
+// Whether a product of at most kNarrowMaxRows rows goes to gemm_few_kernel: up to 64 rows, and above that as long as its tiles of 64
+// rows and 16 or 32 columns fit the GPU at once, two CTAs per SM.  Beyond that its smaller tiles read A and B more often than they
+// help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of gemm_narrow_kernel.  Clusters of four do not get the last few places:
+// LN == 4 at 32 rows, K = 2048: 280 CTAs (N = 4480) 10.2 us against 10.8, 288 CTAs 15.2 against 10.7; N = 8192 18.0 against 12.0.
+// LN == 4 has 16-column tiles whatever N is, so from 17 rows on it is held to that too (up to 16 rows: N = 8192 17.6 against 17.6, N =
+// 10880 24.3 against 26.3).
 inline bool takes_few_rows(int64_t M, int64_t N, int ln) {
-  if (M <= kFewMaxRows) return true;
+  if (M <= (ln == 4 ? 16 : kFewMaxRows)) return true;
   if (ln == 5) return false;
-  const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows;
+  const int64_t row_tiles = (M + kFewMaxRows - 1) / kFewMaxRows, places = 2 * (int64_t)sm_count();
   const int cols = few_rows_cols(M, N, ln);
-  return (N + cols - 1) / cols * row_tiles <= (ln == 4 || ln == 2 ? 256 : 296);
+  return (N + cols - 1) / cols * row_tiles <= (ln == 4 || ln == 2 ? places * 19 / 20 : places);
 }
 
 template <typename OutT, bool GELU, int LN, int NB>

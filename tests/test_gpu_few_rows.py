@@ -76,3 +76,23 @@ def test_products_around_deferred_norms(rows, K_, N):
     ref = zg * torch.sigmoid(1.7 * zg) * (zu + 1)
     assert ((out - ref).abs() <= 4 * (bound[:, :F] + bound[:, F:2 * F]) + ref.abs() * 2.0 ** -8 + 1e-5).all()
     assert K.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 17, 64, 65])
+@pytest.mark.parametrize("N", [4480, 4608, 8192])
+def test_residual_stream_at_the_edge_of_what_fits(rows, N):
+    """Tiles of 16 columns in clusters as long as all of them find room at once (4480 columns), tiles of 64 beyond; bounds as above."""
+    from gpt_triton_b200 import kernels as K
+
+    K_ = 136
+    a, w = _randn(rows, K_, seed=1).bfloat16(), _randn(N, K_, seed=2, scale=K_ ** -0.5).bfloat16()
+    x0, gain = _randn(rows, N, seed=5), 1 + 0.1 * _randn(N, seed=6)
+    x = x0.to(DEV)
+    nxt = K.linear_residual(a.to(DEV), K.operand_rows(w.to(DEV))[0], x, gain.to(DEV), 1e-3)
+    want = x0.double() + a.double() @ w.double().T
+    bound = 2e-6 * (a.double().abs() @ w.double().abs().T) + 1e-6
+    assert ((x.double().cpu() - want).abs() <= bound + want.abs() * 2.0 ** -22).all()
+    assert torch.equal(nxt.data.cpu(), (x.cpu() * gain).bfloat16())
+    part = x.double().cpu().view(rows, N // 64, 64).pow(2).sum(-1).T
+    assert ((nxt.sumsq.double().cpu() - part).abs() <= 1e-5 * part + 1e-9).all()
+    assert K.device_status() == 0
