@@ -11,6 +11,8 @@
 //   attention_decode_kernel   appends the new token's k, v and attends its q over the cache    (B (pos+1) 2H elements read)
 //   sample_rows_kernel        top-k filter + Gumbel-max draw over a row of logits              (passes over B V logits, mostly L2)
 //   decode_append_kernel      tokens[b, column] = next id (also into the buffer the next step embeds); pos += 1
+#include <atomic>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -145,11 +147,28 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
     return;
   }
   if (w >= BH) return;  // (SPLIT > 1: the whole block leaves together)
-  for (int i = lane; i < D; i += 32) {
-    q_s[warp][i + (i >= D / 2 ? 4 : 0)] = dot_operand<T>(to_float(qn[i]));
-    if (part == 0) {
-      kc[(int64_t)pos * pitch + i] = kn[i];
-      vc[(int64_t)pos * pitch + i] = vn[i];
+  // one block of keys: the first warp alone (the host knows how long the cache is, not how many keys it holds; without AHEAD the
+  // registers that this takes cost more than it gives)
+  const bool solo = SPLIT == 1 || (AHEAD && pos < 64);
+  if (solo && part != 0) return;
+  if constexpr (SPLIT == 1) {  // (all loads ahead of the stores; with several warps the registers are dearer)
+    T q_new[DPL], k_new[DPL], v_new[DPL];
+#pragma unroll
+    for (int r = 0; r < DPL; ++r) q_new[r] = qn[r * 32 + lane], k_new[r] = kn[r * 32 + lane], v_new[r] = vn[r * 32 + lane];
+#pragma unroll
+    for (int r = 0; r < DPL; ++r) {
+      const int i = r * 32 + lane;
+      q_s[warp][i + (i >= D / 2 ? 4 : 0)] = dot_operand<T>(to_float(q_new[r]));
+      kc[(int64_t)pos * pitch + i] = k_new[r];
+      vc[(int64_t)pos * pitch + i] = v_new[r];
+    }
+  } else {
+    for (int i = lane; i < D; i += 32) {
+      q_s[warp][i + (i >= D / 2 ? 4 : 0)] = dot_operand<T>(to_float(qn[i]));
+      if (part == 0) {
+        kc[(int64_t)pos * pitch + i] = kn[i];
+        vc[(int64_t)pos * pitch + i] = vn[i];
+      }
     }
   }
   __syncwarp();
@@ -203,7 +222,7 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
     }
     const float bm = warp_max(fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])));
     float m_new = fmaxf(m_all, bm);
-    if (SPLIT > 1) {
+    if (!solo) {
       if (lane == 0) group_max[g & 1][warp] = bm;
       __syncthreads();
 #pragma unroll
@@ -258,7 +277,7 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
   }
   const int col0 = side * DH + kl * DPL;  // first of this lane's DPL output columns
   // o[0 .. DPL) now holds output columns col0 + j of this warp's blocks
-  if (SPLIT > 1) {
+  if (!solo) {
 #pragma unroll
     for (int j = 0; j < DPL; ++j) part_o[warp][col0 + j] = o[j];
     if (lane == 0) part_ml[warp][0] = m_run, part_ml[warp][1] = l_warp;
@@ -295,31 +314,52 @@ int attention_decode_split(const void* qkv_new, void* cache, void* out, int64_t 
   return status_from_cuda(e);
 }
 
+// How many (batch, head) pairs of a variant the current device has room for at once (0 if it cannot be asked).
+template <typename T, int D, int SPLIT, bool AHEAD>
+int64_t heads_at_once() {
+  static std::atomic<int> per_sm[kMaxDevices];  // blocks, + 1; 0: not asked yet
+  const int slot = device_slot();
+  if (slot < 0) return 0;
+  int n = per_sm[slot].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attention_decode_kernel<T, D, SPLIT, AHEAD>, SPLIT == 1 ? 128 : 32 * SPLIT, 0) != cudaSuccess) return 0;
+    per_sm[slot].store(++n, std::memory_order_relaxed);
+  }
+  return (int64_t)(n - 1) * sm_count() * (SPLIT == 1 ? 4 : 1);
+}
+
 template <typename T, int D>
 int attention_decode_sized(const void* qkv_new, void* cache, void* out, int64_t BH, int64_t NH, int64_t cache_len, float sl, const int* pos_dev,
                            int* status_word, cudaStream_t stream) {
-  const int64_t sms = sm_count();
 #define B200_DECODE(SPLIT, AHEAD) return attention_decode_split<T, D, SPLIT, AHEAD>(qkv_new, cache, out, BH, NH, cache_len, sl, pos_dev, status_word, stream)
+#define B200_DECODE_IF_ROOM(SPLIT, AHEAD) \
+  if (BH <= heads_at_once<T, D, SPLIT, AHEAD>()) B200_DECODE(SPLIT, AHEAD)
   if constexpr (sizeof(T) == 2 && D <= 64) {
-    // Warps per (batch, head), us at 12 heads of 64 and 100 / 330 / 1000 keys, the neighbours in brackets:
-    //   8 sequences, eight ahead 4.9 / 6.7 / 12.0 [four ahead 4.3 / 8.2 / 14.8]; 16, four ahead 6.0 / 10.2 / 18.9 [two ahead 5.8 / 11.4 / 24.8];
-    //   32, two ahead 6.6 / 13.4 / 30.1 [four 8.9 / 18.9 / 35.4]; 64, one ahead 9.8 / 20.9 / 49.6, four 11.8 / 20.5 / 42.3;
-    //   128, two 12.7 / 31.3 / 78.1 [one 17.4 / 45.3 / 124]; 256, one 20.9 / 56.0 / 155 [two 23.4 / 60.7 / 160]: these warps are about as many
-    //   as find room at once (24 per SM); 512, two 37.7 / 100 / 272 [one 39.1 / 107 / 304].
-    if (BH <= sms) B200_DECODE(8, true);
-    if (BH <= 2 * sms) B200_DECODE(4, true);
-    if (BH <= 4 * sms) B200_DECODE(2, true);
-    if (BH <= 8 * sms) {
-      if (cache_len <= 256) B200_DECODE(1, true);
-      B200_DECODE(4, false);
+    // Most warps per (batch, head) whose launch still finds room at once: a second wave of blocks costs nearly as much as the first
+    // (12 heads of 64, bf16, 222 sequences are one wave at one warp, 1.1 at two: 52.8 us against 58.4 at 330 keys, 14 against 21 at
+    // 60; 173 sequences are one wave at two: 36 against 47).  A cache of one block of keys has nothing to share out (96 heads, 16
+    // keys: 2.8 us with one warp, 3.8 with eight).  Four warps that load values behind the softmax, against one that loads ahead,
+    // 64 sequences, 100 / 330 / 1000 keys: 11.8 / 20.5 / 42.3 us against 9.8 / 20.0 / 48.5.  Nothing finds room: two warps (512
+    // sequences 67 / 176 us at 330 / 1000 keys against 96 / 275 with one, but 35 against 27 at 60), at head size 32 one that loads
+    // ahead (54 / 141 against 67 / 174 us with two), one for short caches.
+    if (cache_len > 64) {
+      B200_DECODE_IF_ROOM(8, true);
+      B200_DECODE_IF_ROOM(4, true);
+      B200_DECODE_IF_ROOM(2, true);
+      if (cache_len > 256) B200_DECODE_IF_ROOM(4, false);
     }
-    if (BH > 18 * sms && BH <= 24 * sms) B200_DECODE(1, false);
+    B200_DECODE_IF_ROOM(1, true);
+    if (cache_len > 64) B200_DECODE_IF_ROOM(2, false);
+    B200_DECODE_IF_ROOM(1, false);
+    if (cache_len <= 128) B200_DECODE(1, false);
+    if (D == 32) B200_DECODE(1, true);
     B200_DECODE(2, false);
   } else {
     // rows too wide to be held: one warp per (batch, head) fills the GPU from about 16 warps per SM on; below that, four share one
-    if (BH >= sms * 16) B200_DECODE(1, false);
+    if (BH >= (int64_t)sm_count() * 16) B200_DECODE(1, false);
     B200_DECODE(4, false);
   }
+#undef B200_DECODE_IF_ROOM
 #undef B200_DECODE
 }
 
