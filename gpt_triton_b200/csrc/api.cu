@@ -36,7 +36,7 @@ const char* b200_status_string(int status) {
 
 const char* b200_last_cuda_error(void) { return cudaGetErrorString(g_last_cuda); }
 
-int b200_abi_version(void) { return 8; }
+int b200_abi_version(void) { return 9; }
 
 uint64_t b200_launch_count(void) { return b200::launches_so_far(); }
 

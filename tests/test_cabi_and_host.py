@@ -32,9 +32,17 @@ def test_library_builds_and_exports_every_declared_symbol():
         assert hasattr(lib, name), f"{name} is declared in include/b200_gpt.h but not exported"
     assert sorted(_lib.SIGNATURES) == names, "ctypes signature table and header disagree"
     bound = _lib.load()
-    assert bound.b200_abi_version() == 8
+    assert bound.b200_abi_version() == 9
     assert bound.b200_status_string(0) == b"ok"
     assert bound.b200_status_string(6) == b"a kernel abandoned a bounded wait"
+
+
+def test_abi_version_counts_entry_points():
+    """A new entry point bumps the version: 46 of them make version 9; header and library name the same one."""
+    from gpt_triton_b200 import _lib
+
+    assert (_lib.load().b200_abi_version(), len(declared_functions())) == (9, 46)
+    assert "ABI version of this header (9)" in open(HEADER).read()
 
 
 def test_argument_checks_need_no_gpu():
