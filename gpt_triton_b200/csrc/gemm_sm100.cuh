@@ -1935,8 +1935,7 @@ inline int few_rows_cols(int64_t M, int64_t N, int ln) {
 // rows and 16 or 32 columns fit the GPU at once, two CTAs per SM.  Beyond that its smaller tiles read A and B more often than they
 // help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of gemm_narrow_kernel.  Clusters of four do not get the last few places:
 // LN == 4 at 32 rows, K = 2048: 280 CTAs (N = 4480) 10.2 us against 10.8, 288 CTAs 15.2 against 10.7; N = 8192 18.0 against 12.0.
-// LN == 4 has 16-column tiles whatever N is, so from 17 rows on it is held to that too (up to 16 rows: N = 8192 17.6 against 17.6, N =
-// 10880 24.3 against 26.3).
+// LN == 4 has 16-column tiles whatever N is, so from 17 rows on it is held to that too (up to 16 rows linear_few_kernel takes K >= 512).
 inline bool takes_few_rows(int64_t M, int64_t N, int ln) {
   if (M <= (ln == 4 ? 16 : kFewMaxRows)) return true;
   if (ln == 5) return false;

@@ -3,11 +3,20 @@
 #include "gemm_sm100.cuh"
 
 namespace b200 {
+
+// linear_few.cu: at most 16 rows, cut along K
+bool linear_few_takes(const b200_linear_args& p, int ln);
+template <typename OutT, int LN>
+int launch_linear_few(const b200_linear_args& p, const gemm::EpilogueArgs<OutT>& epi, cudaStream_t stream);
+
 namespace {
 
 template <typename OutT, int LN>
 int launch(const b200_linear_args& p, const gemm::EpilogueArgs<OutT>& epi, cudaStream_t stream) {
   const gemm::LnArgs none;
+  if constexpr (!std::is_same<OutT, __half>::value) {
+    if (linear_few_takes(p, LN)) return launch_linear_few<OutT, LN>(p, epi, stream);
+  }
   if (p.M <= gemm::kNarrowMaxRows)
     return gemm::launch_narrow<OutT, false, LN>(p.a, p.b, epi, p.M, p.N, p.K, p.lda, p.ldb, p.op_dtype, none, p.status_word, stream);
   return gemm::launch_wide<OutT, false, 0, LN>(p.a, p.b, epi, p.M, p.N, p.K, p.lda, p.ldb, p.op_dtype, none, p.status_word, stream);
