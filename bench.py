@@ -414,6 +414,7 @@ def run_gpu_arm(args, rank, world, local_rank):
             return z
         return fn
 
+    model.whole_passes = False  # operator by operator: what is timed here
     K.fused_ffn = timed_ffn
     K.flash_attention_v1 = timed("attention", "flash_attention_v1")
     K.fused_layer_norm = timed("layernorm", "fused_layer_norm")
@@ -426,6 +427,7 @@ def run_gpu_arm(args, rank, world, local_rank):
     finally:
         for name, fn in orig.items():
             setattr(K, name, fn)
+        model.whole_passes = True
     check_device_status("per-operator probe passes")
     # Per shape, the MEDIAN launch duration (a host stall on a shared box can leave the GPU idle inside one bracket)
     by_shape = {}

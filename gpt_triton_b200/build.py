@@ -17,6 +17,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "_obj")
 LIB_PATH = os.path.join(PKG_DIR, "libb200gpt.so")
+PASSES_PATH = os.path.join(PKG_DIR, "libb200passes.so")  # host code on top of it (csrc/passes.cpp)
 SOURCES = ["api.cu", "elementwise.cu", "gemm_sm100.cu", "linear_sm100.cu", "linear_few.cu", "linear_f32.cu", "attention.cu", "attention_sm100.cu", "latent.cu",
            "latent_decode.cu", "lightning.cu", "stream.cu", "rotary.cu", "pair_attention.cu", "pair_attention_sm100.cu", "pair_decode.cu", "delta.cu", "delta_chunk.cu", "decode.cu", "ffn_static_scratch.cu", "selftest.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "sm100_primitives.cuh"), os.path.join(CSRC, "gemm_sm100.cuh"),
@@ -40,14 +41,18 @@ def _newer(path, deps):
     return os.path.exists(path) and all(os.path.getmtime(d) <= os.path.getmtime(path) for d in deps)
 
 
+PASSES_SOURCES = [os.path.join(CSRC, "passes.cpp"), os.path.join(os.path.dirname(PKG_DIR), "include", "b200_passes.h"),
+                  os.path.join(os.path.dirname(PKG_DIR), "include", "b200_gpt.h")]
+
+
 def is_stale():
-    return not _newer(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
+    return not (_newer(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS) and _newer(PASSES_PATH, PASSES_SOURCES))
 
 
 def _run(cmd):
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + res.stdout + res.stderr)
     return res.stderr
 
 
@@ -73,6 +78,10 @@ def build(force=False, verbose=False):
         part = os.path.join(tmp, "lib.so")
         _run([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", part, *objects])
         os.replace(part, LIB_PATH)
+        part = os.path.join(tmp, "passes.so")
+        _run([shutil.which("g++") or "g++", "-shared", "-fPIC", "-O2", "-std=c++17", PASSES_SOURCES[0], "-o", part, "-L" + PKG_DIR, "-l:" + os.path.basename(LIB_PATH),
+              "-Wl,-rpath,$ORIGIN"])
+        os.replace(part, PASSES_PATH)
     if verbose:
         print("".join(log))
     return LIB_PATH

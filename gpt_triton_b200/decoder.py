@@ -15,6 +15,7 @@ from .module_base import _EvalOnly
 
 class StreamDecoder(GeneratesTokens, _EvalOnly):
     exact_float32 = True  # float32 models run in true 32-bit
+    whole_passes = True  # issue a pass's launches from one host call (passes.py); False: operator by operator.  The same launches.
     TENSOR_NAMES = ()  # (name in the checkpoint, name of the parameter) where a dot of the one is not a submodule of the other
 
     # ---- weights

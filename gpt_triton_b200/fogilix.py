@@ -12,6 +12,7 @@ import torch
 from torch import nn
 
 from . import kernels as K
+from . import passes
 from .decoder import StreamDecoder
 from .mixers import DenseFeedForward, LatentAttention, LightningAttention, _weight
 from .module_base import _OperandCache
@@ -129,9 +130,39 @@ class Fogilix(StreamDecoder):
         dev, dtype = self.embed.device, self.embed.dtype
         return [layer.mix.new_cache(batch, capacity, dev, dtype) for layer in self.layers]
 
+    def _table(self):
+        first, subs = self._sublayers()
+        entries, tensors, layers = (passes.Sublayer * len(subs))(), [self._gain(first)], []
+        for i, layer in enumerate(self.layers):
+            layers += [i] if layer.mlp is None else [i, None]
+        at = {layer: place for place, layer in enumerate(layers) if layer is not None}
+        for e, (sub, norm) in zip(entries, subs):
+            named = sub.describe(e, at)
+            if named is None:
+                return None
+            e.gain = self._gain(norm).data_ptr()
+            tensors += [*named, self._gain(norm)]
+        return passes.Table(entries, tensors, both_norms=False, eps=self.config.eps, first_gain=self._gain(first).data_ptr(), layers=layers, subs=[s for s, _ in subs])
+
+    def _whole_pass(self, ids, ctx, step):
+        """The pass as one host call, None where that does not cover it."""
+        table = passes.table_of(self, ("pass",), self._table) if len(self.layers) and passes.call_ok(self, ids, ctx, step) else None
+        if table is None:
+            return None
+        memories = None
+        if ctx.cache is not None:
+            memories = [None if i is None else s.memory(ctx.cache[i], ctx.batch) for s, i in zip(table.extra["subs"], table.extra["layers"])]
+            if any(m is False for m in memories):
+                return None
+        return K.NormedRows(*passes.decoder_rows(self, ids, ctx, step, table, memories), self.config.width, self.config.eps)
+
     def _run(self, ids, ctx, phase, tap=None):
         """ids (rows,) -> NormedRows behind the final norm.  `tap` (for tests) is called with the stream after every layer."""
         self._check_eval()
+        if self.whole_passes and tap is None:
+            rows = self._whole_pass(ids, ctx, phase == "step")
+            if rows is not None:
+                return rows
         eps = self.config.eps
         first, subs = self._sublayers()
         x, rows = K.embedding_rms(ids, self.embed.data, self._gain(first), eps)

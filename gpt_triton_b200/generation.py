@@ -17,7 +17,7 @@ import gc
 import torch
 
 from . import kernels as K
-from .module_base import _OperandCache
+from .module_base import parameter_tags
 
 
 class GenerationSession:
@@ -47,7 +47,7 @@ class GenerationSession:
         return self.cache
 
     def _signature(self):
-        return tuple(_OperandCache._tag(p) for p in self.model.parameters())
+        return parameter_tags(self.model)
 
     def stale(self):
         """True once a parameter has been reloaded, cast or moved: a captured step holds the old operands."""

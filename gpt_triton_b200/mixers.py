@@ -17,6 +17,7 @@ import torch
 from torch import nn
 
 from . import kernels as K
+from . import passes
 from .module_base import _EvalOnly, _OperandCache
 
 
@@ -61,6 +62,17 @@ class _Sublayer(_EvalOnly):
         p = getattr(self, name)
         return self._operand.derived(("f32", name), (p,), lambda: p.data.float().contiguous())
 
+    def _describe(self, e, kind, w_in, starts, w_out, **vectors):
+        """Fills what every passes.Sublayer `e` has; `vectors`: its tensors by field.  Returns the tensors it names."""
+        e.kind = kind
+        passes.operand(e, "in", w_in)
+        passes.sections(e, starts)
+        passes.operand(e, "out", w_out)
+        e.k_out = w_out.shape[1]
+        for name, t in vectors.items():
+            setattr(e, name, t.data_ptr())
+        return [w_in, w_out, *vectors.values()]
+
 
 class LatentAttention(_Sublayer):
     """Sliding-window softmax attention whose keys and values are linear in one latent vector per token, without
@@ -86,6 +98,25 @@ class LatentAttention(_Sublayer):
         if self.shares is not None:
             return None
         return torch.empty((batch, min(self.reach, capacity), self.kv_rank), device=device, dtype=dtype)
+
+    def describe(self, e, at):
+        """passes.Sublayer of this layer, `at`: layer -> place among the sublayers; the tensors it names, None: not covered."""
+        if self.kv_rank % 8 or not (self.uk.is_contiguous() and self.uv.is_contiguous()):
+            return None
+        w, starts = self._stacked("q") if self.shares is not None else self._stacked("q", "dkv")
+        extra = {} if self.shares is not None else {"norm": self._f32("dkv_norm")}
+        tensors = self._describe(e, passes.LATENT, w, starts, self._stacked("o")[0], sink=self._f32("sink"), w_uk=self.uk.data, w_uv=self.uv.data, **extra)
+        mid, starts = self._stacked("uk", "uv")
+        passes.operand(e, "mid", mid)
+        e.off_mid, e.source = starts[1], at[self.source]
+        e.heads, e.dim, e.vdim, e.rank, e.window, e.reach, e.scale, e.eps = self.heads, self.dim, self.vdim, self.kv_rank, self.window, self.reach, self.scale, self.eps
+        return tensors + [mid]
+
+    def memory(self, cache, batch):
+        """This layer's memory as the passes take it (None: it has none), False: not covered."""
+        if self.shares is not None:
+            return None
+        return (cache,) if passes.tensor_ok(cache, (batch, None, self.kv_rank), self.uk.dtype, self.uk.device) else False
 
     def _project(self, rows):
         """-> (queries, latents before their norm or None)"""
@@ -134,6 +165,14 @@ class LightningAttention(_Sublayer):
     def new_cache(self, batch, capacity, device, dtype):
         return torch.empty((batch, self.heads, self.dim, self.vdim), device=device, dtype=torch.float32)
 
+    def describe(self, e, at):
+        w, starts = self._stacked("q", "k", "v", "g")
+        e.heads, e.dim, e.vdim, e.eps = self.heads, self.dim, self.vdim, self.eps
+        return self._describe(e, passes.LIGHTNING, w, starts, self._stacked("o")[0], decay=self._decay_on(self.q.device), norm=self._f32("norm"))
+
+    def memory(self, cache, batch):
+        return (cache,) if passes.tensor_ok(cache, (batch, self.heads, self.dim, self.vdim), torch.float32, self.q.device) else False
+
     def _decay_on(self, device):
         return self._operand.derived(("decay",), (self.q,), lambda: torch.tensor(self.decay, dtype=torch.float64, device=device))
 
@@ -157,8 +196,15 @@ class DenseFeedForward(_Sublayer):
 
     def __init__(self, width, ff, act="gelu_tanh"):
         super().__init__()
-        self.act = act
+        self.act, self.ff = act, ff
         self.up, self.down = _weight(ff, width), _weight(width, ff)
+
+    def describe(self, e, at):
+        e.act, e.ff = K.ACTIVATIONS[self.act], self.ff
+        return self._describe(e, passes.DENSE, self._stacked("up")[0], (), self._stacked("down")[0])
+
+    def memory(self, cache, batch):
+        return None
 
     def prompt(self, x, rows, ctx, next_gain, next_eps):
         y = K.linear(rows, self._stacked("up")[0], act=self.act)
@@ -187,6 +233,20 @@ class DifferentialAttention(_Sublayer):
         """Keys and values of the tokens that the window can see."""
         ring = min(self.window, capacity)
         return tuple(torch.empty((batch, self.kv_heads, ring, cols), device=device, dtype=dtype) for cols in (2 * self.dim, self.vdim))
+
+    def describe(self, e, at):
+        w, starts = self._stacked("q", "k", "v", "g")
+        freq = self._frequencies()
+        e.heads, e.kv_heads, e.dim, e.vdim, e.window, e.rot_dims = self.heads, self.kv_heads, self.dim, self.vdim, self.window, 2 * freq.shape[0]
+        e.scale, e.softcap, e.eps, e.out_scale = self.scale, self.softcap, self.eps, 1.0 - self.diff
+        e.v_dtype = K.dtype_code(K.pair_attention_v_dtype(self.dim, self.vdim, self.q.dtype))
+        return self._describe(e, passes.DIFFERENTIAL, w, starts, self._stacked("o")[0], norm=self._f32("q_norm"), norm2=self._f32("k_norm"), freq=freq,
+                              lambda_=self._lambda())
+
+    def memory(self, cache, batch):
+        ok = (isinstance(cache, tuple) and len(cache) == 2 and passes.tensor_ok(cache[0], (batch, self.kv_heads, None, 2 * self.dim), self.q.dtype, self.q.device)
+              and passes.tensor_ok(cache[1], (batch, self.kv_heads, cache[0].shape[2], self.vdim), self.q.dtype, self.q.device))
+        return cache if ok else False
 
     def _lambda(self):
         def make():
@@ -245,6 +305,18 @@ class GatedDeltaRule(_Sublayer):
         return (torch.empty((batch, self.heads, self.dim, self.vdim), device=device, dtype=torch.float32),
                 torch.empty((batch, self.taps, self._conv_cols()), device=device, dtype=dtype))
 
+    def describe(self, e, at):
+        w, starts = self._stacked("q", "k", "v", "a", "b", "g")
+        e.heads, e.kv_heads, e.dim, e.vdim, e.taps, e.conv_cols = self.heads, self.kv_heads, self.dim, self.vdim, self.taps, self._conv_cols()
+        e.eps, e.q_scale, e.unit_eps = self.eps, self.dim ** -0.5, K.UNIT_EPS
+        return self._describe(e, passes.DELTA, w, starts, self._stacked("o")[0], conv_w=self._taps(starts), a_log=self._f32("A_log"), dt_bias=self._f32("dt_bias"),
+                              norm=self._f32("norm"))
+
+    def memory(self, cache, batch):
+        ok = (isinstance(cache, tuple) and len(cache) == 2 and passes.tensor_ok(cache[0], (batch, self.heads, self.dim, self.vdim), torch.float32, self.q.device)
+              and passes.tensor_ok(cache[1], (batch, self.taps, self._conv_cols()), self.q.dtype, self.q.device))
+        return cache if ok else False
+
     def _taps(self, starts):
         """(columns, taps) float32 in the column order of the stacked product."""
         def make():
@@ -282,9 +354,21 @@ class GatedFeedForward(_Sublayer):
         self.gate, self.up, self.down = _weight(ff, width), _weight(ff, width), _weight(width, ff)
         self.gate_b, self.up_b, self.down_b = _weight(ff), _weight(ff), _weight(width)
 
-    def prompt(self, rows, ctx):
+    def _pairs(self):
         w = self._operand.derived(("pairs",), (self.gate, self.up), lambda: K.operand_rows(K.interleave_gated(self.gate.data, self.up.data))[0])
         b = self._operand.derived(("pair biases",), (self.gate_b, self.up_b), lambda: K.interleave_gated(self.gate_b.data, self.up_b.data).float())
+        return w, b
+
+    def describe(self, e, at):
+        w, b = self._pairs()
+        e.ff, e.limit, e.alpha = self.ff, self.limit, self.alpha
+        return self._describe(e, passes.GATED, w, (), self._stacked("down")[0], bias_in=b, bias_out=self._f32("down_b"))
+
+    def memory(self, cache, batch):
+        return None
+
+    def prompt(self, rows, ctx):
+        w, b = self._pairs()
         y = K.gated_linear(rows, w, b, self.ff, limit=self.limit, alpha=self.alpha)
         return K.linear(y, self._stacked("down")[0], bias=self._f32("down_b"))
 

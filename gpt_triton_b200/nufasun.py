@@ -14,6 +14,7 @@ import torch
 from torch import nn
 
 from . import kernels as K
+from . import passes
 from .decoder import StreamDecoder
 from .mixers import DifferentialAttention, GatedDeltaRule, GatedFeedForward, _weight
 from .module_base import _OperandCache
@@ -156,9 +157,45 @@ class Nufasun(StreamDecoder):
     def _f32(self, param):
         return self._operand.derived(("f32", id(param)), (param,), lambda: param.data.float().contiguous())
 
+    def _table(self):
+        c, steps = self.config, self._f32(self.loop_step)
+        subs, runs, tensors = [], [], [steps, self._f32(self.final_norm)]
+        described = []
+        for run, (layer, entered) in enumerate(c.runs()):
+            for first, (sub, gain, behind) in zip((True, False), self.layers[layer].sublayers()):
+                e = passes.Sublayer()
+                named = sub.describe(e, {})
+                if named is None:
+                    return None
+                e.gain, e.behind = self._f32(gain).data_ptr(), self._f32(behind).data_ptr()
+                if first and entered is not None:
+                    e.shift, e.add_embedding = steps[entered].data_ptr(), int(entered > 0)
+                tensors += [*named, self._f32(gain), self._f32(behind)]
+                described.append(e)
+                subs.append(sub)
+                runs.append(run if first else None)
+        return passes.Table((passes.Sublayer * len(described))(*described), tensors, both_norms=True, eps=c.eps, table_scale=c.embedding_scale,
+                            final_gain=self._f32(self.final_norm).data_ptr(), subs=subs, runs=runs)
+
+    def _whole_pass(self, ids, ctx, step):
+        """The pass as one host call, None where that does not cover it."""
+        table = passes.table_of(self, ("pass",), self._table) if passes.call_ok(self, ids, ctx, step) else None
+        if table is None:
+            return None
+        memories = None
+        if ctx.cache is not None:
+            memories = [None if run is None else s.memory(ctx.cache[run], ctx.batch) for s, run in zip(table.extra["subs"], table.extra["runs"])]
+            if any(m is False for m in memories):
+                return None
+        return passes.decoder_rows(self, ids, ctx, step, table, memories)[0]
+
     def _run(self, ids, ctx, phase, tap=None):
         """ids (rows,) -> rows behind the final norm.  `tap` (for tests) is called with the stream after every layer run."""
         self._check_eval()
+        if self.whole_passes and tap is None:
+            rows = self._whole_pass(ids, ctx, phase == "step")
+            if rows is not None:
+                return rows
         c = self.config
         steps = self._f32(self.loop_step)
         embedded = dict(ids=ids, table=self.embed.data, table_scale=c.embedding_scale)

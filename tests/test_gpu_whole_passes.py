@@ -1,0 +1,141 @@
+"""A pass issued as one host call (passes.py) against the operators one by one: the same bits, the same launches."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _launches(fn):
+    from gpt_triton_b200 import _lib
+
+    n0 = _lib.load().b200_launch_count()
+    out = fn()
+    return out, _lib.load().b200_launch_count() - n0
+
+
+def _both(model, fn):
+    """fn() as whole passes and operator by operator; results must be equal, launches too."""
+    a, na = _launches(fn)
+    model.whole_passes = False
+    b, nb = _launches(fn)
+    model.whole_passes = True
+    a, b = (x if isinstance(x, (list, tuple)) else [x] for x in (a, b))
+    assert len(a) == len(b) and all(torch.equal(x, y) for x, y in zip(a, b)) and na == nb > 0
+
+
+def _gpt(dtype, hidden=128, heads=4, layers=3):
+    from gpt_triton_b200.gpt import FusedGPT, GPTConfig
+
+    torch.manual_seed(hidden + layers)
+    model = FusedGPT(GPTConfig(vocab_size=300, block_size=96, n_layer=layers, n_head=heads, n_embd=hidden)).to(DEV)
+    for p in model.parameters():
+        p.data.copy_(torch.randn_like(p) * 0.05 + (1.0 if p.dim() == 1 and p.shape[0] == hidden else 0.0))
+    return model.to(dtype).eval()
+
+
+@pytest.mark.parametrize("dtype,fold", [(torch.float16, True), (torch.bfloat16, True), (torch.bfloat16, False), (torch.float32, False)])
+@pytest.mark.parametrize("B,L", [(1, 1), (3, 43), (2, 64), (4, 96)])  # on both sides of 128 rows
+def test_gpt(dtype, fold, B, L):
+    from gpt_triton_b200 import kernels as K
+    from gpt_triton_b200 import passes
+    from gpt_triton_b200.generation import GenerationSession
+    from gpt_triton_b200.gpt import FusedAttention, FusedMLP
+
+    model = _gpt(dtype)
+    model.fold_layer_norm = fold
+    ids = torch.randint(0, 300, (B, L), device=DEV)
+    model.logits(ids)
+    assert passes.gpt_body(model, ids, None, None, FusedAttention, FusedMLP) is not None  # (covered)
+    _both(model, lambda: model(ids))
+
+    def request():
+        s = GenerationSession(model, B, capacity=96, use_cuda_graph=False)
+        rows = [s.extend(ids[:, :L - 1].contiguous())] if L > 1 else []
+        return rows + [s.extend(ids[:, L - 1:].contiguous()), *[c[:, :L].contiguous() for c in s.cache]]
+
+    _both(model, request)
+    assert K.device_status() == 0
+
+
+def test_gpt_notices_changes():
+    model = _gpt(torch.float16)
+    ids = torch.randint(0, 300, (2, 40), device=DEV)
+    first = model(ids)
+    with torch.no_grad():
+        model.blocks[1][1].ffn1_weight.mul_(1.5)
+    model(ids)
+    _both(model, lambda: model(ids))
+    assert not torch.equal(model(ids), first)
+    model.blocks[0][0].c_proj_weight.data.mul_(0.5)  # (no counter notices)
+    model.blocks[0][0].refresh_operands()
+    model(ids)
+    _both(model, lambda: model(ids))
+    model.blocks[2] = torch.nn.Sequential(*reversed(list(model.blocks[2].children())))  # a shape that is not covered
+    with pytest.raises(Exception):
+        model(ids)
+
+
+def _decoder(kind, width=64, passes=2):
+    from gpt_triton_b200.fogilix import Fogilix
+    from gpt_triton_b200.nufasun import Nufasun
+
+    mlp = {"kind": "dense", "ff": 96}
+    if kind == "fogilix":
+        latent = {"heads": 4, "dim": 16, "vdim": 24, "kv_rank": 32, "mask": {"size": 20}, "scale": 0.25}
+        lightning = {"heads": 4, "dim": 16, "vdim": 16, "decay": [0.9, 0.95, 0.99, 1.0]}
+        layers = [{"type": "lightning", "mixer": lightning, "mlp": mlp}, {"type": "latent_attention", "mixer": latent}, {"type": "lightning", "mixer": lightning},
+                  {"type": "latent_attention", "mixer": {**latent, "kv_from": 1, "heads": 2, "mask": {"size": 33}}, "mlp": mlp}]
+        cfg, cls = {"vocab": 211, "width": width, "layers": layers, "norm": {"eps": 1e-5}, "logit_scale": 1.0}, Fogilix
+        model = cls(__import__("gpt_triton_b200.fogilix", fromlist=["x"]).FogilixConfig.from_dict(cfg))
+    else:
+        mlp = {"kind": "dense", "ff": 104, "limit": 2.0}
+        delta = {"heads": 4, "kv_heads": 2, "dim": 16, "vdim": 16, "conv": 4}
+        pair = {"heads": 4, "kv_heads": 2, "dim": 16, "vdim": 24, "mask": {"size": 21}, "diff": 0.4, "softcap": 20.0, "scale": 0.25, "rot": {"base": 1e4, "dims": 8}}
+        layers = [{"type": "delta", "mixer": delta, "mlp": mlp}, {"type": "attention", "mixer": pair, "mlp": mlp}, {"type": "delta", "mixer": delta},
+                  {"type": "attention", "mixer": pair}]
+        cfg = {"vocab": 211, "width": width, "layers": layers, "norm": {"eps": 1e-5}, "embedding": {"scale": 2.0}, "logit_softcap": 15.0,
+               "loop": {"start": 1, "stop": 3, "times": passes}}
+        model = Nufasun(__import__("gpt_triton_b200.nufasun", fromlist=["x"]).NufasunConfig.from_dict(cfg))
+    torch.manual_seed(1)
+    for p in model.parameters():
+        p.data.copy_(torch.randn_like(p) * (0.3 if p.dim() < 2 else p.shape[-1] ** -0.5))
+    return model.to(DEV).to(torch.bfloat16).eval()
+
+
+@pytest.mark.parametrize("kind", ["fogilix", "nufasun"])
+@pytest.mark.parametrize("B,n", [(1, 5), (2, 70), (3, 300)])
+def test_decoders(kind, B, n):
+    from gpt_triton_b200 import kernels as K
+    from gpt_triton_b200.generation import GenerationSession
+    from gpt_triton_b200.mixers import PromptContext
+
+    model = _decoder(kind)
+    ids = torch.randint(0, 211, (B, n + 3), device=DEV)
+    model.logits(ids)
+    assert model._whole_pass(ids.reshape(-1), PromptContext(B, n + 3, 0, None), False) is not None  # (covered)
+    _both(model, lambda: model.logits(ids))
+
+    def request():
+        s = GenerationSession(model, B, capacity=n + 3, use_cuda_graph=False)
+        out = [s.extend(ids[:, :n // 2].contiguous()), s.extend(ids[:, n // 2:n].contiguous()), s.extend(ids[:, n:n + 1].contiguous()), s.extend(ids[:, n + 1:n + 2].contiguous())]
+        out = [t for r in out for t in ((r.data, r.sumsq) if isinstance(r, K.NormedRows) else (r,))]
+        return out + [model.head_logits(s.extend(ids[:, n + 2:].contiguous()))]
+
+    _both(model, request)
+    assert K.device_status() == 0
+
+
+def test_a_decoder_notices_changes():
+    model = _decoder("fogilix")
+    ids = torch.randint(0, 211, (2, 50), device=DEV)
+    first = model.logits(ids)
+    model.layers[1].mix.window = 5
+    model.logits(ids)
+    _both(model, lambda: model.logits(ids))
+    with torch.no_grad():
+        model.layers[0].mix.q.mul_(2.0)
+    model.logits(ids)
+    _both(model, lambda: model.logits(ids))
+    assert not torch.equal(model.logits(ids), first)
