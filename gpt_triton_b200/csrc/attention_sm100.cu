@@ -1,5 +1,5 @@
 // Causal flash attention on the 5th-generation tensor cores, fp16 or bf16 storage: head sizes 64 and 128 (template parameter WIN
-// off), or sliding-window attention with a sink, an earlier part of the sequence in front of the queries and separate
+// off; attention_causal_sm100.cu has the kernel for many tiles of up to 64 columns), or sliding-window attention with a sink, an earlier part of the sequence in front of the queries and separate
 // key/value sizes of up to 64 or up to 128 (WIN on; smaller sizes are zero-filled by the loads).
 // bf16 Q and K feed S = Q K^T as they are (exact products).  P is fp16 for both storage types, as in the
 // reference, and both operands of one MMA must have the same format, so a bf16 V tile is converted to
@@ -504,14 +504,30 @@ static int launch_causal(const void* q, const void* k, const void* v, void* out,
   return status_from_cuda(e);
 }
 
+// attention_causal_sm100.cu: head sizes up to 64
+int launch_causal_attention_sm100(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t NH, int64_t L, int64_t D,
+                                  const int64_t* qs, const int64_t* ks, const int64_t* vs, const int64_t* os, float scale, int dtype, int* status_word,
+                                  cudaStream_t stream);
+
 // Returns B200_ERR_UNSUPPORTED when the problem does not fit these kernels (the caller then takes the generic one).
 int launch_attention_sm100(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t NH, int64_t L, int64_t D,
                            const int64_t* qs, const int64_t* ks, const int64_t* vs, const int64_t* os, float scale, int in_dtype,
                            int out_dtype, int* status_word, cudaStream_t stream) {
   if (in_dtype != out_dtype || (in_dtype != B200_F16 && in_dtype != B200_BF16) || !(scale > 0.f)) return B200_ERR_UNSUPPORTED;
   if (D == 128) return launch_causal<128>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
-  if (D != 64) return B200_ERR_UNSUPPORTED;
-  return launch_causal<64>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
+  if (D > 64) return B200_ERR_UNSUPPORTED;
+  // Up to 64 columns: four tiles an SM (attention_causal_sm100.cu) give the higher rate, two of this kernel's a tile's result sooner.
+  // The same bits, so the choice may follow the batch.  us, fp16, 12 heads of 64, here | there: 8 x 300 (288 tiles) 9.4 | 9.8, 9 x 300
+  // (324) 11.1 | 10.1, 64 x 300 42 | 32; 2 x 2048 (384) 42.6 | 44.1, 3 x 2048 (576) 51.6 | 47.2, 16 x 2048 219 | 181; one tile per
+  // sequence 4.8 | 4.3.
+  // Smaller heads are zero-filled to 64, which the generic kernel does not need: up to 128 rows it stays (2 x 4 x 64 x 16 2.7 | 4.0,
+  // 16 x 25 x 64 x 32 5.0 | 5.6; 64 x 25 x 64 x 32 12.6 | 9.7, but the two differ in the order of their sums, and what a row gives is
+  // not to depend on the batch).  Beyond: 4 x 12 x 300 x 32 11.6 | 8.8, 16 x 12 x 1024 x 32 123 | 49.
+  if (D < 64 && L <= 128) return B200_ERR_UNSUPPORTED;
+  const int64_t n_items = (L + attn100::BLOCK_M - 1) / attn100::BLOCK_M * B * NH;
+  if (D == 64 && L > 128 && n_items <= (L <= 1024 ? 2 : 3) * (int64_t)sm_count())
+    return launch_causal<64>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
+  return launch_causal_attention_sm100(q, k, v, out, B, NH, L, D, qs, ks, vs, os, scale, in_dtype, status_word, stream);
 }
 
 namespace attn100 {
