@@ -234,11 +234,10 @@ int launch_gemm_ln(const void* a, const void* b, const void* bias, const void* r
   else B200_GEMM_LN_DISPATCH(__nv_bfloat16);
 #undef B200_GEMM_LN_DISPATCH
   if (st != B200_OK || !stats_out) return st;
-  // width of the column slices whose moments the GEMM left: the wide kernel's epilogue warps cover EPI_COLS columns, the others
-  // leave NARROW_BN
-  const bool narrow = io_dtype == B200_F16 ? takes_narrow_tiles<__half, 0>(M, out, ld_out, residual, ld_res)
-                                           : takes_narrow_tiles<__nv_bfloat16, 0>(M, out, ld_out, residual, ld_res);
-  const int slice_cols = narrow ? NARROW_BN : EPI_COLS;
+  // width of the column slices whose moments the GEMM left: 64 up to kNarrowMaxRows rows, 128 beyond and from the wide kernel
+  const bool small = io_dtype == B200_F16 ? takes_narrow_tiles<__half, 0>(M, N, 2, out, ld_out, residual, ld_res)
+                                          : takes_narrow_tiles<__nv_bfloat16, 0>(M, N, 2, out, ld_out, residual, ld_res);
+  const int slice_cols = small && M <= kNarrowMaxRows ? NARROW_BN : EPI_COLS;
   const int slices = (int)((N + slice_cols - 1) / slice_cols);
   const cudaError_t e = io_dtype == B200_F16
                             ? launch_ln_stats<__half>(ln.stats_out, ln.stats_out_ld, slices, slice_cols, N, eps, M, stats_out, ext_out, stream)

@@ -1327,50 +1327,58 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
 
 // ------------------------------------------------------------------ narrow-tile variant for few rows
-// With M <= kNarrowMaxRows (one generated token per sequence; tiny configurations) the 256 x 256 tiles of the kernel
-// above leave most of the GPU idle: a 512 x 768 x 3072 product is 6 tiles, each a serial loop of 48 k-blocks.  This
-// kernel computes ONE 128 x 64 tile per CTA (grid = column tiles x row tiles, no persistence, one accumulator), so
+// With a few hundred or a few thousand rows the 256 x 256 tiles of the kernel above leave most of the GPU idle: a 512 x 768 x 3072
+// product is 6 tiles, each a serial loop of 48 k-blocks.  This kernel computes ONE 128 x 64 tile per CTA (grid = column tiles x row tiles, no persistence, one accumulator), so
 // the same product becomes 48 CTAs: the same TMA ring, tcgen05.mma (M = 128, N = 64, cta_group::1) and fused
 // epilogue arithmetic (epilogue_chunk, direct 16-byte stores), k-blocks in the same order, hence the same bits.
-// 16-bit output, no row statistics of the argmax kind; LN = 1 / 2 as above, the moments of LN = 2 per 64-column slice.
+// No row statistics of the argmax kind; LN = 1 / 2 as above.  The moments of LN = 2 and the sums of squares of LN = 4 are left per 64
+// columns, or, beyond kNarrowMaxRows, per 128 and to the bit as the wide kernel leaves them, so that a row's results do not depend on
+// how many there are (PAIR_SLICES: the CTAs of 128 columns form a cluster; the second one's epilogue goes on from the sums that the
+// first one sends it).
+// Six stages when every tile finds an SM of its own, four (two CTAs an SM) when there are more tiles than SMs: 288 tiles, 1024 rows,
+// 768 -> 2304: 9.3 us with one CTA an SM, 7.5 with two; 96 tiles, 768 -> 768: 4.7 and 6.1.
 // Warp 0: TMA producer; warp 1: tensor-memory owner and MMA issuer; warps 2-5: epilogue (one row per thread).
 constexpr int NARROW_BN = 64;
-constexpr int NARROW_STAGES = 6;
+constexpr int NARROW_MAX_STAGES = 6;
 constexpr int NARROW_A_BYTES = BM * BK * 2;         // 16 KB
 constexpr int NARROW_B_BYTES = NARROW_BN * BK * 2;  // 8 KB
 constexpr int NARROW_STAGE_BYTES = NARROW_A_BYTES + NARROW_B_BYTES;
 constexpr int NARROW_THREADS = 192;
 constexpr int NARROW_CTRL_BYTES = 256;
-constexpr int NARROW_SMEM_BYTES = NARROW_STAGES * NARROW_STAGE_BYTES + 1024 + NARROW_CTRL_BYTES + NARROW_BN * 4;
-constexpr int kNarrowMaxRows = 512;
+constexpr int NARROW_TAIL_BYTES = NARROW_CTRL_BYTES + NARROW_BN * 4 + 4 * BM * 4;  // control, bias, the other CTA's row sums
+constexpr int narrow_smem_bytes(int stages) { return stages * NARROW_STAGE_BYTES + 1024 + NARROW_TAIL_BYTES; }
+static_assert(2 * (narrow_smem_bytes(4) + 1024) <= 228 * 1024, "two CTAs per SM");
+constexpr int kNarrowMaxRows = 512;  // moments and sums of squares come per 64 columns up to here, per 128 beyond
 
-template <typename OutT, bool GELU, int LN>
-__global__ void __launch_bounds__(NARROW_THREADS, 1)
+template <typename OutT, bool GELU, int LN, bool PAIR_SLICES>
+__global__ void __launch_bounds__(NARROW_THREADS, 2)
 gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ CUtensorMap map_a_ext, const __grid_constant__ CUtensorMap map_b_ext, EpilogueArgs<OutT> epi,
-                   int64_t M, int64_t N, int64_t K, uint32_t idesc, int* status_word) {
-  static_assert(sizeof(OutT) == 2 || LN >= 3, "fp32 outputs exist behind a deferred RMS norm only");
+                   int64_t M, int64_t N, int64_t K, int stages, uint32_t idesc, int* status_word) {
+  static_assert(!PAIR_SLICES || LN == 2 || LN == 4, "what is left per slice");
+  static_assert(sizeof(OutT) == 2 || LN == 0 || LN >= 3, "the folded LayerNorm is 16-bit");
   constexpr int esz = (int)sizeof(OutT);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;  // 128-byte-swizzled tiles need 1024-byte aligned bases
   uint8_t* smem = smem_raw + (base - raw);
   const uint32_t smem_a = base;
-  const uint32_t smem_b = base + NARROW_STAGES * NARROW_A_BYTES;
-  uint8_t* ctrl = smem + NARROW_STAGES * NARROW_STAGE_BYTES;
+  const uint32_t smem_b = base + (uint32_t)(stages * NARROW_A_BYTES);
+  uint8_t* ctrl = smem + stages * NARROW_STAGE_BYTES;
   const uint32_t bars = smem_u32(ctrl);
-  const uint32_t bar_full = bars, bar_empty = bars + 8 * NARROW_STAGES, bar_acc = bars + 16 * NARROW_STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 16 * NARROW_STAGES + 8);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 16 * NARROW_STAGES + 16);
-  static_assert(16 * NARROW_STAGES + 24 <= NARROW_CTRL_BYTES, "control block too small");
+  const uint32_t bar_full = bars, bar_empty = bars + 8 * NARROW_MAX_STAGES, bar_acc = bars + 16 * NARROW_MAX_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ctrl + 16 * NARROW_MAX_STAGES + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(ctrl + 16 * NARROW_MAX_STAGES + 16);
+  static_assert(16 * NARROW_MAX_STAGES + 24 <= NARROW_CTRL_BYTES, "control block too small");
   float* bias_s = reinterpret_cast<float*>(ctrl + NARROW_CTRL_BYTES);
+  float* sums_s = bias_s + NARROW_BN;  // PAIR_SLICES, second CTA: [4][BM], what the first one has summed
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * NARROW_BN, m0 = blockIdx.y * BM;
   const int num_kb_ab = (int)((K + BK - 1) / BK);
   const int num_kb = num_kb_ab + (LN == 1 ? 1 : 0);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NARROW_STAGES; ++i) {
+    for (int i = 0; i < stages; ++i) {
       mbar_init(bar_full + 8 * i, 1);
       mbar_init(bar_empty + 8 * i, 1);
     }
@@ -1385,11 +1393,13 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR_SLICES) cluster_sync_all();  // the second CTA's shared memory exists before the first writes to it
   tc_fence_after();
   const uint32_t tmem_d = *tmem_slot;
   pdl_launch_dependents();
   pdl_wait();
 
+  [[maybe_unused]] const bool second = PAIR_SLICES && (blockIdx.x & 1);
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0;
@@ -1400,7 +1410,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         mbar_arrive_expect_tx(bar_full + 8 * stage, NARROW_STAGE_BYTES);
         tma_load_2d(smem_a + stage * NARROW_A_BYTES, ext ? &map_a_ext : &map_a, bar_full + 8 * stage, ext ? 0 : kb * BK, m0);
         tma_load_2d(smem_b + stage * NARROW_B_BYTES, ext ? &map_b_ext : &map_b, bar_full + 8 * stage, ext ? 0 : kb * BK, n0);
-        if (++stage == NARROW_STAGES) stage = 0, phase ^= 1u;
+        if (++stage == stages) stage = 0, phase ^= 1u;
       }
     }
   } else if (warp == 1) {
@@ -1423,7 +1433,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           umma_f16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (uint32_t)((kb | k) != 0));
         }
         umma_commit(bar_empty + 8 * stage);
-        if (++stage == NARROW_STAGES) stage = 0, phase ^= 1u;
+        if (++stage == stages) stage = 0, phase ^= 1u;
       }
       if (alive) umma_commit(bar_acc);
     }
@@ -1466,10 +1476,16 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (int i = 0; i < NARROW_BN / 8; ++i)
         if (n0 + (i / 4) * 32 + 32 <= N) res[i] = *reinterpret_cast<const uint4*>(rrow + i * 8);
     }
+    SliceMoments mom{0.f, 0.f, 0.f, 0.f};
+    [[maybe_unused]] const int r_in_tile = quarter * 32 + lane;
+    if (second) {
+      __syncwarp();
+      cluster_sync_all();
+      mom = SliceMoments{sums_s[r_in_tile], sums_s[BM + r_in_tile], sums_s[2 * BM + r_in_tile], sums_s[3 * BM + r_in_tile]};
+    }
     if (mbar_wait(bar_acc, 0, abort_flag, status_word, 33)) {
       tc_fence_after();
       RowStats unused{-INFINITY, 0, 0.f, -1};
-      SliceMoments mom{0.f, 0.f, 0.f, 0.f};
       if constexpr (LN == 5) {
         static_assert(NARROW_BN == 64, "one block of gate and up columns per tile");
         uint32_t za[32], zb[32];
@@ -1492,18 +1508,32 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           epilogue_chunk<OutT, GELU, 0, LN>(v, bias_s + c * 32, epi, (res_in_regs && col0 + 32 <= N) ? &res[c * 4] : nullptr, row, col0, N, mode, 0u,
                                             c & 1, lane, row_ok, false, unused, ln_r, mom);
       }
-      if constexpr (LN == 4) {
-        if (row_ok && epi.gain) epi.sq_out[(int64_t)blockIdx.x * epi.sq_out_ld + row] = mom.s2;
-      }
-      if constexpr (LN == 2) {
-        if (row_ok && mom.n > 0.f) {
-          const float inv = 1.0f / mom.n;
-          epi.stats_out[(int64_t)blockIdx.x * epi.stats_out_ld + row] = make_float2(fmaf(mom.s1, inv, mom.shift), fmaxf(mom.s2 - mom.s1 * mom.s1 * inv, 0.f));
+      if (PAIR_SLICES && !second) {
+        const uint32_t to = mapa_shared(smem_u32(sums_s + r_in_tile), 1);
+        const float sums[4] = {mom.shift, mom.s1, mom.s2, mom.n};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to + i * BM * 4), "f"(sums[i]) : "memory");
+      } else {
+        const int64_t slice = PAIR_SLICES ? blockIdx.x >> 1 : blockIdx.x;
+        if constexpr (LN == 4) {
+          if (row_ok && epi.gain) epi.sq_out[slice * epi.sq_out_ld + row] = mom.s2;
+        }
+        if constexpr (LN == 2) {
+          if (row_ok && mom.n > 0.f) {
+            const float inv = 1.0f / mom.n;
+            epi.stats_out[slice * epi.stats_out_ld + row] = make_float2(fmaf(mom.s1, inv, mom.shift), fmaxf(mom.s2 - mom.s1 * mom.s1 * inv, 0.f));
+          }
         }
       }
     }
   }
 
+  if constexpr (PAIR_SLICES) {
+    if (!second || warp < 2) {
+      __syncwarp();
+      cluster_sync_all();
+    }
+  }
   // ------------------------------------------------------------ teardown
   __syncwarp();
   if (*abort_flag) {
@@ -1931,7 +1961,21 @@ inline int few_rows_cols(int64_t M, int64_t N, int ln) {
   if (row_tiles == 1 && (N + 63) / 64 > enough) return 64;
   return (N + 31) / 32 * row_tiles > enough ? 32 : 16;
 }
-// Whether a product of at most kNarrowMaxRows rows goes to gemm_few_kernel: up to 64 rows, and above that as long as its tiles of 64
+// Whether tiles of 128 x 64 are faster than the wide kernel's: as long as they need no more rounds of the GPU, two CTAs an SM.  A
+// round of the wide kernel takes longer, but covers four times as much, and its first one has 6 us of set-up that these tiles do
+// without.  us, narrow | wide, rows: 768 -> 768 600 4.2 | 10.5, 1536 4.8 | 10.8, 3072 (288 tiles) 7.6 | 11.3, 4096 (384) 13 | 11.3; 3072 -> 768
+// with row statistics 1024 13 | 25, 3072 23 | 26; 768 -> 2304 1024 (288) 7.5 | 11.2, 1280 (360) 13 | 11.3; 2048 -> 2048 1024 (256) 13 | 21;
+// 2048 -> 8192 256 (256) 12.8 | 21.1, 512 (512) 24.1 | 21.8; 2048 -> 10880 384 rows (510 against 86: two rounds each) 22.6 | 26.8, 512 (680) 31.6 | 27.0.
+// Beyond kNarrowMaxRows a row's sums pass from one CTA to the next (PAIR_SLICES), which two CTAs an SM do not hide: x += z 1024 -> 1024, 1024 rows
+// (128 tiles) 11.5 | 15.9, 1536 (192) 18.5 | 16.1; row statistics 1024 -> 1024, 2048 rows (256) 14.7 | 16.0, 768 -> 768, 3072 (288) 15.3 | 14.9.
+inline bool narrow_is_faster(int64_t M, int64_t N, int ln) {
+  const int64_t sms = sm_count(), narrow = (M + BM - 1) / BM * ((N + NARROW_BN - 1) / NARROW_BN);
+  if (M > kNarrowMaxRows && ln == 4) return narrow <= sms;
+  if (M > kNarrowMaxRows && ln == 2) return 4 * narrow <= 7 * sms;
+  const int64_t wide = M > BM ? (M + 2 * BM - 1) / (2 * BM) * ((N + BN - 1) / BN) : (N + BN - 1) / BN, places = M > BM ? sms / 2 : sms;
+  return (narrow + 2 * sms - 1) / (2 * sms) <= (wide + places - 1) / places;
+}
+// Whether a product goes to gemm_few_kernel: up to 64 rows, and above that as long as its tiles of 64
 // rows and 16 or 32 columns fit the GPU at once, two CTAs per SM.  Beyond that its smaller tiles read A and B more often than they
 // help: 192 rows, N x K = 8192 x 2048: 20.2 us against 16.2 of gemm_narrow_kernel.  Clusters of four do not get the last few places:
 // LN == 4 at 32 rows, K = 2048: 280 CTAs (N = 4480) 10.2 us against 10.8, 288 CTAs 15.2 against 10.7; N = 8192 18.0 against 12.0.
@@ -2000,42 +2044,60 @@ static int launch_few(const void* a, const void* b, const EpilogueArgs<OutT>& ep
   }
 }
 
+template <typename OutT, bool GELU, int LN, bool PAIR_SLICES>
+static int launch_narrow_tiles(const void* a, const void* b, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                               int op_dtype, const LnArgs& ln, int* status_word, cudaStream_t stream) {
+  auto* kernel = gemm_narrow_kernel<OutT, GELU, LN, PAIR_SLICES>;
+  static std::atomic<bool> attr_set[kMaxDevices];
+  const int slot = device_slot();
+  if (slot < 0) return B200_ERR_CUDA;
+  if (!attr_set[slot].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, narrow_smem_bytes(NARROW_MAX_STAGES)) != cudaSuccess) return B200_ERR_CUDA;
+    attr_set[slot].store(true, std::memory_order_release);
+  }
+  CUtensorMap ma, mb, mae, mbe;
+  memset(&mae, 0, sizeof(mae));
+  memset(&mbe, 0, sizeof(mbe));
+  int st = make_map(&ma, a, M, K, lda, BM, op_dtype);
+  if (st == B200_OK) st = make_map(&mb, b, N, K, ldb, NARROW_BN, op_dtype);
+  if (st == B200_OK && LN == 1) st = make_map(&mae, ln.a_ext, M, kLnExtCols, kLnExtCols, BM, op_dtype);
+  if (st == B200_OK && LN == 1) st = make_map(&mbe, ln.b_ext, N, kLnExtCols, kLnExtCols, NARROW_BN, op_dtype);
+  if (st != B200_OK) return st;
+  unsigned cols = (unsigned)((N + NARROW_BN - 1) / NARROW_BN);
+  const unsigned row_tiles = (unsigned)((M + BM - 1) / BM);
+  const int stages = (int64_t)cols * row_tiles <= sm_count() ? NARROW_MAX_STAGES : 4;
+  if (PAIR_SLICES) cols = (cols + 1) / 2 * 2;
+  LaunchSetup ls(dim3(cols, row_tiles), dim3(NARROW_THREADS), (size_t)narrow_smem_bytes(stages), stream, PAIR_SLICES ? 2 : 1, true);
+  const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, gemm_narrow_kernel<OutT, GELU, LN, PAIR_SLICES>, ma, mb, mae, mbe, epi, M, N, K, stages,
+                                           make_idesc_narrow(op_dtype == B200_BF16 ? 1 : 0), status_word);
+  note_launches(1);
+  return status_from_cuda(e);
+}
+
 template <typename OutT, bool GELU, int LN>
 static int launch_narrow(const void* a, const void* b, const EpilogueArgs<OutT>& epi, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                          int op_dtype, const LnArgs& ln, int* status_word, cudaStream_t stream) {
-  if constexpr (sizeof(OutT) != 2 && LN < 3) {
+  if constexpr (sizeof(OutT) != 2 && (LN == 1 || LN == 2)) {
     return B200_ERR_UNSUPPORTED;
   } else {
-    if (takes_few_rows(M, N, LN)) return launch_few<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
-    static std::atomic<bool> attr_set[kMaxDevices];
-    const int slot = device_slot();
-    if (slot < 0) return B200_ERR_CUDA;
-    if (!attr_set[slot].load(std::memory_order_acquire)) {
-      if (cudaFuncSetAttribute(gemm_narrow_kernel<OutT, GELU, LN>, cudaFuncAttributeMaxDynamicSharedMemorySize, NARROW_SMEM_BYTES) != cudaSuccess)
-        return B200_ERR_CUDA;
-      attr_set[slot].store(true, std::memory_order_release);
+    if constexpr (LN == 2 || LN == 4) {
+      if (M > kNarrowMaxRows) return launch_narrow_tiles<OutT, GELU, LN, true>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
     }
-    CUtensorMap ma, mb, mae, mbe;
-    memset(&mae, 0, sizeof(mae));
-    memset(&mbe, 0, sizeof(mbe));
-    int st = make_map(&ma, a, M, K, lda, BM, op_dtype);
-    if (st == B200_OK) st = make_map(&mb, b, N, K, ldb, NARROW_BN, op_dtype);
-    if (st == B200_OK && LN == 1) st = make_map(&mae, ln.a_ext, M, kLnExtCols, kLnExtCols, BM, op_dtype);
-    if (st == B200_OK && LN == 1) st = make_map(&mbe, ln.b_ext, N, kLnExtCols, kLnExtCols, NARROW_BN, op_dtype);
-    if (st != B200_OK) return st;
-    LaunchSetup ls(dim3((unsigned)((N + NARROW_BN - 1) / NARROW_BN), (unsigned)((M + BM - 1) / BM)), dim3(NARROW_THREADS), NARROW_SMEM_BYTES, stream, 1, true);
-    const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, gemm_narrow_kernel<OutT, GELU, LN>, ma, mb, mae, mbe, epi, M, N, K,
-                                             make_idesc_narrow(op_dtype == B200_BF16 ? 1 : 0), status_word);
-    note_launches(1);
-    return status_from_cuda(e);
+    if ((sizeof(OutT) == 2 || LN >= 3) && takes_few_rows(M, N, LN)) return launch_few<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+    return launch_narrow_tiles<OutT, GELU, LN, false>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
   }
 }
 
-// Whether a product goes to the narrow-tile kernel: few rows, 16-bit output, vector-aligned output and residual.
+// Whether a plain or LayerNorm-aware product goes to the kernels with small tiles: vector-aligned output and residual where they are
+// 16-bit.  LN == 2 always does up to kNarrowMaxRows rows, for moments that do not depend on their number.
 template <typename OutT, int STATS>
-static bool takes_narrow_tiles(int64_t M, const void* out, int64_t ld_out, const void* residual, int64_t ld_res) {
-  return STATS == 0 && sizeof(OutT) == 2 && M <= kNarrowMaxRows && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ld_out % 8 == 0 &&
-         (!residual || ((reinterpret_cast<uintptr_t>(residual) & 15) == 0 && ld_res % 8 == 0));
+static bool takes_narrow_tiles(int64_t M, int64_t N, int ln, const void* out, int64_t ld_out, const void* residual, int64_t ld_res) {
+  if (STATS != 0) return false;
+  if (sizeof(OutT) == 2) {
+    if ((reinterpret_cast<uintptr_t>(out) & 15) || ld_out % 8 || (residual && ((reinterpret_cast<uintptr_t>(residual) & 15) || ld_res % 8))) return false;
+    if (ln == 2 ? M <= kNarrowMaxRows : takes_few_rows(M, N, ln)) return true;
+  }
+  return narrow_is_faster(M, N, ln);
 }
 
 // The persistent kernel: TMA epilogue where output and residual allow it, CTA pairs where there is more than one row tile.
@@ -2095,7 +2157,7 @@ static int launch_typed(const void* a, const void* b, const void* bias, const vo
   EpilogueArgs<OutT> epi{(const OutT*)bias, (const OutT*)residual, (OutT*)out, ld_res, ld_out, 0, am.val, am.idx, am.sum, am.ld, targets, target_val, 0,
                          ln.stats, ln.stats_out, ln.stats_out_ld};
   if constexpr (STATS == 0) {
-    if (takes_narrow_tiles<OutT, STATS>(M, out, ld_out, residual, ld_res)) return launch_narrow<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
+    if (takes_narrow_tiles<OutT, STATS>(M, N, LN, out, ld_out, residual, ld_res)) return launch_narrow<OutT, GELU, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
   }
   return launch_wide<OutT, GELU, STATS, LN>(a, b, epi, M, N, K, lda, ldb, op_dtype, ln, status_word, stream);
 }

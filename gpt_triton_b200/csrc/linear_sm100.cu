@@ -17,7 +17,11 @@ int launch(const b200_linear_args& p, const gemm::EpilogueArgs<OutT>& epi, cudaS
   if constexpr (!std::is_same<OutT, __half>::value) {
     if (linear_few_takes(p, LN)) return launch_linear_few<OutT, LN>(p, epi, stream);
   }
-  if (p.M <= gemm::kNarrowMaxRows)
+  // LN == 4 promises its sums of squares per 64 columns up to kNarrowMaxRows rows, which the wide kernel does not leave; LN == 5 needs an
+  // output that a tensor map takes there, and beyond those rows everywhere.
+  const bool mapped = LN != 5 || ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && p.ld_out % 8 == 0);
+  const bool small = LN == 4 ? gemm::narrow_is_faster(p.M, p.N, LN) : gemm::takes_few_rows(p.M, p.N, LN) || gemm::narrow_is_faster(p.M, p.N, LN);
+  if (p.M <= gemm::kNarrowMaxRows ? small || LN == 4 || !mapped : small && mapped)
     return gemm::launch_narrow<OutT, false, LN>(p.a, p.b, epi, p.M, p.N, p.K, p.lda, p.ldb, p.op_dtype, none, p.status_word, stream);
   return gemm::launch_wide<OutT, false, 0, LN>(p.a, p.b, epi, p.M, p.N, p.K, p.lda, p.ldb, p.op_dtype, none, p.status_word, stream);
 }
