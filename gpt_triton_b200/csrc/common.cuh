@@ -180,12 +180,20 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK : B200_ERR_CUDA; }
 
 // Whether kernels that do not ask for it are launched with the programmatic-stream-serialization attribute too: only when
-// the environment variable B200GPT_PDL=1 (read once) says so.  Long kernels do not ask: in a replayed CUDA graph they already
-// follow each other within 0.3 us, and letting the next kernel's CTAs take their SMs early cost 2 % of a forward at 512 x 300
-// tokens and 3 % at 64 x 300.  Launches of a few rows (kFewRowsPdl) do: they last 2-10 us, of which the start of the next
-// kernel is a good part.
+// the environment variable B200GPT_PDL=1 (read once) says so.  Who asks:
+//   - launches of a few rows (kFewRowsPdl): they last 2-10 us, of which the start of the next kernel is a good part;
+//   - every wide product: its CTAs hold nearly all of an SM's shared memory, so what starts early only fills SMs that the
+//     kernel in front has left, and barriers, tensor memory and descriptors are ready when it ends (a forward of the 124M
+//     model without | with: 10 x 300 tokens 1454 | 1359 us, 40 x 300 3592 | 3410; 355M, 4 x 500 2729 | 2594; 16 x 300 in
+//     fp32 2253 | 2175);
+//   - LayerNorms, row statistics out of moments, and attention of one launch's few tiles up to kMidRowsPdl rows.  Further
+//     up their many small CTAs take the SMs from the last tiles in front of them: LayerNorms on top of the wide products'
+//     gain at 4800 rows in fp32 2175 | 2140 us, at 19200 6773 | 6916; statistics at 3000 rows 1359 | 1326, at 4500
+//     1601 | 1571, at 6000 1927 | 1981; such attention at 2000 rows (355M) 2594 | 2551, at 8000 6365 | 6391.
+// Attention of many tiles does not: four CTAs of it fit an SM, and back to back they slow each other by up to 28 %.
 bool pdl_enabled();
 constexpr int64_t kFewRowsPdl = 512;
+constexpr int64_t kMidRowsPdl = 5120;
 
 // cudaLaunchConfig_t with room for the two attributes this library uses: cluster size and programmatic serialization.
 struct LaunchSetup {

@@ -175,7 +175,7 @@ static cudaError_t launch_ln_stats(const float2* moments, int64_t ld, int slices
     return cudaLaunchKernelEx(&ls.cfg, ln_stats_few_rows_kernel<T>, moments, ld, slices, slice_cols, (int)N, eps, (int)M, reinterpret_cast<float2*>(stats),
                               static_cast<T*>(ext));
   }
-  LaunchSetup ls(dim3((unsigned)((M + 255) / 256)), dim3(256), 0, stream);
+  LaunchSetup ls(dim3((unsigned)((M + 255) / 256)), dim3(256), 0, stream, 1, pdl_enabled() || M <= kMidRowsPdl);
   return cudaLaunchKernelEx(&ls.cfg, ln_stats_from_moments_kernel<T>, moments, ld, slices, slice_cols, (int)N, eps, M, reinterpret_cast<float2*>(stats),
                             static_cast<T*>(ext));
 }

@@ -1926,7 +1926,7 @@ static int launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, const CU
     attr_set[slot].store(true, std::memory_order_release);
   }
   const uint32_t idesc = make_idesc(op_dtype == B200_BF16 ? 1 : 0, BM * CTAS);
-  LaunchSetup ls(dim3((unsigned)(groups * CTAS)), dim3(NUM_THREADS), C::SMEM_BYTES, stream, CTAS);
+  LaunchSetup ls(dim3((unsigned)(groups * CTAS)), dim3(NUM_THREADS), C::SMEM_BYTES, stream, CTAS, true);
   // column panel: about 16 MB of B (panel_n * 256 rows of K 16-bit elements), at least 8 tiles
   int panel_n = (int)(16e6 / ((double)BN * (double)K * 2.0));
   if (panel_n < 8) panel_n = 8;
