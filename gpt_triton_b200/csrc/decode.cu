@@ -14,6 +14,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "mma_sync.cuh"
 
 namespace b200 {
 namespace {
@@ -95,13 +96,25 @@ __device__ __forceinline__ float warp_max(float v) {
 // rows of 16-bit data of at most 64 bytes): all keys and values of a block are loaded into registers before the first is used, one
 // trip to memory per block instead of two; worth it while the warps that these registers cost are not missed.
 // Before (four warps, or one from 16 per SM on, values loaded behind the softmax) -> now, us (HBM alone), 12 heads of 64, bf16: 8
-// sequences, 330 keys 17.5 -> 6.7; 16 17.6 -> 10.2; 32 18.2 -> 13.4; 128 38.8 -> 31.3 (20); 197 56.7 -> 39.3 (31); 256 56.0 (40), as
-// before; 512, 1000 keys 305 -> 272 (242).
-template <typename T, int D, int SPLIT, bool AHEAD>
-__global__ void __launch_bounds__(SPLIT == 1 ? 128 : 32 * SPLIT)
+// sequences, 330 keys 17.5 -> 6.7; 16 17.6 -> 10.2; 32 18.2 -> 13.4; 197 56.7 -> 39.3 (31).
+// STAGED (one warp per row, 16-bit data): with many sequences what bounds it is how much of the cache is on its way, and registers
+// hold too little of that.  Keys and values of a block come by cp.async into two slots of shared memory per warp; a slot is
+// refilled as soon as it has been read, so that 8 to 16 KB per warp are in flight at 12 warps an SM.  The same bits as the other
+// variants of one warp.  us, before -> now (HBM alone), 330 and 1000 keys: 128 sequences 31.3 -> 26.3 (20) and 78.7 -> 62.6 (61); 256
+// 56.2 -> 47.1 (40) and 155 -> 121 (122); 512 102 -> 89 (81) and 272 -> 240 (244); 25 heads of 32, 256 sequences 58 -> 49 and 154 -> 132.
+constexpr int kStagedWarps = 2;  // per block
+template <int D>
+constexpr int kStagedSlot = 64 * D * 2;  // bytes of a block of 16-bit keys, or of values
+template <int SPLIT, bool STAGED>
+constexpr int kDecodeWarps = SPLIT > 1 ? SPLIT : STAGED ? kStagedWarps : 4;
+
+template <typename T, int D, int SPLIT, bool AHEAD, bool STAGED = false>
+__global__ void __launch_bounds__(32 * kDecodeWarps<SPLIT, STAGED>)
 attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__ out, int64_t BH, int NH, int64_t cache_len, float scale_log2e,
                         const int* pos_dev, int* status_word) {
-  constexpr int WARPS = SPLIT == 1 ? 4 : SPLIT;
+  constexpr int WARPS = kDecodeWarps<SPLIT, STAGED>;
+  static_assert(!STAGED || (SPLIT == 1 && !AHEAD && sizeof(T) == 2), "one warp per row, 16-bit rows");
+  extern __shared__ __align__(128) uint8_t ring[];  // STAGED: per warp a slot for keys and one for values
   __shared__ __align__(16) float q_s[WARPS][D + 4];  // the second half of q sits 4 floats further on: the two lanes of a pair read different banks
   __shared__ float part_o[SPLIT == 1 ? 1 : WARPS][D];
   __shared__ float part_ml[WARPS][2];
@@ -112,7 +125,7 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
   static_assert(!AHEAD || (sizeof(T) == 2 && VECS <= 4), "a block's keys and values fit the registers");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int side = lane & 1, kl = lane >> 1;  // which half of the rows; which of the 16 key slots
-  const int64_t w = SPLIT == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
+  const int64_t w = SPLIT == 1 ? (int64_t)blockIdx.x * WARPS + warp : (int64_t)blockIdx.x;
   const int part = SPLIT == 1 ? 0 : warp;
   const int64_t b = w / NH;
   const int h = (int)(w % NH);
@@ -174,6 +187,29 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
   __syncwarp();
   // (the new token's own key and value are read from qkv_new below, not back from the cache)
   const int n_keys = pos + 1;
+  // STAGED: a block's rows on their way into a slot; a warp-wide copy covers whole rows, and the 16-byte pieces of a row are permuted by
+  // its number, so that the lanes' reads fall into different banks
+  constexpr int ROW = D * (int)sizeof(T), PIECES = ROW / 16;
+  uint8_t* const keys_s = ring + (STAGED ? warp * 2 * kStagedSlot<D> : 0);
+  uint8_t* const values_s = keys_s + (STAGED ? kStagedSlot<D> : 0);
+  auto fetch = [&](uint8_t* slot, const T* rows, const T* newest, int k0) {
+    if (k0 < n_keys) {
+      const uint32_t to = (uint32_t)__cvta_generic_to_shared(slot);
+      const int c = lane % PIECES;
+#pragma unroll
+      for (int i = 0; i < 64 * PIECES / 32; ++i) {
+        const int r = i * (32 / PIECES) + lane / PIECES, key = k0 + r;
+        const T* src = (key == pos ? newest : rows + (int64_t)min(key, pos) * pitch) + c * 8;
+        warp_mma::cp_async16(to + (uint32_t)(r * ROW + ((c ^ (r & (PIECES - 1))) << 4)), src, key < n_keys);
+      }
+    }
+    warp_mma::cp_async_commit();  // (possibly empty: the waits count groups)
+  };
+  auto staged = [&](const uint8_t* slot, int r, int piece) { return *reinterpret_cast<const uint4*>(slot + r * ROW + ((piece ^ (r & (PIECES - 1))) << 4)); };
+  if constexpr (STAGED) {
+    fetch(keys_s, kc, kn, 0);
+    fetch(values_s, vc, vn, 0);
+  }
   const int n_groups = (n_keys + 64 * SPLIT - 1) / (64 * SPLIT);
   float m_run = -INFINITY;  // reference maximum of this warp's latest block
   float m_all = -INFINITY;  // running maximum over all blocks of the groups done so far
@@ -201,6 +237,10 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
         for (int c = 0; c < VECS; ++c) vraw[j][c] = key < n_keys ? vr[c] : make_uint4(0u, 0u, 0u, 0u);
       }
     }
+    if constexpr (STAGED) {
+      warp_mma::cp_async_wait<1>();  // the keys are there (the values may not be)
+      __syncwarp();
+    }
     float s[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -212,6 +252,7 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
         for (int c = 0; c < DH; c += 8) {
           float f[8];
           if constexpr (AHEAD) unpack8<T>(kraw[j][c / 8], f);
+          else if constexpr (STAGED) unpack8<T>(staged(keys_s, j * 16 + kl, side * (PIECES / 2) + c / 8), f);
           else load8(kr + c, f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) a = fmaf(q_mine[c + i], dot_operand<T>(f[i]), a);
@@ -219,6 +260,10 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
       }
       a += __shfl_xor_sync(0xffffffffu, a, 1);                      // the other half of the dot product
       s[j] = key < n_keys ? a * scale_log2e : -INFINITY;            // score in log2 units
+    }
+    if constexpr (STAGED) {
+      __syncwarp();
+      fetch(keys_s, kc, kn, k0 + 64);
     }
     const float bm = warp_max(fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])));
     float m_new = fmaxf(m_all, bm);
@@ -247,6 +292,10 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
     l_lane = fmaf(l_lane, mult, side == 0 ? psum : 0.f);  // (both lanes of a pair hold the same scores: count them once)
 #pragma unroll
     for (int d = 0; d < DH; ++d) o[d] *= mult;
+    if constexpr (STAGED) {
+      warp_mma::cp_async_wait<1>();  // the values are there (the next keys may not be)
+      __syncwarp();
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int key = k0 + j * 16 + kl;
@@ -256,11 +305,16 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
         for (int c = 0; c < DH; c += 8) {
           float f[8];
           if constexpr (AHEAD) unpack8<T>(vraw[j][c / 8], f);
+          else if constexpr (STAGED) unpack8<T>(staged(values_s, j * 16 + kl, side * (PIECES / 2) + c / 8), f);
           else load8(vr + c, f);
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[c + i] = fmaf(ph[j], dot_operand<T>(f[i]), o[c + i]);
         }
       }
+    }
+    if constexpr (STAGED) {
+      __syncwarp();
+      fetch(values_s, vc, vn, k0 + 64);
     }
   }
   // add up the lanes' pieces and denominators (all relative to the same maximum m_run)
@@ -302,30 +356,34 @@ attention_decode_kernel(const T* qkv_new, T* __restrict__ cache, T* __restrict__
   *reinterpret_cast<Vec<T, DPL>*>(out + b * H + (int64_t)h * D + col0) = res;
 }
 
-template <typename T, int D, int SPLIT, bool AHEAD>
+template <typename T, int D, int SPLIT, bool AHEAD, bool STAGED = false>
 int attention_decode_split(const void* qkv_new, void* cache, void* out, int64_t BH, int64_t NH, int64_t cache_len, float sl, const int* pos_dev,
                            int* status_word, cudaStream_t stream) {
-  const int64_t blocks = SPLIT == 1 ? (BH + 3) / 4 : BH;
+  constexpr int warps = kDecodeWarps<SPLIT, STAGED>;
+  const int64_t blocks = SPLIT == 1 ? (BH + warps - 1) / warps : BH;
   // (an early start helps blocks that all find room; 3072 of them in the way of the product in front cost a step with 256 sequences 10 %)
-  LaunchSetup ls(dim3((unsigned)blocks), dim3(SPLIT == 1 ? 128 : 32 * SPLIT), 0, stream, 1, pdl_enabled() || blocks <= 2 * sm_count());
-  const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, attention_decode_kernel<T, D, SPLIT, AHEAD>, (const T*)qkv_new, (T*)cache, (T*)out, BH, (int)NH, cache_len, sl,
-                                           pos_dev, status_word);
+  LaunchSetup ls(dim3((unsigned)blocks), dim3(32 * warps), STAGED ? warps * 2 * kStagedSlot<D> : 0, stream, 1, pdl_enabled() || blocks <= 2 * sm_count());
+  const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, attention_decode_kernel<T, D, SPLIT, AHEAD, STAGED>, (const T*)qkv_new, (T*)cache, (T*)out, BH, (int)NH,
+                                           cache_len, sl, pos_dev, status_word);
   note_launches(1);
   return status_from_cuda(e);
 }
 
 // How many (batch, head) pairs of a variant the current device has room for at once (0 if it cannot be asked).
-template <typename T, int D, int SPLIT, bool AHEAD>
+template <typename T, int D, int SPLIT, bool AHEAD, bool STAGED = false>
 int64_t heads_at_once() {
   static std::atomic<int> per_sm[kMaxDevices];  // blocks, + 1; 0: not asked yet
   const int slot = device_slot();
   if (slot < 0) return 0;
+  constexpr int warps = kDecodeWarps<SPLIT, STAGED>;
   int n = per_sm[slot].load(std::memory_order_relaxed);
   if (n == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attention_decode_kernel<T, D, SPLIT, AHEAD>, SPLIT == 1 ? 128 : 32 * SPLIT, 0) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attention_decode_kernel<T, D, SPLIT, AHEAD, STAGED>, 32 * warps,
+                                                      STAGED ? warps * 2 * kStagedSlot<D> : 0) != cudaSuccess)
+      return 0;
     per_sm[slot].store(++n, std::memory_order_relaxed);
   }
-  return (int64_t)(n - 1) * sm_count() * (SPLIT == 1 ? 4 : 1);
+  return (int64_t)(n - 1) * sm_count() * (SPLIT == 1 ? warps : 1);
 }
 
 template <typename T, int D>
@@ -339,9 +397,18 @@ int attention_decode_sized(const void* qkv_new, void* cache, void* out, int64_t 
     // (12 heads of 64, bf16, 222 sequences are one wave at one warp, 1.1 at two: 52.8 us against 58.4 at 330 keys, 14 against 21 at
     // 60; 173 sequences are one wave at two: 36 against 47).  A cache of one block of keys has nothing to share out (96 heads, 16
     // keys: 2.8 us with one warp, 3.8 with eight).  Four warps that load values behind the softmax, against one that loads ahead,
-    // 64 sequences, 100 / 330 / 1000 keys: 11.8 / 20.5 / 42.3 us against 9.8 / 20.0 / 48.5.  Nothing finds room: two warps (512
-    // sequences 67 / 176 us at 330 / 1000 keys against 96 / 275 with one, but 35 against 27 at 60), at head size 32 one that loads
-    // ahead (54 / 141 against 67 / 174 us with two), one for short caches.
+    // 64 sequences, 100 / 330 / 1000 keys: 11.8 / 20.5 / 42.3 us against 9.8 / 20.0 / 48.5.
+    // Many rows of more than one block: keys and values staged in shared memory (see the kernel).  Below 6 pairs per SM (10 of half the
+    // size) several warps per pair can be faster (12 heads of 64, 330 / 1000 keys: 32 sequences 13.7 / 30.5 us against 15.9 / 37.5, 64
+    // 20.5 / 42.6 against 18.6 / 45.0, but 128 31.3 / 78.7 against 26.3 / 62.6; 25 heads of 32: 32 sequences 12.8 / 23.8 against 12.9 /
+    // 29.5, 64 16.9 / 40.2 against 15.9 / 37.3).  At head size 64 an SM has room for 12 pairs, and a second wave that is not half
+    // full costs what it would save: 170 sequences 35.9 / 91.9 against 40.2 / 105.7, 197 39.7 / 102 against 41.8 / 116, but 222 52.7 / 145
+    // against 44.9 / 118.  At 32 it pays from one wave on (170 x 25 heads 42.0 / 117 against 37.6 / 98.7).
+    if (cache_len > 64 && BH >= (D == 64 ? 6 : 10) * (int64_t)sm_count()) {
+      const int64_t room = heads_at_once<T, D, 1, false, true>();
+      if (BH <= room || D == 32 || 2 * BH >= 3 * room)
+        return attention_decode_split<T, D, 1, false, true>(qkv_new, cache, out, BH, NH, cache_len, sl, pos_dev, status_word, stream);
+    }
     if (cache_len > 64) {
       B200_DECODE_IF_ROOM(8, true);
       B200_DECODE_IF_ROOM(4, true);
@@ -351,9 +418,7 @@ int attention_decode_sized(const void* qkv_new, void* cache, void* out, int64_t 
     B200_DECODE_IF_ROOM(1, true);
     if (cache_len > 64) B200_DECODE_IF_ROOM(2, false);
     B200_DECODE_IF_ROOM(1, false);
-    if (cache_len <= 128) B200_DECODE(1, false);
-    if (D == 32) B200_DECODE(1, true);
-    B200_DECODE(2, false);
+    B200_DECODE(1, false);
   } else {
     // rows too wide to be held: one warp per (batch, head) fills the GPU from about 16 warps per SM on; below that, four share one
     if (BH >= (int64_t)sm_count() * 16) B200_DECODE(1, false);
