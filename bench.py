@@ -480,7 +480,7 @@ def run_gpu_arm(args, rank, world, local_rank):
             "weak_per_gpu": weak,
             "device_status": status["code"],
             "gpu_launches": int(launches), "launch_mode": f"CUDA graph replay, {launches_per_forward} library kernels per forward, "
-                                                          f"programmatic dependent launch {'on' if os.environ.get('B200GPT_PDL', '0') == '1' else 'off'}",
+                                                          f"programmatic dependent launch of {'every kernel' if os.environ.get('B200GPT_PDL', '0') == '1' else 'products'}",
             "roofline": {"kernel": "gemm_tn_kernel (tcgen05, all GEMM shapes of the forward)", "bound": "tensor",
                          "achieved": achieved_tflops, "peak": peak_tflops, "unit": "TFLOP/s", "frac": achieved_tflops / peak_tflops,
                          "peak_source": f"{peak_kind}: cuBLAS bf16 sustained",
