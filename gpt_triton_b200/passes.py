@@ -110,6 +110,12 @@ def _run(name, args, device):
         check(run(ctypes.byref(args), stream_ptr(device)), name)
 
 
+def registered(module, names):
+    """Whether the weights `names` of a module are parameters of its own.  Others (computed, or put beside the parameter as pruning does)
+    change without a trace that a table's tags would show; the operators read them anew in every pass."""
+    return all(module._parameters.get(n) is not None for n in names)
+
+
 # ----------------------------------------------------------------------------- FusedGPT
 def _gpt_table(model, blocks, folded):
     h, wte = model.config.n_embd, model.wte_weight
@@ -120,15 +126,15 @@ def _gpt_table(model, blocks, folded):
               {"layer_norm_weight": (h,), "layer_norm_bias": (h,), "ffn1_weight": (h, 4 * h), "ffn1_bias": (4 * h,), "ffn2_weight": (4 * h, h), "ffn2_bias": (h,)})
     if model.wpe_weight.shape[1] != h or wte.shape[1] != h or not (wte.is_contiguous() and model.wpe_weight.is_contiguous()) or model.wpe_weight.dtype != wte.dtype:
         return None
-    entries, tensors = (GptBlock * len(blocks))(), []
-    for entry, pair in zip(entries, blocks):
+    for pair in blocks:
         if pair[0].num_heads != heads:
             return None
         for m, want in zip(pair, shapes):
-            if any(tuple(m._parameters[n].shape) != s or m._parameters[n].dtype != wte.dtype or m._parameters[n].device != wte.device
-                   or not m._parameters[n].is_contiguous() for n, s in want.items()):
+            if not registered(m, want) or any(tuple(m._parameters[n].shape) != s or m._parameters[n].dtype != wte.dtype or m._parameters[n].device != wte.device
+                                              or not m._parameters[n].is_contiguous() for n, s in want.items()):
                 return None
-        att, mlp = pair
+    entries, tensors = (GptBlock * len(blocks))(), []
+    for entry, (att, mlp) in zip(entries, blocks):
         if folded:
             qkv = att._operand.folded(att.c_attn_weight, att.layer_norm_weight, att.layer_norm_bias, att.c_attn_bias)
             up = mlp._operand.folded(mlp.ffn1_weight, mlp.layer_norm_weight, mlp.layer_norm_bias, mlp.ffn1_bias)

@@ -139,3 +139,19 @@ def test_a_decoder_notices_changes():
     model.logits(ids)
     _both(model, lambda: model.logits(ids))
     assert not torch.equal(model.logits(ids), first)
+
+
+def test_a_pruned_gpt_runs_its_operators():
+    from torch.nn.utils import prune
+
+    from gpt_triton_b200 import passes
+    from gpt_triton_b200.gpt import FusedAttention, FusedMLP
+
+    model = _gpt(torch.float16)
+    ids = torch.randint(0, 300, (2, 40), device=DEV)
+    for _ in range(3):
+        first = model(ids)
+    prune.l1_unstructured(model.blocks[1][1], "ffn2_bias", amount=0.5)
+    for _ in range(3):
+        assert not torch.equal(model(ids), first)
+    assert passes.gpt_body(model, ids, None, None, FusedAttention, FusedMLP) is None
