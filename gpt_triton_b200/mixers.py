@@ -62,6 +62,10 @@ class _Sublayer(_EvalOnly):
         p = getattr(self, name)
         return self._operand.derived(("f32", name), (p,), lambda: p.data.float().contiguous())
 
+    def _shapes(self, width):
+        """Name -> shape of the weights that a whole pass reads."""
+        raise NotImplementedError
+
     def _describe(self, e, kind, w_in, starts, w_out, **vectors):
         """Fills what every passes.Sublayer `e` has; `vectors`: its tensors by field.  Returns the tensors it names."""
         e.kind = kind
@@ -92,6 +96,11 @@ class LatentAttention(_Sublayer):
         self.uk, self.uv = _weight(heads * dim, kv_rank), _weight(heads * vdim, kv_rank)
         self.sink = _weight(heads)
         self.o = _weight(width, heads * vdim)
+
+    def _shapes(self, width):
+        q, v, r = self.heads * self.dim, self.heads * self.vdim, self.kv_rank
+        own = {} if self.shares is not None else {"dkv": (r, width), "dkv_norm": (r,)}
+        return {"q": (q, width), **own, "uk": (q, r), "uv": (v, r), "sink": (self.heads,), "o": (width, v)}
 
     def new_cache(self, batch, capacity, device, dtype):
         """Latents of the last tokens: as many as any reader's window sees."""
@@ -162,6 +171,10 @@ class LightningAttention(_Sublayer):
         self.norm = _weight(heads * vdim)
         self.o = _weight(width, heads * vdim)
 
+    def _shapes(self, width):
+        q, v = self.heads * self.dim, self.heads * self.vdim
+        return {"q": (q, width), "k": (q, width), "v": (v, width), "g": (v, width), "norm": (v,), "o": (width, v)}
+
     def new_cache(self, batch, capacity, device, dtype):
         return torch.empty((batch, self.heads, self.dim, self.vdim), device=device, dtype=torch.float32)
 
@@ -199,6 +212,9 @@ class DenseFeedForward(_Sublayer):
         self.act, self.ff = act, ff
         self.up, self.down = _weight(ff, width), _weight(width, ff)
 
+    def _shapes(self, width):
+        return {"up": (self.ff, width), "down": (width, self.ff)}
+
     def describe(self, e, at):
         e.act, e.ff = K.ACTIVATIONS[self.act], self.ff
         return self._describe(e, passes.DENSE, self._stacked("up")[0], (), self._stacked("down")[0])
@@ -228,6 +244,11 @@ class DifferentialAttention(_Sublayer):
         self.lq1, self.lk1, self.lq2, self.lk2 = (_weight(dim) for _ in range(4))
         self.g = _weight(heads, width)
         self.o = _weight(width, heads * vdim)
+
+    def _shapes(self, width):
+        q, k, v = 2 * self.heads * self.dim, 2 * self.kv_heads * self.dim, self.kv_heads * self.vdim
+        per_head = dict.fromkeys(("q_norm", "k_norm", "lq1", "lk1", "lq2", "lk2"), (self.dim,))
+        return {"q": (q, width), "k": (k, width), "v": (v, width), **per_head, "g": (self.heads, width), "o": (width, self.heads * self.vdim)}
 
     def new_cache(self, batch, capacity, device, dtype):
         """Keys and values of the tokens that the window can see."""
@@ -296,6 +317,11 @@ class GatedDeltaRule(_Sublayer):
         self.norm = _weight(vdim)
         self.o = _weight(width, heads * vdim)
 
+    def _shapes(self, width):
+        h, k, v = self.heads, self.kv_heads * self.dim, self.heads * self.vdim
+        return {"q": (k, width), "k": (k, width), "v": (v, width), "q_conv": (k, self.taps), "k_conv": (k, self.taps), "v_conv": (v, self.taps),
+                "a": (h, width), "b": (h, width), "g": (v, width), "A_log": (h,), "dt_bias": (h,), "norm": (self.vdim,), "o": (width, v)}
+
     def _conv_cols(self):
         up = lambda n: (n + 7) // 8 * 8
         return 2 * up(self.kv_heads * self.dim) + self.heads * self.vdim
@@ -353,6 +379,9 @@ class GatedFeedForward(_Sublayer):
         self.ff, self.limit, self.alpha = ff, limit, alpha
         self.gate, self.up, self.down = _weight(ff, width), _weight(ff, width), _weight(width, ff)
         self.gate_b, self.up_b, self.down_b = _weight(ff), _weight(ff), _weight(width)
+
+    def _shapes(self, width):
+        return {"gate": (self.ff, width), "up": (self.ff, width), "down": (width, self.ff), "gate_b": (self.ff,), "up_b": (self.ff,), "down_b": (width,)}
 
     def _pairs(self):
         w = self._operand.derived(("pairs",), (self.gate, self.up), lambda: K.operand_rows(K.interleave_gated(self.gate.data, self.up.data))[0])

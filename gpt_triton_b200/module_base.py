@@ -49,17 +49,18 @@ _PLAIN = {int, float, str, tuple, type(None)}
 
 def parameter_tags(module, structure=False):
     """What tells whether a parameter of `module` or of one below it was replaced, cast, moved or written in place: equal lists, no
-    change.  With `structure` also whether a module was exchanged, one of its constants set or derived operands dropped.  (A walk over the module tree's own
-    dictionaries: Module.parameters() takes 3 us per parameter, as long as a launch.)"""
+    change.  With `structure` also whether one was renamed, added or taken away (a weight that is pruned, say, is no parameter any more), a
+    module exchanged, one of its constants set or derived operands dropped.  (A walk over the module tree's own dictionaries:
+    Module.parameters() takes 3 us per parameter, as long as a launch.)"""
     tags, stack = [], [module]
     while stack:
         m = stack.pop()
         d = m.__dict__
         if structure:
-            tags.append(m.__class__)
+            tags += (m.__class__, *d["_parameters"])
             cache = d.get("_operand")
             if cache is not None:
-                tags.append((cache.cleared, d.get("config"), [v for v in d.values() if v.__class__ in _PLAIN]))
+                tags.append((cache.cleared, d.get("config"), [(k, v) for k, v in d.items() if v.__class__ in _PLAIN]))
         for p in d["_parameters"].values():
             if p is not None:
                 tags.append((p.data_ptr(), p._version, p.dtype, p.device, p.shape))

@@ -158,6 +158,9 @@ class Nufasun(StreamDecoder):
         return self._operand.derived(("f32", id(param)), (param,), lambda: param.data.float().contiguous())
 
     def _table(self):
+        norms = [(layer, ("norm1", "norm1b") if layer.mlp is None else ("norm1", "norm1b", "norm2", "norm2b")) for layer in self.layers]
+        if not passes.stock(self, ("loop_step", "final_norm"), norms):
+            return None
         c, steps = self.config, self._f32(self.loop_step)
         subs, runs, tensors = [], [], [steps, self._f32(self.final_norm)]
         described = []

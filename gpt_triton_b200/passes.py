@@ -193,6 +193,14 @@ def gpt_body(model, ids, kv_caches, pos, attention_type, mlp_type):
 
 
 # ----------------------------------------------------------------------------- decoders with an fp32 residual stream
+def stock(model, names, layers):
+    """Whether a decoder is made of what a table describes: `names`: weights of its own, `layers`: (layer, names of its norms' weights), each
+    with a mixer `mix` and a feed-forward `mlp` or None."""
+    subs = [s for layer, _ in layers for s in (layer.mix, layer.mlp) if s is not None]
+    return (registered(model, names) and all(registered(layer, norms) for layer, norms in layers)
+            and all(registered(s, s._shapes(model.config.width)) for s in subs))
+
+
 def operand(entry, name, weight):
     """A (N, K) operand into the fields `name`, n_ / ld_ of the same suffix."""
     setattr(entry, "w_" + name, weight.data_ptr())

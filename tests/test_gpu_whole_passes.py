@@ -155,3 +155,23 @@ def test_a_pruned_gpt_runs_its_operators():
     for _ in range(3):
         assert not torch.equal(model(ids), first)
     assert passes.gpt_body(model, ids, None, None, FusedAttention, FusedMLP) is None
+
+
+@pytest.mark.parametrize("kind,where", [("fogilix", "layers.0.mlp.down"), ("fogilix", "layers.1.mix.o"), ("nufasun", "layers.0.mix.o"),
+                                        ("nufasun", "layers.1.mlp.down_b"), ("nufasun", "layers.1.norm1b")])
+def test_a_decoder_notices_pruning(kind, where):
+    """A pruned weight is no parameter any more; pruned again it is another tensor under the same name."""
+    from torch.nn.utils import prune
+
+    model = _decoder(kind)
+    ids = torch.randint(0, 211, (2, 50), device=DEV)
+    owner, _, name = where.rpartition(".")
+    last = model.logits(ids)
+    for _ in range(2):
+        for _ in range(3):
+            model.logits(ids)
+        prune.random_unstructured(model.get_submodule(owner), name, amount=0.5)
+        for _ in range(3):
+            _both(model, lambda: model.logits(ids))
+        assert not torch.equal(model.logits(ids), last)
+        last = model.logits(ids)

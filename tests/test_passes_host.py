@@ -5,12 +5,40 @@ import pytest
 import torch
 from torch.nn.utils import prune
 
+import fogilix_cases
+import nufasun_cases
 from gpt_triton_b200 import passes
+from gpt_triton_b200.fogilix import Fogilix, FogilixConfig
 from gpt_triton_b200.gpt import FusedGPT, GPTConfig
+from gpt_triton_b200.module_base import parameter_tags
+from gpt_triton_b200.nufasun import Nufasun, NufasunConfig
 
 
 def _gpt():
     return FusedGPT(GPTConfig(vocab_size=64, block_size=16, n_layer=2, n_head=2, n_embd=32)).eval()
+
+
+def _decoder(kind):
+    if kind == "fogilix":
+        return Fogilix(FogilixConfig.from_dict(fogilix_cases.CONFIGS["mixed"])).bfloat16().eval()
+    return Nufasun(NufasunConfig.from_dict(nufasun_cases.CONFIGS["mixed"])).bfloat16().eval()
+
+
+def _is_stock(model):
+    """Whether the checks in front of a table let the model through (what follows them launches kernels)."""
+    class Passed(Exception):
+        pass
+
+    def derived(*args):
+        raise Passed
+
+    model._operand.derived = derived
+    try:
+        return model._table() is not None
+    except Passed:
+        return True
+    finally:
+        del model._operand.derived
 
 
 def _blocks(model):
@@ -22,3 +50,17 @@ def test_a_gpt_weight_that_is_no_parameter_is_not_covered(slot, name):
     model = _gpt()
     prune.random_unstructured(model.blocks[1][slot], name, amount=0.5)
     assert passes._gpt_table(model, _blocks(model), folded=False) is None
+
+
+@pytest.mark.parametrize("kind", ["fogilix", "nufasun"])
+def test_pruning_is_noticed_and_not_covered(kind):
+    """Also of the last parameter of a module, whose successor `..._orig` takes its place."""
+    for name in ("mix.o", "mix.q", "mlp.down", "mlp.up", "norm1"):
+        model = _decoder(kind)
+        assert _is_stock(model)
+        owner, _, weight = name.rpartition(".")
+        before = parameter_tags(model, structure=True)
+        assert parameter_tags(model, structure=True) == before
+        prune.random_unstructured(model.layers[0].get_submodule(owner), weight, amount=0.5)
+        assert parameter_tags(model, structure=True) != before
+        assert not _is_stock(model)
