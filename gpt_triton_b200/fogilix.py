@@ -131,7 +131,7 @@ class Fogilix(StreamDecoder):
         return [layer.mix.new_cache(batch, capacity, dev, dtype) for layer in self.layers]
 
     def _table(self):
-        if not passes.stock(self, ("final_norm",), [(layer, ("norm1",) if layer.mlp is None else ("norm1", "norm2")) for layer in self.layers]):
+        if not passes.stock(self, [("final_norm", (self.config.width,))], [(layer, ("norm1",) if layer.mlp is None else ("norm1", "norm2")) for layer in self.layers]):
             return None
         first, subs = self._sublayers()
         entries, tensors, layers = (passes.Sublayer * len(subs))(), [self._gain(first)], []

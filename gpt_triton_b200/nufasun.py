@@ -159,7 +159,8 @@ class Nufasun(StreamDecoder):
 
     def _table(self):
         norms = [(layer, ("norm1", "norm1b") if layer.mlp is None else ("norm1", "norm1b", "norm2", "norm2b")) for layer in self.layers]
-        if not passes.stock(self, ("loop_step", "final_norm"), norms):
+        width = self.config.width
+        if not passes.stock(self, [("loop_step", (self.config.loop.times, width)), ("final_norm", (width,))], norms):
             return None
         c, steps = self.config, self._f32(self.loop_step)
         subs, runs, tensors = [], [], [steps, self._f32(self.final_norm)]

@@ -193,12 +193,16 @@ def gpt_body(model, ids, kv_caches, pos, attention_type, mlp_type):
 
 
 # ----------------------------------------------------------------------------- decoders with an fp32 residual stream
-def stock(model, names, layers):
-    """Whether a decoder is made of what a table describes: `names`: weights of its own, `layers`: (layer, names of its norms' weights), each
-    with a mixer `mix` and a feed-forward `mlp` or None."""
-    subs = [s for layer, _ in layers for s in (layer.mix, layer.mlp) if s is not None]
-    return (registered(model, names) and all(registered(layer, norms) for layer, norms in layers)
-            and all(registered(s, s._shapes(model.config.width)) for s in subs))
+def stock(model, norms, layers):
+    """Whether a decoder is what a table describes: `norms`: (name, shape) of weights of its own, `layers`: (layer, names of its norms'
+    weights), each with a mixer `mix` and a feed-forward `mlp` or None.  Every weight has the shape that the modules' constants give (those
+    size the workspace: wider weights would be written past it), the type of the embeddings, and lies where they do."""
+    embed, W = model.embed, model.config.width
+    weights = [(model, {"embed": (embed.shape[0], W), **dict(norms)})] + [(layer, dict.fromkeys(names, (W,))) for layer, names in layers]
+    weights += [(s, s._shapes(W)) for layer, _ in layers for s in (layer.mix, layer.mlp) if s is not None]
+    return embed.is_contiguous() and all(registered(m, shapes) and all(p.shape == shape and p.dtype == embed.dtype and p.device == embed.device
+                                                                       for p, shape in ((m._parameters[n], shapes[n]) for n in shapes))
+                                         for m, shapes in weights)
 
 
 def operand(entry, name, weight):
@@ -217,14 +221,14 @@ def sections(entry, starts):
 def decoder_rows(model, ids, ctx, step, table, memories):
     """ids (rows,) -> (rows behind the last norm as written, sums of squares or None); `memories`: one tuple of tensors (or None)
     per sublayer, as `memory_ok` has passed them."""
-    dev, extra, subs = model.embed.device, table.extra, table.entries
-    n_subs, T, W = len(subs), ids.numel(), model.embed.shape[1]
+    embed, extra, subs = model.embed, table.extra, table.entries
+    dev, n_subs, T, W = embed.device, len(subs), ids.numel(), embed.shape[1]
     B = ctx.batch
     n = T // B
-    out = K._rows_empty(T, W, model.embed.dtype, dev)
+    out = K._rows_empty(T, W, embed.dtype, dev)
     sumsq = None
-    args = DecoderPassArgs(subs=ctypes.addressof(subs), ids=ids.data_ptr(), table=model.embed.data_ptr(), first_gain=extra.get("first_gain"),
-                           final_gain=extra.get("final_gain"), out=out.data_ptr(), n_subs=n_subs, B=B, n=n, V=model.embed.shape[0], W=W,
+    args = DecoderPassArgs(subs=ctypes.addressof(subs), ids=ids.data_ptr(), table=embed.data_ptr(), first_gain=extra.get("first_gain"),
+                           final_gain=extra.get("final_gain"), out=out.data_ptr(), n_subs=n_subs, B=B, n=n, V=embed.shape[0], W=W,
                            ld_out=max(out.stride(0), W), eps=extra["eps"], table_scale=extra.get("table_scale", 1.0), both_norms=int(extra["both_norms"]),
                            status_word=K._status_ptr(dev))
     if not extra["both_norms"]:
@@ -251,8 +255,9 @@ def decoder_rows(model, ids, ctx, step, table, memories):
 
 def call_ok(model, ids, ctx, step):
     """Whether a call is one the passes cover: bf16, ids and positions where the model is, nothing being captured."""
-    dev = model.embed.device
-    if model.embed.dtype != torch.bfloat16 or not (ids.is_cuda and ids.device == dev and ids.dtype == torch.int64 and ids.is_contiguous()):
+    embed = model.embed
+    dev = embed.device
+    if embed.dtype != torch.bfloat16 or not (embed.is_contiguous() and ids.is_cuda and ids.device == dev and ids.dtype == torch.int64 and ids.is_contiguous()):
         return False
     if ids.numel() == 0 or ids.numel() % ctx.batch or torch.cuda.is_current_stream_capturing():
         return False

@@ -175,3 +175,20 @@ def test_a_decoder_notices_pruning(kind, where):
             _both(model, lambda: model.logits(ids))
         assert not torch.equal(model.logits(ids), last)
         last = model.logits(ids)
+
+
+@pytest.mark.parametrize("kind", ["fogilix", "nufasun"])
+def test_a_decoder_with_a_wider_feed_forward_runs_its_operators(kind):
+    """The feed-forward's width is a constant of its module; the weights are twice as wide (Nufasun: a constant that the products check)."""
+    model = _decoder(kind)
+    ids = torch.randint(0, 211, (2, 50), device=DEV)
+    first = [model.logits(ids) for _ in range(3)][-1]
+    mlp = model.layers[0].mlp
+    if kind == "nufasun":
+        mlp.ff *= 2
+    for name, p in list(mlp._parameters.items()):
+        if name != "down_b":
+            setattr(mlp, name, torch.nn.Parameter(torch.cat([p.data, 0.5 * p.data], 1 if name == "down" else 0)))
+    for _ in range(3):
+        _both(model, lambda: model.logits(ids))
+    assert not torch.equal(model.logits(ids), first)

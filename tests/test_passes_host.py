@@ -64,3 +64,34 @@ def test_pruning_is_noticed_and_not_covered(kind):
         prune.random_unstructured(model.layers[0].get_submodule(owner), weight, amount=0.5)
         assert parameter_tags(model, structure=True) != before
         assert not _is_stock(model)
+
+
+@pytest.mark.parametrize("kind", ["fogilix", "nufasun"])
+def test_weights_of_other_sizes_types_and_places_are_not_covered(kind):
+    """The constants of the modules size the workspace, so weights of other sizes stay with the operators, which go by the weights."""
+    def wider(model):
+        mlp = model.layers[0].mlp
+        for name, dim in (("gate", 0), ("up", 0), ("gate_b", 0), ("up_b", 0), ("down", 1)):
+            if name in mlp._parameters:
+                p = mlp._parameters[name]
+                setattr(mlp, name, torch.nn.Parameter(torch.cat([p.data, p.data], dim)))
+
+    def deeper(model):
+        model.layers[0].mix.o = torch.nn.Parameter(torch.zeros(144, 8).bfloat16())
+
+    def float32(model):
+        model.layers[1].mix.q.data = model.layers[1].mix.q.data.float()
+
+    def transposed(model):
+        model.embed.data = model.embed.data.t().contiguous().t()
+
+    def elsewhere(model):
+        model.layers[0].mix.q = torch.nn.Parameter(model.layers[0].mix.q.data.to("meta"))
+
+    for change in (wider, deeper, float32, transposed, elsewhere):
+        model = _decoder(kind)
+        assert _is_stock(model)
+        before = parameter_tags(model, structure=True)
+        change(model)
+        assert not _is_stock(model), change
+        assert parameter_tags(model, structure=True) != before
