@@ -16,6 +16,11 @@ class _OperandCache:
         self._slots = {}
         self.cleared = 0  # times; what is derived from these operands elsewhere goes with them
 
+    def __reduce__(self):
+        """A copied or pickled model starts without: everything here can be derived again, and what holds addresses (passes.Table) would
+        name the original's operands."""
+        return type(self), ()
+
     def clear(self):
         self._slots.clear()
         self.cleared += 1

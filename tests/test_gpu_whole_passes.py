@@ -192,3 +192,21 @@ def test_a_decoder_with_a_wider_feed_forward_runs_its_operators(kind):
     for _ in range(3):
         _both(model, lambda: model.logits(ids))
     assert not torch.equal(model.logits(ids), first)
+
+
+@pytest.mark.parametrize("make", [lambda: _gpt(torch.bfloat16), lambda: _decoder("fogilix"), lambda: _decoder("nufasun")])
+def test_a_copy_is_a_model_of_its_own(make):
+    import copy
+
+    model = make()
+    ids = torch.randint(0, 200, (2, 50), device=DEV)
+    first = [model.logits(ids) for _ in range(3)][-1]
+    other = copy.deepcopy(model)
+    for _ in range(3):
+        assert torch.equal(other.logits(ids), first)
+    with torch.no_grad():
+        for p in other.parameters():
+            p.mul_(1.25)
+    for _ in range(3):
+        _both(other, lambda: other.logits(ids))
+        assert torch.equal(model.logits(ids), first) and not torch.equal(other.logits(ids), first)

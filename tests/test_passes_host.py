@@ -1,6 +1,10 @@
 """What decides whether a pass is issued as one host call (passes.py), as far as no GPU is needed: models that it does not cover, changes
 of a model that a table must notice."""
 
+import copy
+import io
+import pickle
+
 import pytest
 import torch
 from torch.nn.utils import prune
@@ -95,3 +99,16 @@ def test_weights_of_other_sizes_types_and_places_are_not_covered(kind):
         change(model)
         assert not _is_stock(model), change
         assert parameter_tags(model, structure=True) != before
+
+
+@pytest.mark.parametrize("make", [_gpt, lambda: _decoder("fogilix"), lambda: _decoder("nufasun")])
+def test_a_model_with_a_table_can_be_copied_and_saved(make):
+    model = make()
+    model._operand._slots[("pass",)] = ("tags", passes.Table((passes.Sublayer * 2)(), []))
+    model._operand._slots[("gpt pass", True)] = ("tags", passes.Table((passes.GptBlock * 2)(), []))
+    file = io.BytesIO()
+    torch.save(model, file)
+    file.seek(0)
+    for other in (copy.deepcopy(model), pickle.loads(pickle.dumps(model)), torch.load(file, weights_only=False)):
+        assert other._operand is not model._operand and not other._operand._slots and len(model._operand._slots) == 2
+        assert all(torch.equal(a, b) and a.data_ptr() != b.data_ptr() for a, b in zip(model.parameters(), other.parameters()))
