@@ -209,14 +209,14 @@ class DenseFeedForward(_Sublayer):
 
     def __init__(self, width, ff, act="gelu_tanh"):
         super().__init__()
-        self.act, self.ff = act, ff
+        self.act = act
         self.up, self.down = _weight(ff, width), _weight(width, ff)
 
     def _shapes(self, width):
-        return {"up": (self.ff, width), "down": (width, self.ff)}
+        return {"up": (self.up.shape[0], width), "down": (width, self.up.shape[0])}
 
     def describe(self, e, at):
-        e.act, e.ff = K.ACTIVATIONS[self.act], self.ff
+        e.act, e.ff = K.ACTIVATIONS[self.act], self.up.shape[0]
         return self._describe(e, passes.DENSE, self._stacked("up")[0], (), self._stacked("down")[0])
 
     def memory(self, cache, batch):

@@ -12,9 +12,10 @@ class _OperandCache:
     so it cannot serve).  Writes made *through* ``param.data`` (``param.data.mul_(2)``) bump no counter torch
     exposes: after such a write call ``refresh_operands()`` on the model."""
 
+    cleared = 0  # times; what is derived from these operands elsewhere goes with them (of the class: files of earlier versions have none)
+
     def __init__(self):
         self._slots = {}
-        self.cleared = 0  # times; what is derived from these operands elsewhere goes with them
 
     def __reduce__(self):
         """A copied or pickled model starts without: everything here can be derived again, and what holds addresses (passes.Table) would

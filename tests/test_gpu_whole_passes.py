@@ -178,8 +178,8 @@ def test_a_decoder_notices_pruning(kind, where):
 
 
 @pytest.mark.parametrize("kind", ["fogilix", "nufasun"])
-def test_a_decoder_with_a_wider_feed_forward_runs_its_operators(kind):
-    """The feed-forward's width is a constant of its module; the weights are twice as wide (Nufasun: a constant that the products check)."""
+def test_a_decoder_with_a_wider_feed_forward(kind):
+    """Weights twice as wide (Nufasun's width is a constant of the module too, which the products check)."""
     model = _decoder(kind)
     ids = torch.randint(0, 211, (2, 50), device=DEV)
     first = [model.logits(ids) for _ in range(3)][-1]

@@ -92,7 +92,7 @@ def test_weights_of_other_sizes_types_and_places_are_not_covered(kind):
     def elsewhere(model):
         model.layers[0].mix.q = torch.nn.Parameter(model.layers[0].mix.q.data.to("meta"))
 
-    for change in (wider, deeper, float32, transposed, elsewhere):
+    for change in ((wider,) if kind == "nufasun" else ()) + (deeper, float32, transposed, elsewhere):
         model = _decoder(kind)
         assert _is_stock(model)
         before = parameter_tags(model, structure=True)
@@ -112,3 +112,18 @@ def test_a_model_with_a_table_can_be_copied_and_saved(make):
     for other in (copy.deepcopy(model), pickle.loads(pickle.dumps(model)), torch.load(file, weights_only=False)):
         assert other._operand is not model._operand and not other._operand._slots and len(model._operand._slots) == 2
         assert all(torch.equal(a, b) and a.data_ptr() != b.data_ptr() for a, b in zip(model.parameters(), other.parameters()))
+
+
+def test_a_model_saved_by_an_earlier_version():
+    """Its caches came with slots and without a count, its feed-forwards without a width."""
+    model = _decoder("fogilix")
+    for m in model.modules():
+        if "_operand" in m.__dict__:
+            cache = object.__new__(type(m._operand))
+            cache.__dict__["_slots"] = {}
+            m._operand = cache
+    assert not hasattr(model.layers[0].mlp, "ff")
+    tags = parameter_tags(model, structure=True)
+    assert _is_stock(model)
+    model.refresh_operands()
+    assert parameter_tags(model, structure=True) != tags
