@@ -402,3 +402,7 @@ class GatedFeedForward(_Sublayer):
         return K.linear(y, self._stacked("down")[0], bias=self._f32("down_b"))
 
     step = prompt
+
+
+for _kind in (LatentAttention, LightningAttention, DenseFeedForward, DifferentialAttention, GatedDeltaRule, GatedFeedForward):
+    passes.stands_for(_kind)

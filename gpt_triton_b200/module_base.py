@@ -63,13 +63,12 @@ def parameter_tags(module, structure=False):
         m = stack.pop()
         d = m.__dict__
         if structure:
-            tags += (m.__class__, *d["_parameters"])
+            tags.append(m.__class__)
+            tags.extend(d["_parameters"])
             cache = d.get("_operand")
             if cache is not None:
-                tags.append((cache.cleared, d.get("config"), [(k, v) for k, v in d.items() if v.__class__ in _PLAIN]))
-        for p in d["_parameters"].values():
-            if p is not None:
-                tags.append((p.data_ptr(), p._version, p.dtype, p.device, p.shape))
+                tags.append((cache.cleared, d.get("config"), [v for v in d.values() if v.__class__ in _PLAIN]))
+        tags.extend([(p.data_ptr(), p._version, p.dtype, p.device, p.shape) for p in d["_parameters"].values() if p is not None])
         stack.extend(c for c in d["_modules"].values() if c is not None)
     return tags
 

@@ -13,9 +13,11 @@ hidden rows 1810 -> 380, Fogilix prompt 1370 -> 350, Nufasun prompt 1890 -> 500;
 """
 
 import ctypes
+import operator
 import os
 
 import torch
+from torch import nn
 from torch.nn.modules import module as _nn_module
 
 from . import _lib
@@ -95,6 +97,33 @@ def table_of(model, key, build):
     return slot[1]
 
 
+_replaced = {}  # owner -> (its namespace, reads the names out of it, the functions): what a pass runs in the place of
+_methods = {}  # class of a module -> the names of its functions
+
+
+def stands_for(owner, *names):
+    """Passes run in the place of the functions `names` of kernels.py, or of all functions of a module's class."""
+    places = [(owner, names)]
+    if isinstance(owner, type):
+        places = [(c, [n for n, f in vars(c).items() if callable(f)]) for c in owner.__mro__[:owner.__mro__.index(nn.Module)]]
+        _methods[owner] = {n for _, names in places for n in names}
+    for place, names in places:
+        read = operator.itemgetter(*names)
+        _replaced[place] = (vars(place), read, read(vars(place)))
+
+
+def unchanged(modules):
+    """Whether every function that a pass would run in the place of is the package's own: the classes of `modules` exactly, no function
+    set on an instance, none replaced in a class or in kernels.py."""
+    return (all(read(space) == functions for space, read, functions in _replaced.values())
+            and all([m.__class__ in _methods and m.__dict__.keys().isdisjoint(_methods[m.__class__]) for m in modules]))
+
+
+stands_for(K, "fused_embeddings", "fused_layer_norm", "fused_ffn", "takes_operand_rows", "operand_ffn", "operand_ffn_residual", "kv_cache_fill", "split_qkv",
+           "flash_attention_v1", "attention_decode", "embedding_rms", "linear", "linear_residual", "latent_append", "window_attention", "latent_decode",
+           "decayed_attention", "stream_update", "gated_linear", "rotary_append", "pair_attention", "gated_delta")
+
+
 def _hooked(modules):
     if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
         return True
@@ -156,8 +185,12 @@ def _gpt_table(model, blocks, folded):
 def gpt_body(model, ids, kv_caches, pos, attention_type, mlp_type):
     """FusedGPT's blocks over ids (B, L) -> the residual stream (B, L, H); `pos`: a decode step (L = 1)."""
     wte, wpe = model.wte_weight, model.wpe_weight
+    if type(model.blocks) is not nn.ModuleList or any(type(b) is not nn.Sequential for b in model.blocks._modules.values()):
+        return None
     blocks = [tuple(b._modules.values()) for b in model.blocks._modules.values()]
     if not blocks or any(len(b) != 2 or type(b[0]) is not attention_type or type(b[1]) is not mlp_type or b[0].training or b[1].training for b in blocks):
+        return None
+    if not unchanged([m for b in blocks for m in b]):
         return None
     folded = model._folds()
     if not folded and _hooked(m for b in blocks for m in b):

@@ -210,3 +210,33 @@ def test_a_copy_is_a_model_of_its_own(make):
     for _ in range(3):
         _both(other, lambda: other.logits(ids))
         assert torch.equal(model.logits(ids), first) and not torch.equal(other.logits(ids), first)
+
+
+def test_functions_set_on_a_model_run():
+    """Set on a block, on a sublayer or in the place of an operator, after whole passes have run."""
+    from gpt_triton_b200 import kernels as K
+
+    ids = torch.randint(0, 200, (2, 50), device=DEV)
+    calls = []
+
+    def counted(fn):
+        def call(*args, **kwargs):
+            calls.append(fn)
+            return fn(*args, **kwargs)
+        return call
+
+    gpt, fogilix, nufasun = _gpt(torch.float16), _decoder("fogilix"), _decoder("nufasun")
+    for model, owner, name, per_pass in ((gpt, gpt.blocks[1][1], "forward_folded", 1), (gpt, K, "flash_attention_v1", 3), (fogilix, fogilix.layers[0].mlp, "prompt", 1),
+                                         (fogilix, K, "linear_residual", 6), (nufasun, nufasun.layers[3].mix, "_mix", 1), (nufasun, K, "gated_delta", 3)):
+        first = [model.logits(ids) for _ in range(3)][-1]
+        before = getattr(owner, name)
+        setattr(owner, name, counted(before))
+        try:
+            calls.clear()
+            for n in range(1, 4):
+                assert torch.equal(model.logits(ids), first) and len(calls) == n * per_pass
+        finally:
+            if owner is K:
+                K.__dict__[name] = before
+            else:
+                delattr(owner, name)

@@ -11,9 +11,10 @@ from torch.nn.utils import prune
 
 import fogilix_cases
 import nufasun_cases
-from gpt_triton_b200 import passes
+from gpt_triton_b200 import kernels as K
+from gpt_triton_b200 import mixers, passes
 from gpt_triton_b200.fogilix import Fogilix, FogilixConfig
-from gpt_triton_b200.gpt import FusedGPT, GPTConfig
+from gpt_triton_b200.gpt import FusedAttention, FusedGPT, GPTConfig
 from gpt_triton_b200.module_base import parameter_tags
 from gpt_triton_b200.nufasun import Nufasun, NufasunConfig
 
@@ -127,3 +128,34 @@ def test_a_model_saved_by_an_earlier_version():
     assert _is_stock(model)
     model.refresh_operands()
     assert parameter_tags(model, structure=True) != tags
+
+
+def test_functions_that_are_not_the_packages_own(monkeypatch):
+    gpt, fogilix = _gpt(), _decoder("fogilix")
+    pairs, subs = [m for b in _blocks(gpt) for m in b], [s for layer in fogilix.layers for s in (layer.mix, layer.mlp) if s is not None]
+    assert passes.unchanged(pairs) and passes.unchanged(subs) and not passes.unchanged([torch.nn.Identity()])
+    for module, name, others in ((pairs[2], "forward_folded", pairs), (pairs[1], "forward", pairs), (subs[0], "prompt", subs), (subs[1], "_stacked", subs)):
+        setattr(module, name, lambda *args, **kwargs: None)
+        assert not passes.unchanged(others)
+        delattr(module, name)
+        assert passes.unchanged(others)
+    kind = type(subs[0])
+    subs[0].__class__ = type("Other", (kind,), {"prompt": lambda *args: None})
+    assert not passes.unchanged(subs)
+    subs[0].__class__ = kind
+    for owner, name in ((K, "linear"), (K, "fused_ffn"), (FusedAttention, "decode"), (mixers.LightningAttention, "_mix"), (mixers._Sublayer, "_stacked")):
+        with monkeypatch.context() as m:
+            m.setattr(owner, name, lambda *args, **kwargs: None)
+            assert not passes.unchanged(subs)
+        assert passes.unchanged(subs)
+
+
+def test_blocks_of_other_kinds_run_their_own_code():
+    """In front of anything that needs the GPU."""
+    for change in ("container", "block"):
+        model = _gpt()
+        if change == "container":
+            model.blocks[1].__class__ = type("Pair", (torch.nn.Sequential,), {})
+        else:
+            model.blocks[1][0].__class__ = type("Other", (FusedAttention,), {})
+        assert passes.gpt_body(model, torch.zeros((1, 4), dtype=torch.int64), None, None, FusedAttention, type(model.blocks[0][1])) is None
