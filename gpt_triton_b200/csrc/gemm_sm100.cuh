@@ -1968,12 +1968,15 @@ inline int few_rows_cols(int64_t M, int64_t N, int ln) {
 // 2048 -> 8192 256 (256) 12.8 | 21.1, 512 (512) 24.1 | 21.8; 2048 -> 10880 384 rows (510 against 86: two rounds each) 22.6 | 26.8, 512 (680) 31.6 | 27.0.
 // Beyond kNarrowMaxRows a row's sums pass from one CTA to the next (PAIR_SLICES), which two CTAs an SM do not hide: x += z 1024 -> 1024, 1024 rows
 // (128 tiles) 11.5 | 15.9, 1536 (192) 18.5 | 16.1; row statistics 1024 -> 1024, 2048 rows (256) 14.7 | 16.0, 768 -> 768, 3072 (288) 15.3 | 14.9.
+// Up to two rounds, as measured: with up to 128 columns the tiles need no more rounds than the wide kernel's however many rows there are, and
+// row tiles are the grid's second dimension, which ends at 65535 (8.4 million rows).
 inline bool narrow_is_faster(int64_t M, int64_t N, int ln) {
   const int64_t sms = sm_count(), narrow = (M + BM - 1) / BM * ((N + NARROW_BN - 1) / NARROW_BN);
   if (M > kNarrowMaxRows && ln == 4) return narrow <= sms;
   if (M > kNarrowMaxRows && ln == 2) return 4 * narrow <= 7 * sms;
   const int64_t wide = M > BM ? (M + 2 * BM - 1) / (2 * BM) * ((N + BN - 1) / BN) : (N + BN - 1) / BN, places = M > BM ? sms / 2 : sms;
-  return (narrow + 2 * sms - 1) / (2 * sms) <= (wide + places - 1) / places;
+  const int64_t rounds = (narrow + 2 * sms - 1) / (2 * sms);
+  return rounds <= 2 && rounds <= (wide + places - 1) / places;
 }
 // Whether a product goes to gemm_few_kernel: up to 64 rows, and above that as long as its tiles of 64
 // rows and 16 or 32 columns fit the GPU at once, two CTAs per SM.  Beyond that its smaller tiles read A and B more often than they

@@ -93,3 +93,22 @@ def test_products_around_deferred_norms(rows, K_, N):
     ref = zg * torch.sigmoid(1.7 * zg) * (zu + 1)
     assert ((out - ref).abs() <= 4 * (bound[:, :F] + bound[:, F:2 * F]) + ref.abs() * 2.0 ** -8 + 1e-5).all()
     assert K.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [64, 72])
+def test_more_row_tiles_than_a_grid_has_rows(N):
+    """65536 tiles of 128 rows: few columns, so that the rounds alone would allow small tiles at any number of rows."""
+    from gpt_triton_b200 import kernels as K
+
+    M, K_ = 65535 * 128 + 1, 16
+    a = torch.randn((M, K_), device=DEV, dtype=torch.float16)
+    w = torch.randn((N, K_), device=DEV, dtype=torch.float16) * 0.25
+    rows = torch.tensor([0, 127, 128, M // 2, M - 129, M - 2, M - 1], device=DEV)
+    want = a[rows].double() @ w.double().T
+    bound = 2e-6 * (a[rows].double().abs() @ w.double().abs().T) + 1e-6  # an fp32 sum of 16 exact products
+    got = K.fused_ffn(a, K.pack_weight(w, weight_is_nk=True))[rows].double()
+    assert ((got - want).abs() <= bound + want.abs() * 2.0 ** -11).all()
+    got = K.linear(a.bfloat16(), w.bfloat16(), out_dtype=torch.float32)[rows].double()
+    ab, wb = a[rows].bfloat16().double(), w.bfloat16().double()
+    assert ((got - ab @ wb.T).abs() <= 2e-6 * (ab.abs() @ wb.abs().T) + 1e-6).all()
+    assert K.device_status() == 0
