@@ -57,10 +57,23 @@ int gpt_pass(const b200_gpt_pass_args& p, Arena& arena, void* stream) {
   const int op = p.dtype == B200_BF16 ? B200_BF16 : B200_F16;
   const float scale = (float)(1.0 / sqrt((double)D));
   const int64_t in_strides[3] = {p.L * 3 * H, D, 3 * H}, out_strides[3] = {p.L * H, D, H};
-  void* x = arena.take(T * H * es);
+  // Float32 storage: every product takes fp16 operands; with more than 128 rows they leave their producers as such (except in a decode
+  // step, whose attention leaves float32 rows), else a pass converts them in front of the product.
+  const bool f32 = p.dtype == B200_F32;
+  auto attention_operands = [&](const b200_gpt_block& b) { return f32 && T > 128 && !p.pos_dev && aligned16(b.qkv_bias); };
+  auto mlp_operands = [&](const b200_gpt_block& b) { return f32 && T > 128 && aligned16(b.up_bias); };
+  int attention_es = f32 ? 2 : es, mlp_es = attention_es;  // of the widest rows of any block between its products
+  for (int64_t i = 0; f32 && i < p.n_blocks; ++i) {
+    if (!attention_operands(p.blocks[i])) attention_es = 4;
+    if (!mlp_operands(p.blocks[i])) mlp_es = 4;
+  }
+  // No more than the operators hold at a time.  The stream: x in front of a block's attention, x2 behind it.  x is the caller's out (the
+  // last product does not read it), and between attention and the end of the block, while x2 is the stream, it holds the normed rows.
+  void* x = p.out && aligned16(p.out) ? p.out : arena.take(T * H * es);
   void* x2 = arena.take(T * H * es);
-  void* wide = arena.take(T * 4 * H * es);  // q | k | v, later the feed-forward's middle
-  void* rows = arena.take(T * H * es);      // attention's output, normed rows
+  const int64_t qkv_bytes = (T * 3 * H * es + 255) & ~(int64_t)255;
+  void* wide = arena.take(std::max(qkv_bytes + T * H * attention_es, T * 4 * H * mlp_es));  // q | k | v and rows, later the feed-forward's middle
+  void* rows = static_cast<uint8_t*>(wide) + qkv_bytes;                                     // attention's output, normed rows in front of it
 
   auto attend = [&](const b200_gpt_block& b, int out_dtype) -> int {
     if (p.pos_dev) {
@@ -106,10 +119,8 @@ int gpt_pass(const b200_gpt_pass_args& p, Arena& arena, void* stream) {
     return B200_OK;
   }
 
-  // Operator by operator.  Float32 storage: every product takes fp16 operands; with more than 128 rows they leave their producers as
-  // such (except in a decode step, whose attention leaves float32 rows), else a pass converts them in front of the product.
-  const bool f32 = p.dtype == B200_F32;
-  void* packed = f32 ? arena.take(T * 4 * H * 2) : nullptr;
+  // Operator by operator.
+  void* packed = f32 && (attention_es == 4 || mlp_es == 4) ? arena.take(T * (mlp_es == 4 ? 4 : 1) * H * 2) : nullptr;
   auto product = [&](const void* a, bool is_operand, const void* w, int64_t ld, const void* bias, const void* residual, void* out, int64_t N, int64_t K,
                      int gelu) -> int {
     if (f32 && !is_operand) {
@@ -123,18 +134,18 @@ int gpt_pass(const b200_gpt_pass_args& p, Arena& arena, void* stream) {
   else B200_RUN(b200_embedding(p.ids, p.wte, p.wpe, x, p.B, p.L, p.V, p.P, H, p.dtype, nullptr, stream));
   for (int64_t i = 0; i < p.n_blocks; ++i) {
     const b200_gpt_block& b = p.blocks[i];
-    bool operands = f32 && T > 128 && !p.pos_dev && aligned16(b.qkv_bias);
+    bool operands = attention_operands(b);
     B200_RUN(b200_layernorm(x, b.ln1_w, b.ln1_b, rows, T, H, p.eps, p.dtype, operands ? B200_F16 : p.dtype, stream));
     B200_RUN(product(rows, operands, b.qkv, b.ld_qkv, b.qkv_bias, nullptr, wide, 3 * H, H, 0));
     const int st = attend(b, operands ? B200_F16 : p.dtype);
     if (st != B200_OK) return st;
     B200_RUN(product(rows, operands, b.proj, b.ld_proj, b.proj_bias, x, x2, H, H, 0));
-    operands = f32 && T > 128 && aligned16(b.up_bias);
-    B200_RUN(b200_layernorm(x2, b.ln2_w, b.ln2_b, rows, T, H, p.eps, p.dtype, operands ? B200_F16 : p.dtype, stream));
+    operands = mlp_operands(b);
+    B200_RUN(b200_layernorm(x2, b.ln2_w, b.ln2_b, x, T, H, p.eps, p.dtype, operands ? B200_F16 : p.dtype, stream));
     if (operands) {
-      B200_RUN(b200_gemm_operand(rows, b.up, static_cast<const float*>(b.up_bias), wide, T, 4 * H, H, H, b.ld_up, 4 * H, 1, p.status_word, stream));
+      B200_RUN(b200_gemm_operand(x, b.up, static_cast<const float*>(b.up_bias), wide, T, 4 * H, H, H, b.ld_up, 4 * H, 1, p.status_word, stream));
     } else {
-      B200_RUN(product(rows, false, b.up, b.ld_up, b.up_bias, nullptr, wide, 4 * H, H, 1));
+      B200_RUN(product(x, false, b.up, b.ld_up, b.up_bias, nullptr, wide, 4 * H, H, 1));
     }
     B200_RUN(product(wide, operands, b.down, b.ld_down, b.down_bias, x2, i + 1 < p.n_blocks ? x : p.out, H, 4 * H, 0));
   }

@@ -22,7 +22,8 @@ typedef struct {
 } b200_gpt_block;
 
 /* ids [B, L] -> the residual stream behind the last block, out [B * L, H].  pos_dev: a decode step (L == 1, every block with kv) at the
- * device-side position pos_dev[0].  H % 8 == 0; folded: 16-bit types only. */
+ * device-side position pos_dev[0].  H % 8 == 0; folded: 16-bit types only.  The workspace's size follows from the arguments, `out` and the
+ * blocks' biases included (a 16-byte aligned `out` holds the stream between blocks). */
 typedef struct {
   const b200_gpt_block* blocks;
   const int64_t* ids;

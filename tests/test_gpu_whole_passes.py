@@ -240,3 +240,21 @@ def test_functions_set_on_a_model_run():
                 K.__dict__[name] = before
             else:
                 delattr(owner, name)
+
+
+@pytest.mark.parametrize("dtype,fold,L", [(torch.float16, True, 96), (torch.bfloat16, False, 96), (torch.float32, False, 96), (torch.float32, False, 1)])
+def test_a_gpt_pass_holds_no_more_than_its_operators(dtype, fold, L):
+    """(The workspace is one block: a little more for sections rounded up to 256 bytes and its own rounding, of up to 2 MB.)"""
+    model = _gpt(dtype, layers=2)
+    model.fold_layer_norm = fold
+    ids = torch.randint(0, 300, (128 if L == 1 else 400, L), device=DEV)
+    peaks = []
+    for model.whole_passes in (True, False):
+        for _ in range(2):
+            model(ids)
+        torch.cuda.empty_cache()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        model(ids)
+        peaks.append(torch.cuda.max_memory_allocated() - before)
+    assert peaks[0] <= peaks[1] * 1.02 + (2 << 20), peaks

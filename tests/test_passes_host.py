@@ -159,3 +159,23 @@ def test_blocks_of_other_kinds_run_their_own_code():
         else:
             model.blocks[1][0].__class__ = type("Other", (FusedAttention,), {})
         assert passes.gpt_body(model, torch.zeros((1, 4), dtype=torch.int64), None, None, FusedAttention, type(model.blocks[0][1])) is None
+
+
+@pytest.mark.parametrize("dtype,folded,aligned,per_value", [("float16", 1, 1, 10), ("bfloat16", 0, 1, 10), ("float32", 0, 1, 18), ("float32", 0, 0, 28)])
+def test_workspace_of_a_gpt_pass(dtype, folded, aligned, per_value):
+    """What the operators hold at a time beside the result, in bytes per row and column of the stream (of which the result has one value):
+    16 bits: the stream 2, the feed-forward's middle 8 (with the result 12); float32 with operands as fp16: stream 4, q | k | v 12, attention's
+    output 2 (22); with products that convert their rows: stream 4, middle 16, converted 8 (32)."""
+    import ctypes
+
+    from gpt_triton_b200._lib import dtype_code
+
+    B, L, H = 16, 300, 768
+    blocks = (passes.GptBlock * 2)()
+    for i, b in enumerate(blocks):
+        b.qkv_bias = b.up_bias = 4096 if aligned or i == 0 else 4100
+    args = passes.GptPassArgs(blocks=ctypes.addressof(blocks), out=4096, n_blocks=2, heads=12, B=B, L=L, V=100, P=512, H=H, eps=1e-5,
+                              dtype=dtype_code(getattr(torch, dtype)), folded=folded)
+    need = passes._passes.b200_gpt_pass_workspace_bytes(ctypes.byref(args))
+    statistics = B * L * (8 + 64 * 2 + 8 * (H // 64 + 1)) if folded else 0
+    assert per_value * B * L * H <= need <= per_value * B * L * H + statistics + 8 * 256
