@@ -398,6 +398,11 @@ bool decoder_args_ok(const b200_decoder_pass_args* p) {
 
 extern "C" {
 
+int b200_passes_version(void) { return B200_PASSES_VERSION; }
+void b200_passes_struct_bytes(int64_t sizes[4]) {
+  sizes[0] = sizeof(b200_gpt_block), sizes[1] = sizeof(b200_gpt_pass_args), sizes[2] = sizeof(b200_sublayer), sizes[3] = sizeof(b200_decoder_pass_args);
+}
+
 int64_t b200_gpt_pass_workspace_bytes(const b200_gpt_pass_args* args) {
   if (!gpt_args_ok(args)) return 0;
   Arena arena(nullptr, 0);

@@ -55,11 +55,19 @@ class DecoderPassArgs(ctypes.Structure):
                   "int both_norms; ptr workspace; i64 workspace_bytes; ptr status_word")
 
 
+VERSION = 1  # of the structures above (B200_PASSES_VERSION)
+
+
 def _load():
     if not os.path.exists(PASSES_PATH):
         raise ImportError(f"{PASSES_PATH} is missing: run `python -m gpt_triton_b200.build`")
     _lib.load()  # first: the passes call it
     lib = ctypes.CDLL(PASSES_PATH)
+    sizes = (c_i64 * 4)()
+    if hasattr(lib, "b200_passes_struct_bytes"):
+        lib.b200_passes_struct_bytes(sizes)
+    if list(sizes) != [ctypes.sizeof(c) for c in (GptBlock, GptPassArgs, Sublayer, DecoderPassArgs)] or lib.b200_passes_version() != VERSION:
+        raise ImportError(f"{PASSES_PATH} was built from another version of include/b200_passes.h: run `python -m gpt_triton_b200.build`")
     for name, args in (("b200_gpt_pass", GptPassArgs), ("b200_decoder_pass", DecoderPassArgs)):
         size, run = getattr(lib, name + "_workspace_bytes"), getattr(lib, name)
         size.restype, size.argtypes = c_i64, [ctypes.POINTER(args)]

@@ -12,6 +12,12 @@
 extern "C" {
 #endif
 
+/* Counts changes of the structures below; b200_passes_version gives the library's.  A caller in another language, whose structures repeat
+ * these by hand, compares their sizes too: b200_gpt_block, b200_gpt_pass_args, b200_sublayer, b200_decoder_pass_args. */
+#define B200_PASSES_VERSION 1
+int b200_passes_version(void);
+void b200_passes_struct_bytes(int64_t sizes[4]);
+
 /* One block of a FusedGPT.  Operands are [N, ld] K-major 16-bit (b200_pack_operand; qkv and up with the LayerNorm in front folded in:
  * b200_fold_layernorm, whose extension they then have instead of a bias); biases and LayerNorm vectors in the storage type. */
 typedef struct {

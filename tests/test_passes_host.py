@@ -2,8 +2,11 @@
 of a model that a table must notice."""
 
 import copy
+import ctypes
 import io
+import os
 import pickle
+import re
 
 import pytest
 import torch
@@ -166,8 +169,6 @@ def test_workspace_of_a_gpt_pass(dtype, folded, aligned, per_value):
     """What the operators hold at a time beside the result, in bytes per row and column of the stream (of which the result has one value):
     16 bits: the stream 2, the feed-forward's middle 8 (with the result 12); float32 with operands as fp16: stream 4, q | k | v 12, attention's
     output 2 (22); with products that convert their rows: stream 4, middle 16, converted 8 (32)."""
-    import ctypes
-
     from gpt_triton_b200._lib import dtype_code
 
     B, L, H = 16, 300, 768
@@ -179,3 +180,27 @@ def test_workspace_of_a_gpt_pass(dtype, folded, aligned, per_value):
     need = passes._passes.b200_gpt_pass_workspace_bytes(ctypes.byref(args))
     statistics = B * L * (8 + 64 * 2 + 8 * (H // 64 + 1)) if folded else 0
     assert per_value * B * L * H <= need <= per_value * B * L * H + statistics + 8 * 256
+
+
+def test_structures_are_those_of_the_header():
+    """Names, order and kinds of the fields, which the libraries compare by size only."""
+    from conftest import ROOT
+
+    text = re.sub(r"/\*.*?\*/", "", open(os.path.join(ROOT, "include", "b200_passes.h")).read(), flags=re.S)
+    declared = {name: body for body, name in re.findall(r"typedef struct \{(.*?)\} (\w+);", text, flags=re.S)}
+    kinds = {"int64_t": ctypes.c_int64, "int": ctypes.c_int, "float": ctypes.c_float}
+    for name, ours in (("b200_gpt_block", passes.GptBlock), ("b200_gpt_pass_args", passes.GptPassArgs), ("b200_sublayer", passes.Sublayer),
+                       ("b200_decoder_pass_args", passes.DecoderPassArgs)):
+        fields = []
+        for line in declared.pop(name).split(";"):
+            first, *others = [part.strip() for part in line.split(",")]
+            if not first:
+                continue
+            kind = first.replace("const", "").split()[0].rstrip("*")
+            for part in (first, *others):
+                ident, length = re.search(r"(\w+)(?:\[(\d+)\])?$", part).groups()
+                plain = ctypes.c_void_p if "*" in part else kinds[kind]
+                fields.append((ident, plain * int(length) if length else plain))
+        assert fields == list(ours._fields_), name
+    assert not declared and f"#define B200_PASSES_VERSION {passes.VERSION}\n" in text
+    assert passes._passes.b200_passes_version() == passes.VERSION
