@@ -389,6 +389,7 @@ bool decoder_args_ok(const b200_decoder_pass_args* p) {
   for (int64_t i = 0; i < p->n_subs; ++i) {
     const b200_sublayer& s = p->subs[i];
     if (s.kind < B200_SUB_LIGHTNING || s.kind > B200_SUB_GATED) return false;
+    if (s.k_out != (s.kind == B200_SUB_DENSE || s.kind == B200_SUB_GATED ? s.ff : s.heads * s.vdim)) return false;  // what w_out reads
     if (s.kind == B200_SUB_LATENT && (s.source < 0 || s.source > i || p->subs[s.source].kind != B200_SUB_LATENT || p->subs[s.source].source != s.source)) return false;
   }
   return true;

@@ -204,3 +204,18 @@ def test_structures_are_those_of_the_header():
         assert fields == list(ours._fields_), name
     assert not declared and f"#define B200_PASSES_VERSION {passes.VERSION}\n" in text
     assert passes._passes.b200_passes_version() == passes.VERSION
+
+
+@pytest.mark.parametrize("kind,fields", [(passes.DENSE, {"ff": 96}), (passes.GATED, {"ff": 96}), (passes.LIGHTNING, {"heads": 4, "dim": 16, "vdim": 24}),
+                                         (passes.DELTA, {"heads": 4, "kv_heads": 2, "dim": 16, "vdim": 24, "conv_cols": 160, "taps": 4})])
+def test_an_output_product_of_another_depth_is_refused(kind, fields):
+    sub = (passes.Sublayer * 1)()
+    sub[0].kind, sub[0].k_out, sub[0].n_in = kind, 96, 192
+    for name, value in fields.items():
+        setattr(sub[0], name, value)
+    args = passes.DecoderPassArgs(subs=ctypes.addressof(sub), n_subs=1, B=1, n=5, V=10, W=64, ld_out=64, both_norms=int(kind in (passes.DELTA, passes.GATED)))
+    assert passes._passes.b200_decoder_pass_workspace_bytes(ctypes.byref(args)) > 0
+    sub[0].k_out = 104
+    assert passes._passes.b200_decoder_pass_workspace_bytes(ctypes.byref(args)) == 0
+    args.ids = args.table = args.out = args.sumsq_out = args.workspace = 4096
+    assert passes._passes.b200_decoder_pass(ctypes.byref(args), None) == 1
