@@ -24,7 +24,7 @@ from . import _lib
 from . import kernels as K
 from ._lib import c_i64, c_void_p, check, dtype_code, on_device, stream_ptr
 from .build import PASSES_PATH
-from .module_base import _OperandCache, parameter_tags
+from .module_base import parameter_tags
 
 _F = _lib._fields
 
@@ -261,7 +261,7 @@ def sections(entry, starts):
 
 def decoder_rows(model, ids, ctx, step, table, memories):
     """ids (rows,) -> (rows behind the last norm as written, sums of squares or None); `memories`: one tuple of tensors (or None)
-    per sublayer, as `memory_ok` has passed them."""
+    per sublayer, as its `memory` gave them."""
     embed, extra, subs = model.embed, table.extra, table.entries
     dev, n_subs, T, W = embed.device, len(subs), ids.numel(), embed.shape[1]
     B = ctx.batch

@@ -73,7 +73,7 @@ def test_gpt_notices_changes():
     model(ids)
     _both(model, lambda: model(ids))
     model.blocks[2] = torch.nn.Sequential(*reversed(list(model.blocks[2].children())))  # a shape that is not covered
-    with pytest.raises(Exception):
+    with pytest.raises(TypeError, match="kv_cache"):  # (the operators' own: a feed-forward takes no cache)
         model(ids)
 
 
