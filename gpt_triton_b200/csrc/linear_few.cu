@@ -241,14 +241,22 @@ int few_splits(int64_t N, int64_t K) {
 
 }  // namespace
 
-// Where this kernel is the better one.  Beyond one slice per SM gemm_few_kernel streams as fast (10880 x 2048 11.6 against 12.2 us at one
-// row), except for LN == 4, whose tiles it cuts to 16 columns (22 against 13).  From 9 rows on the sums take twice the MMAs and twice
-// the shared memory: 1024 x 1024 4.0 against 4.4, 4096 x 1024 4.6 against 5.7, gated pairs 8192 x 2048 9.4 against 9.7.
+// Where this kernel is the better one, up to 16 rows at once: which one it is depends on N and K alone, so that a row's result does not
+// depend on how many of them there are (gemm_few_kernel sums in another order).  From 9 rows on the sums take twice the MMAs and twice
+// the shared memory.  us, gemm_few_kernel -> this, N x K, 1 to 8 | 9 to 16 rows:
+//   act(z)  1024 x 512 3.1 -> 3.2 | 3.1 -> 3.9, 1024 x 1024 4.1 -> 3.3 | 4.1 -> 3.9, 1552 x 1024 4.7 -> 3.4 | 4.7 -> 4.2, 3088 x 1024 5.1 -> 4.3 | 5.1 ->
+//           5.2, 4096 x 1024 4.7 -> 4.6 | 4.6 -> 5.7, 2048 x 2048 6.0 -> 4.6 | 6.0 -> 5.4, 8192 x 2048 10.9 -> 9.2 | 10.9 -> 10.3
+//   pairs   5504 x 1024 5.4 -> 4.9 | 5.4 -> 5.9, 4096 x 2048 8.3 -> 5.8 | 8.4 -> 6.4, 8192 x 2048 10.0 -> 9.1 | 10.0 -> 10.0, 9408 x 2048 10.5 -> 10.1 |
+//           10.4 -> 11.1
+// Beyond one slice per SM gemm_few_kernel streams as fast (10880 x 2048 11.6 against 12.2 us at one row), except for LN == 4, whose tiles it
+// cuts to 16 columns (22 against 13).
 bool linear_few_takes(const b200_linear_args& p, int ln) {
   if (p.M < 1 || p.M > 16 || p.K < 512 || p.K % 8 || p.op_dtype != B200_BF16) return false;
-  const int64_t slices = (p.N + kCols - 1) / kCols;
+  const int64_t slices = (p.N + kCols - 1) / kCols, sms = sm_count();
   if (slices > 65535) return false;
-  return ln == 4 || (p.M <= 8 ? slices <= sm_count() : p.K >= 2048 && slices <= (ln == 5 ? sm_count() / 2 : sm_count()));
+  if (ln == 4) return true;
+  if (p.K < 2048) return p.K >= 1024 && 3 * slices <= sms;
+  return 8 * slices <= (ln == 5 ? 7 : 8) * sms;
 }
 
 template <typename OutT, int LN>

@@ -50,10 +50,22 @@ def test_against_64_bits(rows, K_, N):
     assert K.device_status() == 0
 
 
-def test_a_row_does_not_depend_on_the_others():
+@pytest.mark.parametrize("K_,N", [(512, 64), (1016, 1024), (1024, 1024), (1024, 3088), (1024, 4096), (1536, 3200), (2048, 8192), (2048, 8320), (2048, 9408), (4096, 1032)])
+def test_up_to_16_rows_a_row_does_not_depend_on_the_others(K_, N):
+    """Whichever kernel takes the product: on both sides of the lines between the two.  (Beyond 16 rows sums are in another order.)"""
     from gpt_triton_b200 import kernels as K
 
-    a, op = _randn(16, 4096, seed=1).bfloat16().to(DEV), K.operand_rows(_randn(1032, 4096, seed=2).bfloat16().to(DEV))[0]
-    whole = K.linear(a, op, out_dtype=torch.float32)
-    for rows in (1, 3, 8, 9):
-        assert torch.equal(K.linear(a[:rows].contiguous(), op, out_dtype=torch.float32), whole[:rows])
+    a, w = _randn(16, K_, seed=1).bfloat16().to(DEV), _randn(N, K_, seed=2, scale=K_ ** -0.5).bfloat16()
+    op, pairs = K.operand_rows(w.to(DEV))[0], K.operand_rows(K.interleave_gated(w[:N // 2], w[N // 2:]).to(DEV))[0]
+    sumsq, x0, gain, bias = _randn(3, 16, seed=3).abs().to(DEV), _randn(16, N, seed=4).to(DEV), _randn(N, seed=5).to(DEV), _randn(pairs.shape[0], seed=6).to(DEV)
+
+    def results(rows):
+        normed = K.NormedRows(a[:rows].contiguous(), sumsq[:, :rows].contiguous(), K_, 1e-3)
+        x = x0[:rows].clone()
+        following = K.linear_residual(normed, op, x, gain, 1e-3)
+        return [K.linear(normed, op, out_dtype=torch.float32), K.linear(normed, op, act="silu"), x, following.data, following.sumsq.t(),
+                K.gated_linear(normed, pairs, bias, N // 2, limit=1.5, alpha=1.7)]
+
+    whole = results(16)
+    for rows in (1, 3, 8, 9, 15):
+        assert all(torch.equal(few, all_[:rows]) for few, all_ in zip(results(rows), whole))
