@@ -277,7 +277,8 @@ attention_kernel(const TIn* __restrict__ q, const TIn* __restrict__ k, const TIn
 // each thread converts what it has fetched; with two pairs of fp16 tiles that takes one barrier per block instead of two.  Blocks
 // masked for all of a warp's rows are left out warp by warp, and only the warp's diagonal blocks are masked.  12 heads of 64, fp16 out,
 // us, attention_kernel | this: 1 x 300 tokens 17.0 | 9.4, 16 x 300 40.0 | 24.1, 64 x 300 202 | 95, 8 x 1024 231 | 81, 16 x 2048 1389 |
-// 535.  What is left is the instructions of the exponentials, the conversions and mma.sync.
+// 535.  What is left is the instructions of the exponentials, the conversions and mma.sync.  Where four CTAs, or two of eight warps, share
+// an SM the registers end at 128, and heads of 64 spill 16 to 24 bytes per thread, heads of 32 with one pair of tiles 8.
 template <int D, int WARPS, int BUFS, typename TOut>
 struct F32Cfg {
   static constexpr int ROWS = WARPS * 16, THREADS = WARPS * 32, LDS = D + PAD;
@@ -394,7 +395,7 @@ static int launch_f32(const float* q, const float* k, const float* v, TOut* out,
     attr_set[slot].store(true, std::memory_order_release);
   }
   const int64_t tiles = (L + C::ROWS - 1) / C::ROWS * B * NH;
-  LaunchSetup ls(dim3((unsigned)tiles), dim3(C::THREADS), C::SMEM, stream, 1, pdl_enabled() || B * L <= kMidRowsPdl);
+  LaunchSetup ls(dim3((unsigned)tiles), dim3(C::THREADS), C::SMEM, stream, 1, pdl_enabled() || B * L <= 128);
   const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, attention_f32_kernel<D, WARPS, BUFS, TOut>, q, k, v, out, (int)(B * NH), (int)NH, (int)L, sq, sk, sv, so, scale, vec_out);
   note_launches(1);
   return status_from_cuda(e);

@@ -186,14 +186,21 @@ inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK :
 //     kernel in front has left, and barriers, tensor memory and descriptors are ready when it ends (a forward of the 124M
 //     model without | with: 10 x 300 tokens 1454 | 1359 us, 40 x 300 3592 | 3410; 355M, 4 x 500 2729 | 2594; 16 x 300 in
 //     fp32 2253 | 2175);
-//   - LayerNorms, row statistics out of moments, and attention of one launch's few tiles up to kMidRowsPdl rows.  Further
-//     up their many small CTAs take the SMs from the last tiles in front of them: LayerNorms on top of the wide products'
-//     gain at 4800 rows in fp32 2175 | 2140 us, at 19200 6773 | 6916; statistics at 3000 rows 1359 | 1326, at 4500
-//     1601 | 1571, at 6000 1927 | 1981; such attention at 2000 rows (355M) 2594 | 2551, at 8000 6365 | 6391.
+//   - LayerNorms up to kFewRowsPdl rows (forwards in fp32 of 37 to 500 rows 1 to 4 % shorter, in 16 bits as long), row statistics out
+//     of moments up to kMidRowsPdl (124M, 355M and 1.5B models, 600 to 1200 rows: up to 3 % shorter).  Further up their many small CTAs
+//     take the SMs from the last tiles in front of them: LayerNorms at 2400 to 5000 rows up to 2 % longer, statistics up to 4 %;
+//   - attention where a row's chain of key blocks is short: what starts early finds only some SMs free and doubles up there, which a
+//     long chain pays for.  Forward of the 124M model without | with, tcgen05: 2 x 300 tokens 630 | 620 us, 1 x 500 540 | 559, 2 x 500 717 | 736; the
+//     operator alone, back to back, 12 heads of 64: 4 x 160 6.63 | 6.00, 2 x 300 8.54 | 7.90, 8 x 300 (288 tiles) 9.8 | 10.0, 2 x 1024 19.2 |
+//     20.8, 2 x 2048 43.6 | 50.6: up to 320 rows per sequence and 1.5 tiles per SM (kShortChainRows).  In float32 up to 128 rows (2 %
+//     shorter; 1 x 500 745 | 852, 2 x 500 897 | 995);
+//   - attention over a window up to kWindowRowsPdl rows (prompts 0 to 1.3 % shorter).
 // Attention of many tiles does not: four CTAs of it fit an SM, and back to back they slow each other by up to 28 %.
 bool pdl_enabled();
 constexpr int64_t kFewRowsPdl = 512;
-constexpr int64_t kMidRowsPdl = 5120;
+constexpr int64_t kMidRowsPdl = 1280;
+constexpr int64_t kShortChainRows = 320;
+constexpr int64_t kWindowRowsPdl = 5120;
 
 // cudaLaunchConfig_t with room for the two attributes this library uses: cluster size and programmatic serialization.
 struct LaunchSetup {
