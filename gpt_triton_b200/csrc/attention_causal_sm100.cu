@@ -1,4 +1,4 @@
-// Causal flash attention on the 5th-generation tensor cores: fp16 or bf16 storage, head sizes up to 64 (smaller ones are zero-filled by
+// Causal flash attention on the 5th-generation tensor cores: fp16 or bf16 storage, head sizes 32 and 64 (32 columns are zero-filled by
 // the loads).  The arithmetic is that of attention_sm100.cu (64-key blocks, P in fp16 relative to the running maximum of its block:
 // kernels.py:417-474 of the reference), bit for bit; what differs is how the work sits on an SM.
 //

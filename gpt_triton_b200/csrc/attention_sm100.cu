@@ -504,7 +504,7 @@ static int launch_causal(const void* q, const void* k, const void* v, void* out,
   return status_from_cuda(e);
 }
 
-// attention_causal_sm100.cu: head sizes up to 64
+// attention_causal_sm100.cu: head sizes 32 and 64
 int launch_causal_attention_sm100(const void* q, const void* k, const void* v, void* out, int64_t B, int64_t NH, int64_t L, int64_t D,
                                   const int64_t* qs, const int64_t* ks, const int64_t* vs, const int64_t* os, float scale, int dtype, int* status_word,
                                   cudaStream_t stream);
@@ -522,8 +522,10 @@ int launch_attention_sm100(const void* q, const void* k, const void* v, void* ou
   // sequence 4.8 | 4.3.
   // Smaller heads are zero-filled to 64, which the generic kernel does not need: up to 128 rows it stays (2 x 4 x 64 x 16 2.7 | 4.0,
   // 16 x 25 x 64 x 32 5.0 | 5.6; 64 x 25 x 64 x 32 12.6 | 9.7, but the two differ in the order of their sums, and what a row gives is
-  // not to depend on the batch).  Beyond: 4 x 12 x 300 x 32 11.6 | 8.8, 16 x 12 x 1024 x 32 123 | 49.
-  if (D < 64 && L <= 128) return B200_ERR_UNSUPPORTED;
+  // not to depend on the batch).  Beyond, heads of 32: 4 x 12 x 300 11.6 | 8.8, 16 x 12 x 1024 123 | 49; up to 160 rows with fewer than 100
+  // tiles in bf16 6.8 | 7.1, with 600 1.4 times as fast.  Heads of 16 waste three quarters of a tile and stay at any length: bf16, 12 heads,
+  // 4 x 129 5.2 | 6.9, 2 x 300 7.0 | 9.4, 1 x 1024 20.4 | 22.4 (with 500 and more tiles 1.2 to 1.6 times as fast).
+  if (D == 16 || (D < 64 && L <= 128)) return B200_ERR_UNSUPPORTED;
   const int64_t n_items = (L + attn100::BLOCK_M - 1) / attn100::BLOCK_M * B * NH;
   if (D == 64 && L > 128 && n_items <= (L <= 1024 ? 2 : 3) * (int64_t)sm_count())
     return launch_causal<64>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);

@@ -3,13 +3,15 @@
 A pass makes the library calls that the operators of kernels.py make one by one, in the same order and with the same arguments:
 the same results, without 15 to 30 us of Python per launch.  What a pass reads of a model (operand and vector addresses) is a table
 that is kept with the model's derived operands and rebuilt when a parameter changes; what it reads of a call is passed each time.
-Where a model or a call is not what the passes cover, the functions here return None and the caller runs the operators.
+Where a model or a call is not what the passes cover, the functions here return None and the caller runs the operators: weights that are
+no parameters of their modules, sizes other than the modules' constants, subclasses, replaced functions, hooks that would be called.
 
 So does a pass that is being captured: a replay costs the host the same either way, and graphs of the operators, each with buffers of
 its own, replay faster (one sequence of 37 tokens, GPT-2 124M: 398-403 us against 405-415, whatever the workspace's address).
 
 What a pass costs the host, 124M and decoders of width 1024 with 8 layers, operators -> here: GPT-2 fp16 logits 2240 -> 390 us, float32
-hidden rows 1810 -> 380, Fogilix prompt 1370 -> 350, Nufasun prompt 1890 -> 500; most of what is left are the launches.
+hidden rows 1810 -> 380, Fogilix prompt 1370 -> 350, Nufasun prompt 1890 -> 500; most of what is left are the launches.  The first pass of a
+model, and the first after a change of its weights, runs the operators and costs what they do; the second makes the table.
 """
 
 import ctypes

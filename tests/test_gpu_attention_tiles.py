@@ -79,3 +79,15 @@ def test_growing_scores():
     k = k.abs() * (torch.arange(L, device=DEV) / 100.0)[None, None, :, None].half()
     _check(q, k, v, K.flash_attention_v1(q, k, v))
     assert K.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,L", [(16, 100), (16, 129), (16, 300), (16, 1100), (32, 128)])
+def test_small_heads_stay_with_the_generic_kernel(dtype, D, L):
+    """The bits of the one kernel that takes rows at any address."""
+    from gpt_triton_b200 import kernels as K
+
+    q, k, v = _qkv(2, 3, L, D, dtype)
+    anywhere = [torch.empty(t.numel() + 1, dtype=dtype, device=DEV)[1:].view(t.shape).copy_(t) for t in (q, k, v)]
+    assert torch.equal(K.flash_attention_v1(q, k, v), K.flash_attention_v1(*anywhere))
+    assert K.device_status() == 0
