@@ -517,9 +517,9 @@ int launch_attention_sm100(const void* q, const void* k, const void* v, void* ou
   if (D == 128) return launch_causal<128>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
   if (D > 64) return B200_ERR_UNSUPPORTED;
   // Up to 64 columns: four tiles an SM (attention_causal_sm100.cu) give the higher rate, two of this kernel's a tile's result sooner.
-  // The same bits, so the choice may follow the batch.  us, fp16, 12 heads of 64, here | there: 8 x 300 (288 tiles) 9.4 | 9.8, 9 x 300
-  // (324) 11.1 | 10.1, 64 x 300 42 | 32; 2 x 2048 (384) 42.6 | 44.1, 3 x 2048 (576) 51.6 | 47.2, 16 x 2048 219 | 181; one tile per
-  // sequence 4.8 | 4.3.
+  // The same bits, so the choice may follow the batch.  us, 12 heads of 64, fp16 (bf16 alike, 4 to 8 % longer), here | there: 8 x 300
+  // (288 tiles) 9.4 | 9.8, 9 x 300 (324) 11.1 | 10.1, 64 x 300 42 | 32; 8 x 512 (384) 17.3 | 15.9; 4 x 800 (336) 20.0 | 20.8, 5 x 800 (420) 23.6 | 21.5;
+  // 4 x 1024 (384) 26.4 | 25.5; 2 x 2048 (384) 42.6 | 44.1, 3 x 2048 (576) 51.6 | 47.2, 16 x 2048 219 | 181; one tile per sequence 4.8 | 4.3.
   // Smaller heads are zero-filled to 64, which the generic kernel does not need: up to 128 rows it stays (2 x 4 x 64 x 16 2.7 | 4.0,
   // 16 x 25 x 64 x 32 5.0 | 5.6; 64 x 25 x 64 x 32 12.6 | 9.7, but the two differ in the order of their sums, and what a row gives is
   // not to depend on the batch).  Beyond, heads of 32: 4 x 12 x 300 11.6 | 8.8, 16 x 12 x 1024 123 | 49; up to 160 rows with fewer than 100
@@ -527,7 +527,7 @@ int launch_attention_sm100(const void* q, const void* k, const void* v, void* ou
   // 4 x 129 5.2 | 6.9, 2 x 300 7.0 | 9.4, 1 x 1024 20.4 | 22.4 (with 500 and more tiles 1.2 to 1.6 times as fast).
   if (D == 16 || (D < 64 && L <= 128)) return B200_ERR_UNSUPPORTED;
   const int64_t n_items = (L + attn100::BLOCK_M - 1) / attn100::BLOCK_M * B * NH;
-  if (D == 64 && L > 128 && n_items <= (L <= 1024 ? 2 : 3) * (int64_t)sm_count())
+  if (D == 64 && L > 128 && 5 * n_items <= (L <= 512 ? 10 : L <= 1024 ? 12 : 15) * (int64_t)sm_count())
     return launch_causal<64>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
   return launch_causal_attention_sm100(q, k, v, out, B, NH, L, D, qs, ks, vs, os, scale, in_dtype, status_word, stream);
 }
