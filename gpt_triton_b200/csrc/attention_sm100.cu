@@ -496,7 +496,8 @@ static int launch_causal(const void* q, const void* k, const void* v, void* out,
   int64_t grid = (int64_t)sm_count() * C::CTAS_PER_SM;
   if (grid > n_items) grid = n_items;
   // S = Q K^T in the storage format; P V always fp16 x fp16 (see the top of this file)
-  LaunchSetup ls(dim3((unsigned)grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, 1, pdl_enabled() || (L <= kShortChainRows && 2 * n_items <= 3 * (int64_t)sm_count()));
+  const bool early = C::CTAS_PER_SM == 1 ? B * L <= kManyRowsPdl : L <= 200 || (L <= kShortChainRows && 2 * n_items <= 3 * (int64_t)sm_count());
+  LaunchSetup ls(dim3((unsigned)grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, 1, pdl_enabled() || early);
   const cudaError_t e = dtype == B200_BF16
                             ? cudaLaunchKernelEx(&ls.cfg, attention_sm100_kernel<__nv_bfloat16, D, false>, mq, mk, mv, p, idesc(1, 1, 0, BLOCK_N), idesc(0, 0, 1, D))
                             : cudaLaunchKernelEx(&ls.cfg, attention_sm100_kernel<__half, D, false>, mq, mk, mv, p, idesc(0, 0, 0, BLOCK_N), idesc(0, 0, 1, D));
@@ -547,7 +548,7 @@ static int launch_window(const CUtensorMap& mq, const CUtensorMap& mk, const CUt
   }
   int64_t grid = (int64_t)sm_count() * C::CTAS_PER_SM;
   if (grid > n_items) grid = n_items;
-  LaunchSetup ls(dim3((unsigned)grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, 1, pdl_enabled() || (int64_t)p.B * p.L <= kWindowRowsPdl);
+  LaunchSetup ls(dim3((unsigned)grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, 1, pdl_enabled() || (int64_t)p.B * p.L <= kManyRowsPdl);
   const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, kernel, mq, mk, mv, p, idesc(1, 1, 0, BLOCK_N), idesc(0, 0, 1, D));
   note_launches(1);
   return status_from_cuda(e);

@@ -191,16 +191,17 @@ inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK :
 //     take the SMs from the last tiles in front of them: LayerNorms at 2400 to 5000 rows up to 2 % longer, statistics up to 4 %;
 //   - attention where a row's chain of key blocks is short: what starts early finds only some SMs free and doubles up there, which a
 //     long chain pays for.  Forward of the 124M model without | with, tcgen05: 2 x 300 tokens 630 | 620 us, 1 x 500 540 | 559, 2 x 500 717 | 736; the
-//     operator alone, back to back, 12 heads of 64: 4 x 160 6.63 | 6.00, 2 x 300 8.54 | 7.90, 8 x 300 (288 tiles) 9.8 | 10.0, 2 x 1024 19.2 |
-//     20.8, 2 x 2048 43.6 | 50.6: up to 320 rows per sequence and 1.5 tiles per SM (kShortChainRows).  In float32 up to 128 rows (2 %
-//     shorter; 1 x 500 745 | 852, 2 x 500 897 | 995);
-//   - attention over a window up to kWindowRowsPdl rows (prompts 0 to 1.3 % shorter).
+//     operator alone, back to back, 12 heads of 64: 4 x 160 6.63 | 6.00, 12 x 200 (288 tiles) 8.4 | 8.0, 2 x 300 8.54 | 7.90, 8 x 300 (288)
+//     9.8 | 10.0, 2 x 1024 19.2 | 20.8, 2 x 2048 43.6 | 50.6: up to 200 rows per sequence, up to 320 (kShortChainRows) with 1.5 tiles per SM.
+//     In float32 up to 128 rows (2 % shorter; 1 x 500 745 | 852, 2 x 500 897 | 995);
+//   - attention up to kManyRowsPdl rows where nothing doubles up, heads of 128 (one CTA an SM; operator alone, 8 heads, 36 x 64 8.3 | 7.5,
+//     12 x 300 16.0 | 14.9, 1 x 1024 19.7 | 18.6), and over a window (prompts 0 to 1.3 % shorter).
 // Attention of many tiles does not: four CTAs of it fit an SM, and back to back they slow each other by up to 28 %.
 bool pdl_enabled();
 constexpr int64_t kFewRowsPdl = 512;
 constexpr int64_t kMidRowsPdl = 1280;
 constexpr int64_t kShortChainRows = 320;
-constexpr int64_t kWindowRowsPdl = 5120;
+constexpr int64_t kManyRowsPdl = 5120;
 
 // cudaLaunchConfig_t with room for the two attributes this library uses: cluster size and programmatic serialization.
 struct LaunchSetup {
