@@ -496,7 +496,7 @@ static int launch_causal(const void* q, const void* k, const void* v, void* out,
   int64_t grid = (int64_t)sm_count() * C::CTAS_PER_SM;
   if (grid > n_items) grid = n_items;
   // S = Q K^T in the storage format; P V always fp16 x fp16 (see the top of this file)
-  const bool early = C::CTAS_PER_SM == 1 ? B * L <= kManyRowsPdl : L <= 200 || (L <= kShortChainRows && 2 * n_items <= 3 * (int64_t)sm_count());
+  const bool early = C::CTAS_PER_SM == 1 ? B * L <= kManyRowsPdl : L <= kShortChainRows;
   LaunchSetup ls(dim3((unsigned)grid), dim3(NUM_THREADS), C::SMEM_BYTES, stream, 1, pdl_enabled() || early);
   const cudaError_t e = dtype == B200_BF16
                             ? cudaLaunchKernelEx(&ls.cfg, attention_sm100_kernel<__nv_bfloat16, D, false>, mq, mk, mv, p, idesc(1, 1, 0, BLOCK_N), idesc(0, 0, 1, D))

@@ -186,20 +186,21 @@ inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK :
 //     kernel in front has left, and barriers, tensor memory and descriptors are ready when it ends (a forward of the 124M
 //     model without | with: 10 x 300 tokens 1454 | 1359 us, 40 x 300 3592 | 3410; 355M, 4 x 500 2729 | 2594; 16 x 300 in
 //     fp32 2253 | 2175);
-//   - LayerNorms up to kFewRowsPdl rows (forwards in fp32 of 37 to 500 rows 1 to 4 % shorter, in 16 bits as long), row statistics out
-//     of moments up to kMidRowsPdl (124M, 355M and 1.5B models, 600 to 1200 rows: up to 3 % shorter).  Further up their many small CTAs
-//     take the SMs from the last tiles in front of them: LayerNorms at 2400 to 5000 rows up to 2 % longer, statistics up to 4 %;
+//   - LayerNorms up to kManyRowsPdl rows, row statistics out of moments up to kMidRowsPdl.  Time of a forward without : with, launched
+//     call by call | in a replayed graph (where kernels follow each other sooner as it is): LayerNorms, fp32, 500 to 1200 rows
+//     1.02-1.06 | 1.00-1.03, 2400 to 5000 1.00-1.03 | 0.98-1.00; statistics, 124M and 355M models, 600 to 1200 rows 1.00-1.07 |
+//     1.00-1.03, 2400 to 4000 1.01-1.03 | 0.99-1.00, 4800 and 5000 0.97-1.01 | 0.97-1.00, 7200 0.96-0.99;
 //   - attention where a row's chain of key blocks is short: what starts early finds only some SMs free and doubles up there, which a
-//     long chain pays for.  Forward of the 124M model without | with, tcgen05: 2 x 300 tokens 630 | 620 us, 1 x 500 540 | 559, 2 x 500 717 | 736; the
-//     operator alone, back to back, 12 heads of 64: 4 x 160 6.63 | 6.00, 12 x 200 (288 tiles) 8.4 | 8.0, 2 x 300 8.54 | 7.90, 8 x 300 (288)
-//     9.8 | 10.0, 2 x 1024 19.2 | 20.8, 2 x 2048 43.6 | 50.6: up to 200 rows per sequence, up to 320 (kShortChainRows) with 1.5 tiles per SM.
-//     In float32 up to 128 rows (2 % shorter; 1 x 500 745 | 852, 2 x 500 897 | 995);
-//   - attention up to kManyRowsPdl rows where nothing doubles up, heads of 128 (one CTA an SM; operator alone, 8 heads, 36 x 64 8.3 | 7.5,
-//     12 x 300 16.0 | 14.9, 1 x 1024 19.7 | 18.6), and over a window (prompts 0 to 1.3 % shorter).
+//     long chain pays for.  Up to kShortChainRows rows per sequence: 124M, 2 x 300 tokens 1.04 | 1.02, 8 x 300 1.02 | 1.01, but 1 x 500 0.98 | 0.96, 2 x
+//     500 0.98-1.00 | 0.95-0.97; the operator alone, back to back, 12 heads of 64, us without | with: 4 x 160 6.6 | 6.0, 12 x 200 8.4 | 8.0, 2 x 300 8.5 |
+//     7.9, 8 x 300 9.8 | 10.0, 2 x 1024 19.2 | 20.8, 2 x 2048 43.6 | 50.6.  Heads of 128 up to kManyRowsPdl rows: one CTA an SM, nothing doubles up
+//     (alone, 8 heads, 36 x 64 8.3 | 7.5, 12 x 300 16.0 | 14.9, 1 x 1024 19.7 | 18.6); windows too (prompts 1.00-1.01);
+//   - float32 attention up to 128 rows, and up to kManyRowsPdl with six tiles per SM or more, which level what doubles up: 16 x 300 1.02 | 1.01, 5 x
+//     1000 1.03 | 1.03; with fewer 10 x 300 1.00 | 0.99, 4 x 1000 0.98 | 0.96, 2 x 500 0.92 | 0.90.
 // Attention of many tiles does not: four CTAs of it fit an SM, and back to back they slow each other by up to 28 %.
 bool pdl_enabled();
 constexpr int64_t kFewRowsPdl = 512;
-constexpr int64_t kMidRowsPdl = 1280;
+constexpr int64_t kMidRowsPdl = 4096;
 constexpr int64_t kShortChainRows = 320;
 constexpr int64_t kManyRowsPdl = 5120;
 

@@ -342,7 +342,7 @@ layernorm_generic_kernel(const TI* x, const TI* __restrict__ w, const TI* __rest
 template <typename TI, typename TO>
 static int layernorm_typed(const void* x, const void* w, const void* b, void* out, int64_t M, int64_t H, float eps,
                            cudaStream_t stream) {
-  LaunchSetup ls(dim3(row_grid(M)), dim3(kWarpsPerBlock * 32), 0, stream, 1, pdl_enabled() || M <= kFewRowsPdl);
+  LaunchSetup ls(dim3(row_grid(M)), dim3(kWarpsPerBlock * 32), 0, stream, 1, pdl_enabled() || M <= kManyRowsPdl);
   const uintptr_t al = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(out);
   const bool vec = (H % 8 == 0) && (al & 15) == 0 && H <= 4096;
   const TI *xp = (const TI*)x, *wp = (const TI*)w, *bp = (const TI*)b;
