@@ -149,7 +149,7 @@ class Fogilix(StreamDecoder):
     def _whole_pass(self, ids, ctx, step):
         """The pass as one host call, None where that does not cover it."""
         table = passes.table_of(self, ("pass",), self._table) if len(self.layers) and passes.call_ok(self, ids, ctx, step) else None
-        if table is None or not passes.unchanged(table.extra["subs"]):
+        if table is None or not passes.unchanged():
             return None
         memories = None
         if ctx.cache is not None:

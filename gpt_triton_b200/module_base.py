@@ -56,20 +56,23 @@ _PLAIN = {int, float, str, tuple, type(None)}
 def parameter_tags(module, structure=False):
     """What tells whether a parameter of `module` or of one below it was replaced, cast, moved or written in place: equal lists, no
     change.  With `structure` also whether one was renamed, added or taken away (a weight that is pruned, say, is no parameter any more), a
-    module exchanged, one of its constants set or derived operands dropped.  (A walk over the module tree's own dictionaries:
-    Module.parameters() takes 3 us per parameter, as long as a launch.)"""
+    module exchanged, one of its constants set, an attribute (a function, say) set on one below, or derived operands dropped.  (A walk
+    over the module tree's own dictionaries: Module.parameters() takes 3 us per parameter, as long as a launch.)"""
     tags, stack = [], [module]
     while stack:
         m = stack.pop()
         d = m.__dict__
+        params = d["_parameters"]
         if structure:
-            tags.append(m.__class__)
-            tags.extend(d["_parameters"])
             cache = d.get("_operand")
             if cache is not None:
                 tags.append((cache.cleared, d.get("config"), [v for v in d.values() if v.__class__ in _PLAIN]))
-        tags.extend([(p.data_ptr(), p._version, p.dtype, p.device, p.shape) for p in d["_parameters"].values() if p is not None])
-        stack.extend(c for c in d["_modules"].values() if c is not None)
+            tags += (m.__class__, m is module or len(d), *params)
+            # (the device goes with the address)
+            tags += [(p.data_ptr(), p._version, p.dtype, p.shape) for p in params.values() if p is not None]
+        else:
+            tags += [(p.data_ptr(), p._version, p.dtype, p.device, p.shape) for p in params.values() if p is not None]
+        stack.extend([c for c in d["_modules"].values() if c is not None])
     return tags
 
 

@@ -122,11 +122,15 @@ def stands_for(owner, *names):
         _replaced[place] = (vars(place), read, read(vars(place)))
 
 
-def unchanged(modules):
-    """Whether every function that a pass would run in the place of is the package's own: the classes of `modules` exactly, no function
-    set on an instance, none replaced in a class or in kernels.py."""
-    return (all(read(space) == functions for space, read, functions in _replaced.values())
-            and all([m.__class__ in _methods and m.__dict__.keys().isdisjoint(_methods[m.__class__]) for m in modules]))
+def own(modules):
+    """Whether modules are of the package's classes exactly, with no function set on an instance (at the making of a table: its tags
+    show what changes later)."""
+    return all(type(m) in _methods and _methods[type(m)].isdisjoint(m.__dict__) for m in modules)
+
+
+def unchanged():
+    """Whether every function of a class or of kernels.py that a pass would run in the place of is the package's own."""
+    return all([read(space) == functions for space, read, functions in _replaced.values()])
 
 
 stands_for(K, "fused_embeddings", "fused_layer_norm", "fused_ffn", "takes_operand_rows", "operand_ffn", "operand_ffn_residual", "kv_cache_fill", "split_qkv",
@@ -166,7 +170,7 @@ def _gpt_table(model, blocks, folded):
     if model.wpe_weight.shape[1] != h or wte.shape[1] != h or not (wte.is_contiguous() and model.wpe_weight.is_contiguous()) or model.wpe_weight.dtype != wte.dtype:
         return None
     for pair in blocks:
-        if pair[0].num_heads != heads:
+        if not own(pair) or pair[0].num_heads != heads:
             return None
         for m, want in zip(pair, shapes):
             if not registered(m, want) or any(tuple(m._parameters[n].shape) != s or m._parameters[n].dtype != wte.dtype or m._parameters[n].device != wte.device
@@ -200,7 +204,7 @@ def gpt_body(model, ids, kv_caches, pos, attention_type, mlp_type):
     blocks = [tuple(b._modules.values()) for b in model.blocks._modules.values()]
     if not blocks or any(len(b) != 2 or type(b[0]) is not attention_type or type(b[1]) is not mlp_type or b[0].training or b[1].training for b in blocks):
         return None
-    if not unchanged([m for b in blocks for m in b]):
+    if not unchanged():
         return None
     folded = model._folds()
     if not folded and _hooked(m for b in blocks for m in b):
@@ -238,12 +242,12 @@ def gpt_body(model, ids, kv_caches, pos, attention_type, mlp_type):
 # ----------------------------------------------------------------------------- decoders with an fp32 residual stream
 def stock(model, norms, layers):
     """Whether a decoder is what a table describes: `norms`: (name, shape) of weights of its own, `layers`: (layer, names of its norms'
-    weights), each with a mixer `mix` and a feed-forward `mlp` or None.  Every weight has the shape that the modules' constants give (those
+    weights), each with a mixer `mix` and a feed-forward `mlp` or None, of the package's own kinds.  Every weight has the shape that the modules' constants give (those
     size the workspace: wider weights would be written past it), the type of the embeddings, and lies where they do."""
     embed, W = model.embed, model.config.width
     weights = [(model, {"embed": (embed.shape[0], W), **dict(norms)})] + [(layer, dict.fromkeys(names, (W,))) for layer, names in layers]
     weights += [(s, s._shapes(W)) for layer, _ in layers for s in (layer.mix, layer.mlp) if s is not None]
-    return embed.is_contiguous() and all(registered(m, shapes) and all(p.shape == shape and p.dtype == embed.dtype and p.device == embed.device
+    return embed.is_contiguous() and own(m for m, _ in weights[1 + len(layers):]) and all(registered(m, shapes) and all(p.shape == shape and p.dtype == embed.dtype and p.device == embed.device
                                                                        for p, shape in ((m._parameters[n], shapes[n]) for n in shapes))
                                          for m, shapes in weights)
 

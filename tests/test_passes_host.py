@@ -136,21 +136,25 @@ def test_a_model_saved_by_an_earlier_version():
 def test_functions_that_are_not_the_packages_own(monkeypatch):
     gpt, fogilix = _gpt(), _decoder("fogilix")
     pairs, subs = [m for b in _blocks(gpt) for m in b], [s for layer in fogilix.layers for s in (layer.mix, layer.mlp) if s is not None]
-    assert passes.unchanged(pairs) and passes.unchanged(subs) and not passes.unchanged([torch.nn.Identity()])
-    for module, name, others in ((pairs[2], "forward_folded", pairs), (pairs[1], "forward", pairs), (subs[0], "prompt", subs), (subs[1], "_stacked", subs)):
+    assert passes.own(pairs) and passes.own(subs) and not passes.own([torch.nn.Identity()])
+    for model, module, name, others in ((gpt, pairs[2], "forward_folded", pairs), (gpt, pairs[1], "forward", pairs), (fogilix, subs[0], "prompt", subs),
+                                        (fogilix, subs[1], "_stacked", subs)):
+        before = parameter_tags(model, structure=True)
         setattr(module, name, lambda *args, **kwargs: None)
-        assert not passes.unchanged(others)
+        assert not passes.own(others) and parameter_tags(model, structure=True) != before
+        assert model is gpt or not _is_stock(model)
         delattr(module, name)
-        assert passes.unchanged(others)
-    kind = type(subs[0])
+        assert passes.own(others) and parameter_tags(model, structure=True) == before
+    kind, before = type(subs[0]), parameter_tags(fogilix, structure=True)
     subs[0].__class__ = type("Other", (kind,), {"prompt": lambda *args: None})
-    assert not passes.unchanged(subs)
+    assert not passes.own(subs) and not _is_stock(fogilix) and parameter_tags(fogilix, structure=True) != before
     subs[0].__class__ = kind
+    assert _is_stock(fogilix)
     for owner, name in ((K, "linear"), (K, "fused_ffn"), (FusedAttention, "decode"), (mixers.LightningAttention, "_mix"), (mixers._Sublayer, "_stacked")):
         with monkeypatch.context() as m:
             m.setattr(owner, name, lambda *args, **kwargs: None)
-            assert not passes.unchanged(subs)
-        assert passes.unchanged(subs)
+            assert not passes.unchanged()
+        assert passes.unchanged()
 
 
 def test_blocks_of_other_kinds_run_their_own_code():
