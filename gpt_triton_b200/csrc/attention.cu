@@ -395,7 +395,7 @@ static int launch_f32(const float* q, const float* k, const float* v, TOut* out,
     attr_set[slot].store(true, std::memory_order_release);
   }
   const int64_t tiles = (L + C::ROWS - 1) / C::ROWS * B * NH;
-  const bool early = B * L <= 128 || (B * L <= kManyRowsPdl && (L + BLOCK - 1) / BLOCK * B * NH >= 6 * (int64_t)sm_count());
+  const bool early = B * L <= 128 || (B * L <= kManyRowsPdl && (L <= BLOCK || (L + BLOCK - 1) / BLOCK * B * NH >= 6 * (int64_t)sm_count()));
   LaunchSetup ls(dim3((unsigned)tiles), dim3(C::THREADS), C::SMEM, stream, 1, pdl_enabled() || early);
   const cudaError_t e = cudaLaunchKernelEx(&ls.cfg, attention_f32_kernel<D, WARPS, BUFS, TOut>, q, k, v, out, (int)(B * NH), (int)NH, (int)L, sq, sk, sv, so, scale, vec_out);
   note_launches(1);

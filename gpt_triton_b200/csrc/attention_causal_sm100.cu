@@ -14,8 +14,9 @@
 // What bounds it: the chain of a block, 2900 cycles of which 1400 are the two MMAs and their hand-overs, 750 the exponentials, 320 the
 // maximum, 310 the rescaling of O; four chains an SM come to 725 cycles a block, where the special-function unit needs 512 for its
 // 8192 exponentials (54 % busy).  Two tiles an SM with two threads per row (attention_sm100.cu): 1040 cycles.  us, fp16 | bf16, before ->
-// now, batch x heads x rows x columns: 16 x 12 x 2048 x 64 221 -> 175 | 245 -> 191, 64 x 12 x 300 x 64 42.5 -> 30.7 | 45.8 -> 34.1, 16 x 16 x
-// 1024 x 64 87 -> 67 | 96 -> 75; 16 x 12 x 1024 x 32 123 -> 50 | 124 -> 55 (generic kernel before).
+// now, batch x heads x rows x columns, ten calls on views of a fused projection after a pause (calls without end, the clock pulled down):
+// 16 x 12 x 2048 x 64 229 -> 184 | 252 -> 199 (248 -> 208 | 263 -> 218), 64 x 12 x 300 x 64 48 -> 36 | 51 -> 39 (46 -> 37 | 49 -> 38; in a replayed graph
+// 42 -> 31 | 46 -> 34), 16 x 16 x 1024 x 64 95 -> 74 | 103 -> 82; 16 x 12 x 1024 x 32 159 -> 55 | 157 -> 61 (generic kernel before).
 // Tried: three tiles with tensor memory for S, P and O apart, S issued a block ahead (189 us at 16 x 12 x 2048: the three tiles' exponentials
 // fall together, 1450 cycles each, and nothing overlaps them); the same with a turn per scheduler for the exponentials (231) and with two
 // threads per row (222: 72 registers, spills).

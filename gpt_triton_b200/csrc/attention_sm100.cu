@@ -518,7 +518,7 @@ int launch_attention_sm100(const void* q, const void* k, const void* v, void* ou
   if (D == 128) return launch_causal<128>(q, k, v, out, B, NH, L, qs, ks, vs, os, scale, in_dtype, status_word, stream);
   if (D > 64) return B200_ERR_UNSUPPORTED;
   // Up to 64 columns: four tiles an SM (attention_causal_sm100.cu) give the higher rate, two of this kernel's a tile's result sooner.
-  // The same bits, so the choice may follow the batch.  us, 12 heads of 64, fp16 (bf16 alike, 4 to 8 % longer), here | there: 8 x 300
+  // The same bits, so the choice may follow the batch.  us in replayed graphs, 12 heads of 64, fp16 (bf16 alike, 4 to 8 % longer), here | there: 8 x 300
   // (288 tiles) 9.4 | 9.8, 9 x 300 (324) 11.1 | 10.1, 64 x 300 42 | 32; 8 x 512 (384) 17.3 | 15.9; 4 x 800 (336) 20.0 | 20.8, 5 x 800 (420) 23.6 | 21.5;
   // 4 x 1024 (384) 26.4 | 25.5; 2 x 2048 (384) 42.6 | 44.1, 3 x 2048 (576) 51.6 | 47.2, 16 x 2048 219 | 181; one tile per sequence 4.8 | 4.3.
   // Smaller heads are zero-filled to 64, which the generic kernel does not need: up to 128 rows it stays (2 x 4 x 64 x 16 2.7 | 4.0,

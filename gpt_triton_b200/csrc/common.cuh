@@ -195,8 +195,9 @@ inline int status_from_cuda(cudaError_t e) { return e == cudaSuccess ? B200_OK :
 //     500 0.98-1.00 | 0.95-0.97; the operator alone, back to back, 12 heads of 64, us without | with: 4 x 160 6.6 | 6.0, 12 x 200 8.4 | 8.0, 2 x 300 8.5 |
 //     7.9, 8 x 300 9.8 | 10.0, 2 x 1024 19.2 | 20.8, 2 x 2048 43.6 | 50.6.  Heads of 128 up to kManyRowsPdl rows: one CTA an SM, nothing doubles up
 //     (alone, 8 heads, 36 x 64 8.3 | 7.5, 12 x 300 16.0 | 14.9, 1 x 1024 19.7 | 18.6); windows too (prompts 1.00-1.01);
-//   - float32 attention up to 128 rows, and up to kManyRowsPdl with six tiles per SM or more, which level what doubles up: 16 x 300 1.02 | 1.01, 5 x
-//     1000 1.03 | 1.03; with fewer 10 x 300 1.00 | 0.99, 4 x 1000 0.98 | 0.96, 2 x 500 0.92 | 0.90.
+//   - float32 attention up to 128 rows, and up to kManyRowsPdl where a sequence is one block of keys (9 x 61 tokens 1.01 launched call by call) or
+//     six tiles per SM or more level what doubles up: 16 x 300 1.02 | 1.01, 5 x 1000 1.03 | 1.03; else 10 x 300 1.00 | 0.99, 4 x 1000
+//     0.98 | 0.96, 2 x 500 0.92 | 0.90.
 // Attention of many tiles does not: four CTAs of it fit an SM, and back to back they slow each other by up to 28 %.
 bool pdl_enabled();
 constexpr int64_t kFewRowsPdl = 512;
