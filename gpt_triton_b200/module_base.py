@@ -62,7 +62,10 @@ def parameter_tags(module, structure=False):
     while stack:
         m = stack.pop()
         d = m.__dict__
-        params = d["_parameters"]
+        params = d.get("_parameters")
+        if params is None:  # (a model, or a part of one, that is no nn.Module or keeps its parameters elsewhere)
+            tags += [(p.data_ptr(), p._version, p.dtype, p.device, p.shape) for p in m.parameters()]
+            continue
         if structure:
             cache = d.get("_operand")
             if cache is not None:

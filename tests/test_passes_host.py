@@ -223,3 +223,22 @@ def test_an_output_product_of_another_depth_is_refused(kind, fields):
     assert passes._passes.b200_decoder_pass_workspace_bytes(ctypes.byref(args)) == 0
     args.ids = args.table = args.out = args.sumsq_out = args.workspace = 4096
     assert passes._passes.b200_decoder_pass(ctypes.byref(args), None) == 1
+
+
+def test_tags_of_models_that_are_no_modules():
+    """A session's model offers `parameters()`; it need not be an nn.Module."""
+    class Model:
+        def __init__(self):
+            self.weights = [torch.zeros(3), torch.ones(2, 2)]
+
+        def parameters(self):
+            return iter(self.weights)
+
+    model = Model()
+    before = parameter_tags(model)
+    assert len(before) == 2 and parameter_tags(model) == before
+    model.weights[1].add_(1)
+    assert parameter_tags(model) != before
+    holder = torch.nn.Module()
+    holder._modules["part"] = model
+    assert len(parameter_tags(holder)) == 2
